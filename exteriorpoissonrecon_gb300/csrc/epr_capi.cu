@@ -147,7 +147,15 @@ bool Context::sync_system32(int l)
     }
     if (L.N > (dim == 3 ? 27 : 81))
     {
-        const size_t bytes = S * L.N * (lvl32(l) ? sizeof(float) : sizeof(double));
+        const size_t real = lvl32(l) ? sizeof(float) : sizeof(double);
+        if (dim == 3 && pair_level<3>(l))
+        {
+            if (!L.Acb && !alloc(&L.Acb, 56 * L.N * real, "alloc colour blocks")) return false;
+            if (lvl32(l)) launch_to_pair_blocks<float>(l, L.A64, L.B64, (float *)L.Acb, stream);
+            else launch_to_pair_blocks<double>(l, L.A64, L.B64, (double *)L.Acb, stream);
+            return launch_ok("convert system");
+        }
+        const size_t bytes = S * L.N * real;
         if (!L.Acb && (!alloc(&L.Acb, bytes, "alloc colour blocks") || !alloc(&L.Bcb, bytes, "alloc colour blocks"))) return false;
         auto blocks = [&](auto dd) {
             constexpr int D = decltype(dd)::value;
@@ -660,8 +668,6 @@ epr_ctx *epr_create(int dim, int depth, const epr_params *params)
     }
     {
         std::lock_guard<std::mutex> lock(g_create_mutex);
-        if (const char *v = getenv("EPR_GS_VARIANT")) epr::set_gs_variant(atoi(v));
-        if (const char *v = getenv("EPR_LANES_VARIANT")) epr::set_lanes_variant(atoi(v));
         if (const char *v = getenv("EPR_TINY_LEVELS")) epr::set_tiny_levels(atoi(v));
         if (const char *v = getenv("EPR_CLUSTER_LEVELS")) epr::set_cluster_levels(atoi(v));
         static uint64_t prepared = 0;  // devices whose kernel attributes are set

@@ -401,181 +401,259 @@ __device__ __forceinline__ void component_fit_pq3(const Real *x, const Real *y, 
     }
 }
 
-template <int D, typename Real>
-__device__ __forceinline__ void element_fit(const Real *x, const Real *y, int A, Real *h)
-{
-    component_fit<D, 0>(x, y, A, h);
-    component_fit<D, 1>(x, y, A, h);
-    component_fit<D, 2>(x, y, A, h);
-    if constexpr (D == 4)
-    {
-        component_fit<D, 3>(x, y, A, h);
-        component_fit<D, 4>(x, y, A, h);
-        component_fit<D, 5>(x, y, A, h);
-    }
-}
-
 // ---------------------------------------------------------------------------------------------
-// Packed float version of element_fit for corner 0 (canonical orientation), on Blackwell's
-// two-wide FP32 instructions (FFMA2 / FMUL2: two lanes of arithmetic per issue slot).  The x and
-// y fields travel together as (x, y) pairs, so every derivative table is one packed table; at a
-// Gauss point, with p = (x_P, y_P), q = (x_Q, y_Q) the P- and Q-derivatives,
-//   T = phP q - phQ p = (V, -U),   W = y_P x_Q - x_P y_Q,
-// and the five integrals accumulate as (h1, h0) += (w T) * T, (h4, -h3) += (w T) * W and
-// h2 += wU V.  The sums are those of element_fit in another association order (float rounding
-// differs in the last bits); the fast float relaxation uses it, the double path keeps the scalar
-// code.
+// Quadratic-fit integrals of corner 0 (every node's elements are taken in the canonical
+// orientation, mirrored so that the node is their corner 0: mirroring along axis d flips the sign
+// of every d-derivative, and each component of W, U and V carries exactly one derivative along each
+// of its two axes, so the products below keep their sign).
+//
+// On the reference element with t = 2 xi - 1 a field is f = sum_a m_a t^a over subsets a of the
+// axes.  With the corner differences d_c = f_c - f_0 and the signed sums
+//     D_a = sum_c d_c prod_{d in a} (1 - 2 c_d) = (-1)^|a| 2^D m_a      (D_a = 1 for phi_0),
+// the component (P, Q) of W(x, y) is, up to the sign (-1)^|g| of each monomial t^g and a constant,
+//     W = sum_{b with Q, a with P} [D_b, D_a] t^(a+b-P-Q),    [u, v] = u_x v_y - u_y v_x,
+// and U, V (x or y replaced by phi_0) have D_b - D_a in the place of the minor.  So along P and Q
+// only the monomials 1, t_P, t_Q survive (weights 1, 1/3, 1/3; the t_P t_Q minors cancel), and
+// along every other axis U and V carry phi_0's factor (1 + s), s = -t, which all five integrals
+// share: they are exact on the two-point Gauss-Jacobi rule of the weight 1 + s, where the three
+// minors are those of q = D_Q + s D_QR, p = D_P + s D_PR, m = D_PQ + s D_PQR (bilinear in (s_R, s_S)
+// in 4D).  In 3D the sums |U|^2, |V|^2, <U,V> need no points at all: they are one quadratic form of
+// the seven D_a, diagonal in the sums and differences that permuting the axes leaves apart.
+//
+// Per element and node this takes about 230 multiplies and adds in 3D and 1,200 in 4D (the
+// 2 x 2 x 3^(D-2)-point Gauss rule on derivative tables took 750 and 6,000); in float the (x, y)
+// pairs travel on the two-wide FP32 instructions.  The corner differences are formed first, so the
+// rounding is relative to the variation over the element and not to the fields' offset.
 // ---------------------------------------------------------------------------------------------
-struct PackedFit
-{
-    float2 hv = {0.f, 0.f};  // (h1, h0)
-    float2 hw = {0.f, 0.f};  // (h4, -h3)
-    float h2 = 0.f;
-    __device__ __forceinline__ void add_to(float *h) const
-    {
-        h[0] += hv.y;
-        h[1] += hv.x;
-        h[2] += h2;
-        h[3] -= hw.y;
-        h[4] += hw.x;
-    }
-};
-
-__device__ __forceinline__ float2 splat2(float v) { return make_float2(v, v); }
-
-// derivative_partial on (x, y) pairs (a - b formed as fma(b, -1, a), which rounds once like a - b)
-template <int D, int K, bool AisP>
-__device__ __forceinline__ void derivative_partial_packed(const float2 *f, float2 (&t)[2][1 << (D - 2)])
-{
-    using Cp = Component<D, K>;
-    constexpr int NO = 1 << Cp::M;
-    float2 dif[2][NO];
-#pragma unroll
-    for (int bB = 0; bB < 2; bB++)
-#pragma unroll
-        for (int bo = 0; bo < NO; bo++)
-        {
-            int c1 = AisP ? Cp::corner(1, bB, bo) : Cp::corner(bB, 1, bo);
-            int c0 = AisP ? Cp::corner(0, bB, bo) : Cp::corner(bB, 0, bo);
-            dif[bB][bo] = __ffma2_rn(f[c0], splat2(-1.f), f[c1]);
-        }
-#pragma unroll
-    for (int g = 0; g < 2; g++)
-#pragma unroll
-        for (int bo = 0; bo < NO; bo++)
-            t[g][bo] = __ffma2_rn(splat2(hat2<float>(1, g)), dif[1][bo], __fmul2_rn(splat2(hat2<float>(0, g)), dif[0][bo]));
-}
-
-// ... and its value at the other-axis Gauss point go (derivative_at on pairs)
-template <int M>
-__device__ __forceinline__ float2 derivative_at_packed(const float2 *t, int go)
-{
-    if constexpr (M == 1) return __ffma2_rn(splat2(hat3<float>(1, go)), t[1], __fmul2_rn(splat2(hat3<float>(0, go)), t[0]));
-    else
-    {
-        const int g0 = go / 3, g1 = go % 3;
-        const float2 a0 = splat2(hat3<float>(0, g0)), a1 = splat2(hat3<float>(1, g0));
-        const float2 u0 = __ffma2_rn(a1, t[2], __fmul2_rn(a0, t[0]));
-        const float2 u1 = __ffma2_rn(a1, t[3], __fmul2_rn(a0, t[1]));
-        return __ffma2_rn(splat2(hat3<float>(1, g1)), u1, __fmul2_rn(splat2(hat3<float>(0, g1)), u0));
-    }
-}
-
-template <int D, int K>
-__device__ __forceinline__ void component_fit_packed(const float2 *c, PackedFit &acc)
-{
-    using Cp = Component<D, K>;
-    constexpr int M = Cp::M;
-    constexpr int NG = ipow(3, M);
-    float2 tP[2][1 << M], tQ[2][1 << M];
-    derivative_partial_packed<D, K, true>(c, tP);
-    derivative_partial_packed<D, K, false>(c, tQ);
-#pragma unroll
-    for (int go = 0; go < NG; go++)
-    {
-        // corner 0: every hat factor is the one of bit 0, both signs are -1
-        float lo;
-        if constexpr (M == 1) lo = hat3<float>(0, go);
-        else lo = hat3<float>(0, go / 3) * hat3<float>(0, go % 3);
-        const float wo = (float)other_weight<M>(go);
-        float2 Pg[2], Qg[2];
-#pragma unroll
-        for (int g = 0; g < 2; g++)
-        {
-            Pg[g] = derivative_at_packed<M>(tP[g], go);
-            Qg[g] = derivative_at_packed<M>(tQ[g], go);
-        }
-#pragma unroll
-        for (int gp = 0; gp < 2; gp++)
-#pragma unroll
-            for (int gq = 0; gq < 2; gq++)
-            {
-                const float w = (float)(Gauss::W2(gp) * Gauss::W2(gq)) * wo;
-                const float phP = -hat2<float>(0, gq) * lo;
-                const float phQ = -hat2<float>(0, gp) * lo;
-                const float2 p = Pg[gq], q = Qg[gp];
-                const float W = fmaf(p.y, q.x, -(p.x * q.y));
-                const float2 T = __ffma2_rn(splat2(phP), q, __fmul2_rn(splat2(-phQ), p));
-                const float2 wT = __fmul2_rn(splat2(w), T);
-                acc.hv = __ffma2_rn(wT, T, acc.hv);
-                acc.hw = __ffma2_rn(wT, splat2(W), acc.hw);
-                acc.h2 = fmaf(-wT.y, T.x, acc.h2);
-            }
-    }
-}
-
-// element_fit<D, float>(x, y, 0, h) on interleaved (x, y) corners
-template <int D>
-__device__ __forceinline__ void element_fit_packed(const float2 *c, float *h)
-{
-    PackedFit acc;
-    component_fit_packed<D, 0>(c, acc);
-    component_fit_packed<D, 1>(c, acc);
-    component_fit_packed<D, 2>(c, acc);
-    if constexpr (D == 4)
-    {
-        component_fit_packed<D, 3>(c, acc);
-        component_fit_packed<D, 4>(c, acc);
-        component_fit_packed<D, 5>(c, acc);
-    }
-    acc.add_to(h);
-}
-
-// ---------------------------------------------------------------------------------------------
-// Canonical orientation.  Mirroring an element along axis d (xi_d -> 1 - xi_d) flips the sign of
-// every d-derivative; each component of W, U and V carries exactly one derivative along each of
-// its two axes, so all the products in the fit integrals keep their sign.  Any corner A can
-// therefore be evaluated as corner 0 of the element mirrored along the axes where A has a 1 bit,
-// which makes every hat factor a compile-time constant.
-// ---------------------------------------------------------------------------------------------
-template <int D, typename Real>
-struct Corners
-{
-    Real x[1 << D];
-    Real y[1 << D];
-};
 template <typename Real>
-struct Fit5
+struct Ops
 {
-    Real h[5];
+    using V = Real2<Real>;
+    static __device__ __forceinline__ Real add(Real a, Real b) { return a + b; }
+    static __device__ __forceinline__ Real sub(Real a, Real b) { return a - b; }
+    static __device__ __forceinline__ Real mul(Real a, Real b) { return a * b; }
+    static __device__ __forceinline__ Real fma(Real a, Real b, Real c) { return a * b + c; }
+    static __device__ __forceinline__ V add(V a, V b) { return V{a.x + b.x, a.y + b.y}; }
+    static __device__ __forceinline__ V sub(V a, V b) { return V{a.x - b.x, a.y - b.y}; }
+    static __device__ __forceinline__ V scale(Real s, V a) { return V{s * a.x, s * a.y}; }
+    static __device__ __forceinline__ V mul(V a, V b) { return V{a.x * b.x, a.y * b.y}; }
+    static __device__ __forceinline__ V fma(V a, V b, V c) { return V{a.x * b.x + c.x, a.y * b.y + c.y}; }
+    static __device__ __forceinline__ V fma(Real s, V b, V c) { return V{s * b.x + c.x, s * b.y + c.y}; }
+};
+// every rounding explicit, so that each kernel that inlines the fit computes the same bits
+template <>
+struct Ops<double>
+{
+    using V = double2;
+    static __device__ __forceinline__ double add(double a, double b) { return __dadd_rn(a, b); }
+    static __device__ __forceinline__ double sub(double a, double b) { return __dsub_rn(a, b); }
+    static __device__ __forceinline__ double mul(double a, double b) { return __dmul_rn(a, b); }
+    static __device__ __forceinline__ double fma(double a, double b, double c) { return __fma_rn(a, b, c); }
+    static __device__ __forceinline__ V add(V a, V b) { return V{add(a.x, b.x), add(a.y, b.y)}; }
+    static __device__ __forceinline__ V sub(V a, V b) { return V{sub(a.x, b.x), sub(a.y, b.y)}; }
+    static __device__ __forceinline__ V scale(double s, V a) { return V{mul(s, a.x), mul(s, a.y)}; }
+    static __device__ __forceinline__ V mul(V a, V b) { return V{mul(a.x, b.x), mul(a.y, b.y)}; }
+    static __device__ __forceinline__ V fma(V a, V b, V c) { return V{fma(a.x, b.x, c.x), fma(a.y, b.y, c.y)}; }
+    static __device__ __forceinline__ V fma(double s, V b, V c) { return V{fma(s, b.x, c.x), fma(s, b.y, c.y)}; }
+};
+template <>
+struct Ops<float>
+{
+    using V = float2;
+    static __device__ __forceinline__ float add(float a, float b) { return __fadd_rn(a, b); }
+    static __device__ __forceinline__ float sub(float a, float b) { return __fsub_rn(a, b); }
+    static __device__ __forceinline__ float mul(float a, float b) { return __fmul_rn(a, b); }
+    static __device__ __forceinline__ float fma(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+    static __device__ __forceinline__ V add(V a, V b) { return __fadd2_rn(a, b); }
+    static __device__ __forceinline__ V sub(V a, V b) { return __fadd2_rn(a, make_float2(-b.x, -b.y)); }
+    static __device__ __forceinline__ V mul(V a, V b) { return __fmul2_rn(a, b); }
+    static __device__ __forceinline__ V fma(V a, V b, V c) { return __ffma2_rn(a, b, c); }
+    static __device__ __forceinline__ V scale(float s, V a) { return __fmul2_rn(make_float2(s, s), a); }
+    static __device__ __forceinline__ V fma(float s, V b, V c) { return __ffma2_rn(make_float2(s, s), b, c); }
 };
 
-template <int D, typename Real>
-__device__ __noinline__ Fit5<Real> element_fit_canonical(Corners<D, Real> c)
+// minor [u, v] = u_x v_y - u_y v_x
+template <typename Real>
+__device__ __forceinline__ Real minor2(const Real2<Real> &u, const Real2<Real> &v)
 {
-    Fit5<Real> f;
-#pragma unroll
-    for (int k = 0; k < 5; k++) f.h[k] = 0;
-    component_fit<D, 0>(c.x, c.y, 0, f.h);
-    component_fit<D, 1>(c.x, c.y, 0, f.h);
-    component_fit<D, 2>(c.x, c.y, 0, f.h);
-    if constexpr (D == 4)
+    using O = Ops<Real>;
+    return O::fma(u.x, v.y, -O::mul(u.y, v.x));
+}
+
+// The two-point Gauss-Jacobi rule of the weight 1 + s on [-1, 1] (mean value): s = 1/5 -+ sqrt(6)/5.
+// Exact for cubics; its first moments are 1, 1/3, 1/3, 1/5.
+struct Jacobi
+{
+    __host__ __device__ static constexpr double S(int k) { return k == 0 ? -0.28989794855663561964 : 0.68989794855663561964; }
+    __host__ __device__ static constexpr double W(int k) { return k == 0 ? 0.36391723651204561 : 0.63608276348795439; }
+};
+
+// Sums of the fit over a node's elements, unscaled: hv = (|V|^2, |U|^2), h2 = -<U, V>, and the
+// parts of (<V, W>, -<U, W>) per weight of the Jacobi points (a, and m with a further 1/3).
+template <int D, typename Real>
+struct FitSums
+{
+    static constexpr int NW = D == 3 ? 2 : 3;  // distinct point weights
+    Real2<Real> hv, a[NW], m[NW];
+    Real h2;
+    __device__ __forceinline__ void clear()
     {
-        component_fit<D, 3>(c.x, c.y, 0, f.h);
-        component_fit<D, 4>(c.x, c.y, 0, f.h);
-        component_fit<D, 5>(c.x, c.y, 0, f.h);
+        hv = Real2<Real>{(Real)0, (Real)0};
+        h2 = (Real)0;
+#pragma unroll
+        for (int k = 0; k < NW; k++) a[k] = m[k] = Real2<Real>{(Real)0, (Real)0};
     }
-    return f;
+    // h += (|U|^2, |V|^2, <U,V>, <W,U>, <W,V>) in reference units
+    __device__ __forceinline__ void add_to(Real *h) const
+    {
+        using O = Ops<Real>;
+        constexpr double kq = D == 3 ? 11.0 / 6.0 / 192.0 : 1.0 / 4096.0, kl = D == 3 ? 1.0 / 256.0 : 1.0 / 4096.0;
+        constexpr double w[3] = {D == 3 ? Jacobi::W(0) : Jacobi::W(0) * Jacobi::W(0),
+                                 D == 3 ? Jacobi::W(1) : Jacobi::W(0) * Jacobi::W(1), Jacobi::W(1) * Jacobi::W(1)};
+        Real2<Real> hw = {(Real)0, (Real)0};
+#pragma unroll
+        for (int k = 0; k < NW; k++) hw = O::fma((Real)(w[k] * kl), O::fma((Real)(1.0 / 3.0), m[k], a[k]), hw);
+        h[0] = O::fma((Real)kq, hv.y, h[0]);
+        h[1] = O::fma((Real)kq, hv.x, h[1]);
+        h[2] = O::fma((Real)-kq, h2, h[2]);
+        h[3] = O::sub(h[3], hw.y);
+        h[4] = O::add(h[4], hw.x);
+    }
+};
+
+// s.a[k] += q (W1 + WQ/3) - p (W1 + WP/3), s.m[k] += m (WP - WQ): one point of <T, W> (T = (V, -U))
+// with T1 = q - p, TP = m - p, TQ = q - m and the minors W1 = [q, p], WP = [m, p], WQ = [q, m]
+template <int D, typename Real>
+__device__ __forceinline__ void fit_point(FitSums<D, Real> &s, int k, const Real2<Real> &q, const Real2<Real> &p, const Real2<Real> &m)
+{
+    using O = Ops<Real>;
+    const Real third = (Real)(1.0 / 3.0);
+    const Real W1 = minor2<Real>(q, p), WP = minor2<Real>(m, p), WQ = minor2<Real>(q, m);
+    s.a[k] = O::fma(O::fma(third, WQ, W1), q, s.a[k]);
+    s.a[k] = O::fma(-O::fma(third, WP, W1), p, s.a[k]);
+    s.m[k] = O::fma(O::sub(WP, WQ), m, s.m[k]);
+}
+
+// one square of the quadratic forms: hv += w z^2, h2 += w z_x z_y
+template <int D, typename Real>
+__device__ __forceinline__ void fit_square(FitSums<D, Real> &s, double w, const Real2<Real> &z)
+{
+    using O = Ops<Real>;
+    const Real2<Real> wz = w == 1.0 ? z : O::scale((Real)w, z);
+    s.hv = O::fma(wz, z, s.hv);
+    s.h2 = O::fma(wz.x, z.y, s.h2);
+}
+
+// the fit sums of corner 0 from the corner differences d[c] = f_c - f_0 (d[0] unused)
+template <typename Real>
+__device__ __forceinline__ void element_fit_sums(const Real2<Real> (&d)[8], FitSums<3, Real> &s)
+{
+    using O = Ops<Real>;
+    using V = Real2<Real>;
+    // signed sums, one axis at a time (corner bits: axis 0 = 4, axis 1 = 2, axis 2 = 1)
+    const V s01 = O::add(d[2], d[3]), t01 = O::sub(d[2], d[3]);
+    const V s10 = O::add(d[4], d[5]), t10 = O::sub(d[4], d[5]);
+    const V s11 = O::add(d[6], d[7]), t11 = O::sub(d[6], d[7]);
+    const V ss0 = O::add(d[1], s01), st0 = O::sub(d[1], s01);
+    const V ss1 = O::add(s10, s11), st1 = O::sub(s10, s11);
+    const V ts0 = O::sub(t01, d[1]), tt0 = O::add(d[1], t01);  // tt0 with the opposite sign
+    const V ts1 = O::add(t10, t11), tt1 = O::sub(t10, t11);
+    V Dm[3], E[3];
+    Dm[0] = O::sub(ss0, ss1);
+    Dm[1] = O::add(st0, st1);
+    Dm[2] = O::add(ts0, ts1);
+    E[2] = O::sub(st0, st1);
+    E[1] = O::sub(ts0, ts1);
+    E[0] = O::sub(tt1, tt0);
+    const V Fn = O::add(tt0, tt1);  // - D_012
+    // |U|^2, |V|^2, <U,V>: squares of the axis-symmetric and the two axis-antisymmetric combinations
+    {
+        constexpr double kappa = 4.0 / 11.0;
+        constexpr double rho = 0.25 + 1.0 / 72.0 + 0.525 + 1.0 / 30.0 - 11.0 / 9.0 * kappa * kappa;
+        const V d01 = O::add(Dm[0], Dm[1]), e01 = O::add(E[0], E[1]);
+        const V pE = O::sub(E[0], E[1]), qE = O::fma((Real)-2.0, E[2], e01);
+        const V sD = O::add(d01, Dm[2]), sE = O::add(e01, E[2]);
+        fit_square<3, Real>(s, 1.0, O::fma((Real)-kappa, pE, O::sub(Dm[0], Dm[1])));
+        fit_square<3, Real>(s, 1.0 / 3.0, O::fma((Real)-kappa, qE, O::fma((Real)-2.0, Dm[2], d01)));
+        fit_square<3, Real>(s, rho * 9.0 / 11.0, pE);
+        fit_square<3, Real>(s, rho * 3.0 / 11.0, qE);
+        fit_square<3, Real>(s, 4.0 / 33.0, O::fma((Real)1.5, Fn, O::fma((Real)-0.5, sE, sD)));
+        fit_square<3, Real>(s, 1.0 / 55.0, O::fma((Real)3.0, Fn, sE));
+    }
+    // <V,W>, -<U,W> at the two points of the axis that is neither P nor Q
+#pragma unroll
+    for (int k = 0; k < 2; k++)
+    {
+        const Real t = (Real)Jacobi::S(k);
+#pragma unroll
+        for (int P = 1; P < 3; P++)
+#pragma unroll
+            for (int Q = 0; Q < P; Q++)
+                fit_point<3, Real>(s, k, O::fma(t, E[P], Dm[Q]), O::fma(t, E[Q], Dm[P]), O::fma(-t, Fn, E[3 - P - Q]));
+    }
+}
+
+template <typename Real>
+__device__ __forceinline__ void element_fit_sums(const Real2<Real> (&d)[16], FitSums<4, Real> &s)
+{
+    using O = Ops<Real>;
+    using V = Real2<Real>;
+    V D[16];
+    D[0] = V{(Real)0, (Real)0};
+#pragma unroll
+    for (int c = 1; c < 16; c++) D[c] = d[c];
+#pragma unroll
+    for (int b = 1; b < 16; b <<= 1)
+#pragma unroll
+        for (int c = 0; c < 16; c++)
+            if (!(c & b))
+            {
+                const V u = D[c], v = D[c | b];
+                D[c] = (c == 0 && b == 1) ? v : O::add(u, v);
+                D[c | b] = (c == 0 && b == 1) ? V{-v.x, -v.y} : O::sub(u, v);
+            }
+#pragma unroll
+    for (int P = 1; P < 4; P++)
+#pragma unroll
+        for (int Q = 0; Q < P; Q++)
+        {
+            constexpr int ax[4] = {8, 4, 2, 1};
+            const int R = Q > 0 ? 0 : (P > 1 ? 1 : 2), S = 6 - P - Q - R;
+            const int p = ax[P], q = ax[Q], r = ax[R], t = ax[S];
+#pragma unroll
+            for (int i = 0; i < 2; i++)
+            {
+                const Real si = (Real)Jacobi::S(i);
+                const V q0 = O::fma(si, D[q | r], D[q]), q1 = O::fma(si, D[q | r | t], D[q | t]);
+                const V p0 = O::fma(si, D[p | r], D[p]), p1 = O::fma(si, D[p | r | t], D[p | t]);
+                const V m0 = O::fma(si, D[p | q | r], D[p | q]), m1 = O::fma(si, D[p | q | r | t], D[p | q | t]);
+#pragma unroll
+                for (int j = 0; j < 2; j++)
+                {
+                    const Real sj = (Real)Jacobi::S(j);
+                    const V Vq = O::fma(sj, q1, q0), Vp = O::fma(sj, p1, p0), Vm = O::fma(sj, m1, m0);
+                    fit_point<4, Real>(s, i + j, Vq, Vp, Vm);
+                    // |T1|^2 + (|TP|^2 + |TQ|^2) / 3 = 7/6 |q - p|^2 + 1/6 |2 m - p - q|^2
+                    const double wv = Jacobi::W(i) * Jacobi::W(j) * (1.0 + Jacobi::S(i)) * (1.0 + Jacobi::S(j));
+                    fit_square<4, Real>(s, wv * 7.0 / 6.0, O::sub(Vq, Vp));
+                    fit_square<4, Real>(s, wv / 6.0, O::fma((Real)-2.0, Vm, O::add(Vp, Vq)));
+                }
+            }
+        }
+}
+
+// h += the fit integrals of corner 0 of the element with corner values f (canonical orientation)
+template <int D, typename Real>
+__device__ __forceinline__ void element_fit(const Real2<Real> (&f)[1 << D], Real *h)
+{
+    Real2<Real> d[1 << D];
+    d[0] = f[0];
+#pragma unroll
+    for (int c = 1; c < (1 << D); c++) d[c] = Ops<Real>::sub(f[c], f[0]);
+    FitSums<D, Real> s;
+    s.clear();
+    element_fit_sums<Real>(d, s);
+    s.add_to(h);
 }
 
 // ---------------------------------------------------------------------------------------------

@@ -18,8 +18,8 @@ struct LevelPtrs
     Real *xy = nullptr;       // 2N interleaved (x, y)
     const Real *A = nullptr;  // 3^Dim * N column stencil of R + dWeight K (offset-major)
     const Real *B = nullptr;  // 3^Dim * N column stencil of the frame constraint
-    const Real *Acb = nullptr;  // optional colour-blocked copies of A and B (colour_block_base)
-    const Real *Bcb = nullptr;
+    const Real *Acb = nullptr;  // optional colour-blocked copies of A and B (colour_block_base); on pair
+    const Real *Bcb = nullptr;  // levels both in Acb (PairLayout)
     // adaptive indexer: per node 0 (no function), 1 (indexed, held fixed), 2 (active); the
     // Gauss-Seidel kernels update active nodes only.  Null for the regular grid (all active).
     const uint8_t *status = nullptr;
@@ -49,11 +49,6 @@ void launch_quadfit(const LevelPtrs<Real> &L, const Real *xy, double *out, cudaS
 // separate != 0: the reference's SeparateGaussSeidelSolve update (x first, then y with the new x)
 template <int D, typename Real>
 void launch_gs_colour(const LevelPtrs<Real> &L, int colour, unsigned int *err, cudaStream_t s, int separate = 0);
-// selects the colour-kernel variant (0: one thread per node, 1: 2^D lanes per node on a row grid,
-// 2: 2^D lanes per node on a flat grid; 1 is the default, 0.69 ms against 0.70 ms at depth 8;
-// 4: as 1 without the point-split update of the small 3D levels)
-void set_gs_variant(int v);
-void set_lanes_variant(int v);
 // 1 (default): 3D levels 0-1 relax in gs_tiny_kernel (one warp per node-element incidence of a
 // colour); 0: in the block kernels
 void set_tiny_levels(int v);
@@ -96,6 +91,10 @@ void launch_galerkin(int fineLevel, const double *Mf, double *Mc, cudaStream_t s
 // colour-blocked copy (Real) of a natural offset-major double stencil of `level`
 template <int D, typename Real>
 void launch_to_colour_blocks(int level, const double *M, Real *out, cudaStream_t s);
+
+// both natural stencils of a 3D level (level >= kPairLevel) -> its pair layout (PairLayout, 56 values per node)
+template <typename Real>
+void launch_to_pair_blocks(int level, const double *A, const double *B, Real *out, cudaStream_t s);
 
 // elementwise helpers
 template <typename Real>

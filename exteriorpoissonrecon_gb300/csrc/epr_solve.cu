@@ -32,10 +32,10 @@ __device__ __forceinline__ Real2<Real> ld2(const Real *xy, int64_t i)
 }
 
 // r^(4-D)/2: scale from reference-element sums to physical integrals
-template <int D>
-__device__ __forceinline__ double wedge_scale(int r)
+template <int D, typename Real>
+__device__ __forceinline__ Real wedge_scale(int r)
 {
-    return (D == 3 ? (double)r : 1.0) * 0.5;
+    return (D == 3 ? (Real)r : (Real)1) * (Real)0.5;
 }
 
 template <int D>
@@ -69,82 +69,40 @@ __device__ __forceinline__ bool gather_element(const Grid<D> &g, const NodeCtx<D
     return true;
 }
 
-// stencil index of the neighbour at offset (o_0, ..., o_{D-1}), o_d in {-1, 0, 1}
-template <int D>
-__host__ __device__ constexpr int nb_index(const int *off)
-{
-    int o = 0;
-    for (int d = 0; d < D; d++) o = o * 3 + (off[d] + 1);
-    return o;
-}
-
 // Wedge part of the quadratic model of node i, elements in canonical orientation.
 template <int D, typename Real>
 __device__ __forceinline__ void node_wedge_fit(const Grid<D> &g, const NodeCtx<D> &nc, int64_t i, const Real *xy, Real *h)
 {
-    if constexpr (D == 3)
-    {
-        // the 27-node neighbourhood in registers; out-of-domain neighbours are never used
-        Real2<Real> nb[27];
-#pragma unroll
-        for (int o = 0; o < 27; o++)
-        {
-            const int o0 = o / 9 - 1, o1 = (o / 3) % 3 - 1, o2 = o % 3 - 1;
-            bool ok = (nc.I[0] + o0 >= 0) && (nc.I[0] + o0 <= g.r) && (nc.I[1] + o1 >= 0) && (nc.I[1] + o1 <= g.r) &&
-                      (nc.I[2] + o2 >= 0) && (nc.I[2] + o2 <= g.r);
-            int64_t j = i + o0 * nc.stride[0] + o1 * nc.stride[1] + o2 * nc.stride[2];
-            nb[o] = ok ? ld2(xy, j) : Real2<Real>{0, 0};
-        }
-#pragma unroll
-        for (int A = 0; A < 8; A++)
-        {
-            const int a0 = (A >> 2) & 1, a1 = (A >> 1) & 1, a2 = A & 1;
-            bool ok = (nc.I[0] - a0 >= 0) && (nc.I[0] - a0 < g.r) && (nc.I[1] - a1 >= 0) && (nc.I[1] - a1 < g.r) &&
-                      (nc.I[2] - a2 >= 0) && (nc.I[2] - a2 < g.r);
-            if (!ok) continue;
-            Corners<3, Real> c;
-#pragma unroll
-            for (int cc = 0; cc < 8; cc++)
-            {
-                int off[3] = {(a0 ? -1 : 1) * ((cc >> 2) & 1), (a1 ? -1 : 1) * ((cc >> 1) & 1), (a2 ? -1 : 1) * (cc & 1)};
-                Real2<Real> v = nb[nb_index<3>(off)];
-                c.x[cc] = v.x;
-                c.y[cc] = v.y;
-            }
-            Fit5<Real> f = element_fit_canonical<3, Real>(c);
-#pragma unroll
-            for (int k = 0; k < 5; k++) h[k] += f.h[k];
-        }
-    }
-    else
-    {
+    FitSums<D, Real> sums;
+    sums.clear();
+    const Real2<Real> own = ld2(xy, i);
 #pragma unroll 1
-        for (int A = 0; A < (1 << D); A++)
+    for (int A = 0; A < (1 << D); A++)
+    {
+        bool ok = true;
+        int64_t sd[D];
+#pragma unroll
+        for (int d = 0; d < D; d++)
         {
-            bool ok = true;
+            const int e = nc.I[d] - cbit<D>(A, d);
+            ok = ok && e >= 0 && e < g.r;
+            sd[d] = cbit<D>(A, d) ? -nc.stride[d] : nc.stride[d];
+        }
+        if (!ok) continue;
+        Real2<Real> df[1 << D];
+        df[0] = own;
+#pragma unroll
+        for (int cc = 1; cc < (1 << D); cc++)
+        {
+            int64_t j = i;
 #pragma unroll
             for (int d = 0; d < D; d++)
-            {
-                int e = nc.I[d] - cbit<D>(A, d);
-                ok = ok && e >= 0 && e < g.r;
-            }
-            if (!ok) continue;
-            Corners<D, Real> c;
-#pragma unroll
-            for (int cc = 0; cc < (1 << D); cc++)
-            {
-                int64_t j = i;
-#pragma unroll
-                for (int d = 0; d < D; d++) j += (int64_t)(cbit<D>(A, d) ? -cbit<D>(cc, d) : cbit<D>(cc, d)) * nc.stride[d];
-                Real2<Real> v = ld2(xy, j);
-                c.x[cc] = v.x;
-                c.y[cc] = v.y;
-            }
-            Fit5<Real> f = element_fit_canonical<D, Real>(c);
-#pragma unroll
-            for (int k = 0; k < 5; k++) h[k] += f.h[k];
+                if (cbit<D>(cc, d)) j += sd[d];
+            df[cc] = Ops<Real>::sub(ld2(xy, j), own);
         }
+        element_fit_sums<Real>(df, sums);
     }
+    sums.add_to(h);
 }
 
 // Quadratic model of E(x + s e_i, y + t e_i): q = (Q20, Q02, Q11, Q10, Q01)
@@ -154,7 +112,7 @@ __device__ __forceinline__ void node_fit(const LevelPtrs<Real> &L, const Grid<D>
 {
     Real h[5] = {0, 0, 0, 0, 0};
     node_wedge_fit<D, Real>(g, nc, i, xy, h);
-    const Real sc = (Real)wedge_scale<D>(g.r);
+    const Real sc = wedge_scale<D, Real>(g.r);
     q[0] = h[0] * sc;
     q[1] = h[1] * sc;
     q[2] = (Real)2 * h[2] * sc;
@@ -338,43 +296,12 @@ __global__ void __launch_bounds__(kThreads) grad_norm_kernel(LevelPtrs<Real> L, 
     block_sum_store<1>(acc, partial + 4 * blockIdx.x);
 }
 
-// Node step from the quadratic model q = (Q20, Q02, Q11, Q10, Q01) with H = [[2 Q20, Q11], [Q11, 2 Q02]]
-// and grad = (Q10, Q01).  Paired (ExteriorPoissonSolvers.h:173-181): -H^{-1} grad / 2 when
-// |det H| > 1e-20.  Separate (ExteriorPoissonSolvers.h:216-235): p0 = -grad0 / (2 H00) when
-// H00 > 1e-20, then p1 = -((H10 + H01) p0 + grad1) / (2 H11) when H11 > 1e-20.
-template <typename Real>
-__device__ __forceinline__ bool node_step(const Real *q, int separate, Real &p0, Real &p1)
-{
-    Real h00 = (Real)2 * q[0], h11 = (Real)2 * q[1], h01 = q[2];
-    if (separate)
-    {
-        p0 = 0;
-        p1 = 0;
-        if ((double)h00 > 1e-20) p0 = -((h01 + h01) * p1 + q[3]) / ((Real)2 * h00);
-        if ((double)h11 > 1e-20) p1 = -((h01 + h01) * p0 + q[4]) / ((Real)2 * h11);
-        return true;
-    }
-    Real det = h00 * h11 - h01 * h01;
-    if (!(fabs((double)det) > 1e-20)) return false;
-    p0 = -(h11 * q[3] - h01 * q[4]) / det / (Real)2;
-    p1 = -(-h01 * q[3] + h00 * q[4]) / det / (Real)2;
-    return true;
-}
-
-// Whether the Gauss-Seidel step of node i is applied: every node of the regular grid, the active
-// functions of the adaptive indexer (its colour lists hold those only, ExteriorPoisson.h:161-169)
-template <typename Real>
-__device__ __forceinline__ bool relaxed(const LevelPtrs<Real> &L, int64_t i)
-{
-    return L.status == nullptr || L.status[i] == 2;
-}
-
 // Comparisons and finiteness tests in a level's own arithmetic: a double-float tests its pair
 // without converting to FP64 where the leading float decides.
 template <typename Real>
 __device__ __forceinline__ bool exceeds(Real v, double t)
 {
-    return (double)v > t;
+    return v > (Real)t;
 }
 // a double-float compares by its leading float unless that is within a factor of two of t
 template <>
@@ -398,12 +325,57 @@ __device__ __forceinline__ df abs_value<df>(df v)
 template <typename Real>
 __device__ __forceinline__ bool finite_value(Real v)
 {
-    return isfinite((double)v);
+    return isfinite(v);
 }
 template <>
 __device__ __forceinline__ bool finite_value<df>(df v)
 {
     return isfinite(v.hi) && isfinite(v.lo);
+}
+
+// a b - c d; in float with the rounding errors of both products (Kahan's difference of products), since
+// where the fields' gradients are nearly parallel det H is a small difference of large products
+template <typename Real>
+__device__ __forceinline__ Real product_difference(Real a, Real b, Real c, Real d)
+{
+    return a * b - c * d;
+}
+template <>
+__device__ __forceinline__ float product_difference<float>(float a, float b, float c, float d)
+{
+    const float w = __fmul_rn(c, d);
+    return __fadd_rn(__fmaf_rn(a, b, -w), __fmaf_rn(-c, d, w));
+}
+
+// Node step from the quadratic model q = (Q20, Q02, Q11, Q10, Q01) with H = [[2 Q20, Q11], [Q11, 2 Q02]]
+// and grad = (Q10, Q01).  Paired (ExteriorPoissonSolvers.h:173-181): -H^{-1} grad / 2 when
+// |det H| > 1e-20.  Separate (ExteriorPoissonSolvers.h:216-235): p0 = -grad0 / (2 H00) when
+// H00 > 1e-20, then p1 = -((H10 + H01) p0 + grad1) / (2 H11) when H11 > 1e-20.
+template <typename Real>
+__device__ __forceinline__ bool node_step(const Real *q, int separate, Real &p0, Real &p1)
+{
+    Real h00 = (Real)2 * q[0], h11 = (Real)2 * q[1], h01 = q[2];
+    if (separate)
+    {
+        p0 = 0;
+        p1 = 0;
+        if (exceeds<Real>(h00, 1e-20)) p0 = -((h01 + h01) * p1 + q[3]) / ((Real)2 * h00);
+        if (exceeds<Real>(h11, 1e-20)) p1 = -((h01 + h01) * p0 + q[4]) / ((Real)2 * h11);
+        return true;
+    }
+    const Real det = product_difference<Real>(h00, h11, h01, h01);
+    if (!exceeds<Real>(abs_value<Real>(det), 1e-20)) return false;
+    p0 = -product_difference<Real>(h11, q[3], h01, q[4]) / det / (Real)2;
+    p1 = -product_difference<Real>(h00, q[4], h01, q[3]) / det / (Real)2;
+    return true;
+}
+
+// Whether the Gauss-Seidel step of node i is applied: every node of the regular grid, the active
+// functions of the adaptive indexer (its colour lists hold those only, ExteriorPoisson.h:161-169)
+template <typename Real>
+__device__ __forceinline__ bool relaxed(const LevelPtrs<Real> &L, int64_t i)
+{
+    return L.status == nullptr || L.status[i] == 2;
 }
 
 // node_step with the singularity tests in the level's own arithmetic
@@ -426,40 +398,6 @@ __device__ __forceinline__ bool node_step_tiny(const Real *q, int separate, Real
     p0 = (h11 * q[3] - h01 * q[4]) * m;
     p1 = (-h01 * q[3] + h00 * q[4]) * m;
     return true;
-}
-
-// Paired Gauss-Seidel update of node j of a parity colour.
-template <int D, typename Real>
-__device__ __forceinline__ void gs_update(const LevelPtrs<Real> &L, const Grid<D> &g, const Colour<D> &col, int64_t j, unsigned int *err,
-                                          int separate)
-{
-    NodeCtx<D> nc;
-    col.node(j, nc.I);
-#pragma unroll
-    for (int d = 0; d < D; d++) nc.stride[d] = g.stride(d);
-    int64_t i = g.node(nc.I);
-    Real q[5];
-    node_fit<D, Real>(L, g, nc, i, L.xy, q);
-    Real p0, p1;
-    if (relaxed(L, i) && node_step<Real>(q, separate, p0, p1))
-    {
-        Real2<Real> v = ld2(L.xy, i);
-        v.x += p0;
-        v.y += p1;
-        if (!isfinite((double)v.x) || !isfinite((double)v.y)) atomicOr(err, (unsigned int)ERR_NONFINITE);
-        reinterpret_cast<Real2<Real> *>(L.xy)[i] = v;
-    }
-}
-
-// One parity colour: same-colour nodes share no element, so all of them are updated in parallel
-// exactly as the reference's per-colour ParallelFor does.
-template <int D, typename Real>
-__global__ void __launch_bounds__(kThreads) gs_colour_kernel(LevelPtrs<Real> L, Colour<D> col, unsigned int *err, int separate)
-{
-    Grid<D> g(L.level);
-    int64_t j = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (j >= col.n) return;
-    gs_update<D, Real>(L, g, col, j, err, separate);
 }
 
 // Lane-parallel variant: a group of 2^D consecutive lanes updates one node, lane A integrating the
@@ -521,32 +459,109 @@ __device__ __forceinline__ Real wedge_mult(const int *kexp, int level)
     else return (Real)1;
 }
 
-// A block's row of nodes staged in shared memory (3D lane kernel): the (x, y) pairs of the 3 x 3 x W
-// grid points around the row (W = 2 nodes-per-block + 1 along the last axis) and the rows' stencil
-// columns, loaded once per block with coalesced loads, so that a node's 8 lanes read their corners
-// and neighbours from shared memory instead of re-fetching them through L1 / L2.
+// The float kernels fit a sheared pair: (x, y - a x), or (x - b y, y) where y varies more than x, with one
+// factor of at most 1 per node, from the products of the differences along the axes.  W is the same for
+// the sheared pair, and with the step (s + b t, t + a s) the model's Hessian keeps its determinant, so any
+// factor gives the same update in exact arithmetic.  Where the fields' gradients at the node are nearly
+// parallel, |U|^2, |V|^2 and <U, V> of the plain pair agree to most of float's digits in the determinant and
+// their rounding becomes the update's largest error; the sheared field's term is small instead.  (Eight
+// random systems on level 6, one sweep against 64 bits, relative L2: up to 1e-5 with the plain pair, up to
+// 5e-7 with the shear.)  Double (1e-14 off there) and double-float relax the plain pair.
 template <typename Real>
-struct LaneStage
-{
-    const Real2<Real> *tile = nullptr;
-    int tcentre = 0;  // tile index of the node (the tile's row length is a template parameter)
-    const Real *As = nullptr, *Bs = nullptr;  // column o of the block's t-th node at o npb + t
-    int npb = 0, t = 0;
-};
+constexpr bool shears() { return std::is_same<Real, float>::value; }
 
+template <typename Real>
+struct Shear
+{
+    Real a, b;  // one of them 0
+};
+__device__ __forceinline__ Shear<float> shear_of(float sxy, float sxx, float syy)
+{
+    const bool y = sxx >= syy;
+    float f = __fdividef(sxy, y ? sxx : syy);
+    f = fabsf(f) <= 2.f ? f : 0.f;  // also where the ratio is not finite
+    return Shear<float>{y ? f : 0.f, y ? 0.f : f};
+}
+template <typename Real>
+__device__ __forceinline__ Real2<Real> sheared(const Shear<Real> &sh, const Real2<Real> &v)
+{
+    return Real2<Real>{Ops<Real>::fma(-sh.b, v.y, v.x), Ops<Real>::fma(-sh.a, v.x, v.y)};
+}
+
+// q = (Q20, Q02, Q11, Q10, Q01) of the (sheared) pair from a node's wedge sums and its stencil columns:
+// av = sum A_j (x, y)_j, bv = sum B_j (x, y)_j without the centre, acen the centre of A.  Linear in all
+// of them, so lanes that share a node add their parts of q.
+template <int D, typename Real>
+__device__ __forceinline__ void fit_to_model(const FitSums<D, Real> &sums, Real sc, const Real2<Real> &av, const Real2<Real> &bv,
+                                             Real acen, const Shear<Real> &sh, Real *q)
+{
+    using O = Ops<Real>;
+    Real h[5] = {(Real)0, (Real)0, (Real)0, (Real)0, (Real)0};
+    sums.add_to(h);
+    const Real sc2 = O::add(sc, sc);
+    const Real gx = O::mul((Real)2, O::sub(av.x, bv.y)), gy = O::mul((Real)2, O::add(av.y, bv.x));
+    if constexpr (shears<Real>())
+    {
+        const Real aa = O::mul(sh.a, acen), ab = O::mul(sh.b, acen);
+        q[0] = O::fma(h[0], sc, O::fma(sh.a, aa, acen));
+        q[1] = O::fma(h[1], sc, O::fma(sh.b, ab, acen));
+        q[2] = O::fma(h[2], sc2, O::mul((Real)2, O::add(aa, ab)));
+        q[3] = O::fma(h[3], sc2, O::fma(sh.a, gy, gx));
+        q[4] = O::fma(h[4], sc2, O::fma(sh.b, gx, gy));
+    }
+    else
+    {
+        q[0] = O::fma(h[0], sc, acen);
+        q[1] = O::fma(h[1], sc, acen);
+        q[2] = O::mul(h[2], sc2);
+        q[3] = O::fma(h[3], sc2, gx);
+        q[4] = O::fma(h[4], sc2, gy);
+    }
+}
+
+// the step of node i from its whole model, by one thread
+template <typename Real>
+__device__ __forceinline__ void apply_step(const LevelPtrs<Real> &L, Real *xy, int64_t i, const Real *q, const Shear<Real> &sh, int separate,
+                                           unsigned int *err)
+{
+    Real p0, p1;
+    if (relaxed(L, i) && node_step<Real>(q, separate, p0, p1))
+    {
+        if constexpr (shears<Real>())
+        {
+            const Real s = p0;
+            p0 = Ops<Real>::fma(sh.b, p1, p0);
+            p1 = Ops<Real>::fma(sh.a, s, p1);
+        }
+        Real2<Real> v = ld2(xy, i);
+        v.x += p0;
+        v.y += p1;
+        if (!finite_value<Real>(v.x) || !finite_value<Real>(v.y)) atomicOr(err, (unsigned int)ERR_NONFINITE);
+        reinterpret_cast<Real2<Real> *>(xy)[i] = v;
+    }
+}
+
+// Lane A's part of the update of the node at I: the fit of the node's element A and the stencil
+// offsets that lane owns.  An offset's neighbour is a corner of every element on its side, and the
+// lane owns it whose element lies on the lower-numbered existing side of every axis the offset does
+// not move along; so each neighbour is one of the corners already in the lane's registers.
 // Ac, Bc (optional): the colour's block of the colour-blocked stencils, the node being the colour's
-// jc-th of nc; otherwise the natural stencils L.A, L.B are read.  Staged (3D): corners, neighbours
-// and stencil columns come from stg (the same values, so the same arithmetic).
-template <int D, typename Real, bool Packed = false, bool Staged = false, int SW = 1>
+// jc-th of nc; otherwise the natural stencils L.A, L.B are read.
+template <int D, typename Real>
 __device__ __forceinline__ void gs_update_lanes_at(const LevelPtrs<Real> &L, Real *xy, const Grid<D> &g, const int *I, bool active,
                                                    int A, unsigned int *err, int separate = 0, const Real *Ac = nullptr,
                                                    const Real *Bc = nullptr, int64_t jc = 0, int64_t nc = 0,
-                                                   Real wmul = (Real)1, const LaneStage<Real> &stg = LaneStage<Real>())
+                                                   Real wmul = (Real)1)
 {
-    constexpr int C = 1 << D, S = Dims<D>::S;
+    using O = Ops<Real>;
+    using V = Real2<Real>;
+    constexpr int C = 1 << D;
     int64_t i = 0;
-    Real h[5] = {0, 0, 0, 0, 0};
-    Real ax = 0, ay = 0, bx = 0, by = 0, acen = 0;
+    Real q[5] = {(Real)0, (Real)0, (Real)0, (Real)0, (Real)0};
+    V f[C], av = {(Real)0, (Real)0}, bv = {(Real)0, (Real)0};
+    Real acen = (Real)0, sxy = (Real)0, sxx = (Real)0, syy = (Real)0;
+    Shear<Real> sh = {(Real)0, (Real)0};
+    bool ok = active;
     if (active)
     {
         // node indices in 32 bits (every supported grid has < 2^32 nodes); signed strides of the
@@ -555,135 +570,223 @@ __device__ __forceinline__ void gs_update_lanes_at(const LevelPtrs<Real> &L, Rea
         st[D - 1] = 1;
 #pragma unroll
         for (int d = D - 2; d >= 0; d--) st[d] = st[d + 1] * (g.r + 1);
-        // strides of the staged tile (3 x 3 x SW), compile-time constants
-        constexpr int tst[3] = {3 * SW, SW, 1};
         uint32_t iu = 0;
-        bool ok = true;
+        int first = 0;  // the lower-numbered existing side of every axis, as corner bits
 #pragma unroll
         for (int d = 0; d < D; d++)
         {
             iu += (uint32_t)I[d] * (uint32_t)st[d];
             sd[d] = cbit<D>(A, d) ? -st[d] : st[d];
-            int e = I[d] - cbit<D>(A, d);
+            const int e = I[d] - cbit<D>(A, d);
             ok = ok && e >= 0 && e < g.r;
+            if (I[d] >= g.r) first |= 1 << (D - 1 - d);
         }
         i = iu;
         if (ok)
         {
-            if constexpr (std::is_same<Real, float>::value && Packed)
-            {
-                // the (x, y) corner pairs as loaded, on the two-wide FP32 instructions
-                float2 c2[C];
 #pragma unroll
-                for (int cc = 0; cc < C; cc++)
+            for (int cc = 0; cc < C; cc++)
+            {
+                int jj = (int)iu;
+#pragma unroll
+                for (int d = 0; d < D; d++)
+                    if (cbit<D>(cc, d)) jj += sd[d];
+                f[cc] = ld2(xy, (int64_t)(uint32_t)jj);
+            }
+            const int64_t step = Ac ? nc : L.N;
+            const Real *pA = (Ac ? Ac + jc : L.A + i) + (int64_t)Dims<D>::CENTER * step;
+            const Real *pB = (Ac ? Bc + jc : L.B + i) + (int64_t)Dims<D>::CENTER * step;
+            int64_t so[D];
+#pragma unroll
+            for (int d = 0; d < D; d++) so[d] = cbit<D>(A, d) ? -(int64_t)ipow(3, D - 1 - d) * step : (int64_t)ipow(3, D - 1 - d) * step;
+            const int other = A ^ first;
+#pragma unroll
+            for (int cc = 0; cc < C; cc++)
+                if ((other & ~cc & (C - 1)) == 0)
                 {
-                    if constexpr (Staged)
-                    {
-                        int tj = stg.tcentre;
+                    int64_t o = 0;
 #pragma unroll
-                        for (int d = 0; d < 3; d++)
-                            if (cbit<3>(cc, d)) tj += cbit<3>(A, d) ? -tst[d] : tst[d];
-                        c2[cc] = stg.tile[tj];
-                    }
-                    else
-                    {
-                        int jj = (int)iu;
-#pragma unroll
-                        for (int d = 0; d < D; d++)
-                            if (cbit<D>(cc, d)) jj += sd[d];
-                        c2[cc] = ld2(xy, (int64_t)(uint32_t)jj);
-                    }
+                    for (int d = 0; d < D; d++)
+                        if (cbit<D>(cc, d)) o += so[d];
+                    const Real a = pA[o];
+                    av = O::fma(a, f[cc], av);
+                    if (cc == 0) acen = a;
+                    else bv = O::fma(pB[o], f[cc], bv);
                 }
-                element_fit_packed<D>(c2, h);
-            }
-            else
-            {
-                Real x[C], y[C];
 #pragma unroll
-                for (int cc = 0; cc < C; cc++)
+            for (int cc = 1; cc < C; cc++) f[cc] = O::sub(f[cc], f[0]);
+            if constexpr (shears<Real>())
+#pragma unroll
+                for (int d = 0; d < D; d++)
                 {
-                    Real2<Real> v;
-                    if constexpr (Staged)
-                    {
-                        int tj = stg.tcentre;
-#pragma unroll
-                        for (int d = 0; d < 3; d++)
-                            if (cbit<3>(cc, d)) tj += cbit<3>(A, d) ? -tst[d] : tst[d];
-                        v = stg.tile[tj];
-                    }
-                    else
-                    {
-                        int jj = (int)iu;
-#pragma unroll
-                        for (int d = 0; d < D; d++)
-                            if (cbit<D>(cc, d)) jj += sd[d];
-                        v = ld2(xy, (int64_t)(uint32_t)jj);
-                    }
-                    x[cc] = v.x;
-                    y[cc] = v.y;
+                    sxy = O::fma(f[1 << d].x, f[1 << d].y, sxy);
+                    sxx = O::fma(f[1 << d].x, f[1 << d].x, sxx);
+                    syy = O::fma(f[1 << d].y, f[1 << d].y, syy);
                 }
-                element_fit<D, Real>(x, y, 0, h);
-            }
-        }
-        for (int o = A; o < S; o += C)
-        {
-            int off[D];
-            stencil_offset<D>(o, off);
-            bool in = true;
-            int jj = (int)iu;
-#pragma unroll
-            for (int d = 0; d < D; d++)
-            {
-                int t = I[d] + off[d];
-                in = in && (t >= 0) && (t <= g.r);
-                jj += off[d] * st[d];
-            }
-            if (!in) continue;
-            Real a, b;
-            if constexpr (Staged)
-            {
-                a = stg.As[o * stg.npb + stg.t];
-                b = stg.Bs[o * stg.npb + stg.t];
-            }
-            else if (Ac)
-            {
-                a = Ac[(int64_t)o * nc + jc];
-                b = Bc[(int64_t)o * nc + jc];
-            }
-            else
-            {
-                a = L.A[(int64_t)o * L.N + i];
-                b = L.B[(int64_t)o * L.N + i];
-            }
-            Real2<Real> v;
-            if constexpr (Staged) v = stg.tile[stg.tcentre + off[0] * tst[0] + off[1] * tst[1] + off[2] * tst[2]];
-            else v = ld2(xy, (int64_t)(uint32_t)jj);
-            ax += a * v.x;
-            ay += a * v.y;
-            if (o == Dims<D>::CENTER) acen = a;
-            else { bx += b * v.x; by += b * v.y; }
         }
     }
-#pragma unroll
-    for (int k = 0; k < 5; k++) h[k] = group_sum<D>(h[k]);
-    ax = group_sum<D>(ax); ay = group_sum<D>(ay); bx = group_sum<D>(bx); by = group_sum<D>(by); acen = group_sum<D>(acen);
-    if (!active || A != 0) return;
-    const Real sc = (Real)wedge_scale<D>(g.r) * wmul;
-    Real q[5];
-    q[0] = h[0] * sc + acen;
-    q[1] = h[1] * sc + acen;
-    q[2] = (Real)2 * h[2] * sc;
-    q[3] = (Real)2 * h[3] * sc + (Real)2 * ax - (Real)2 * by;
-    q[4] = (Real)2 * h[4] * sc + (Real)2 * ay + (Real)2 * bx;
-    Real p0, p1;
-    if (relaxed(L, i) && node_step<Real>(q, separate, p0, p1))
+    if constexpr (shears<Real>())
+        if (!separate) sh = shear_of(group_sum<D>(sxy), group_sum<D>(sxx), group_sum<D>(syy));
+    if (ok)
     {
-        Real2<Real> v = ld2(xy, i);
-        v.x += p0;
-        v.y += p1;
-        if (!isfinite((double)v.x) || !isfinite((double)v.y)) atomicOr(err, (unsigned int)ERR_NONFINITE);
-        reinterpret_cast<Real2<Real> *>(xy)[i] = v;
+        if constexpr (shears<Real>())
+#pragma unroll
+            for (int cc = 1; cc < C; cc++) f[cc] = sheared<Real>(sh, f[cc]);
+        FitSums<D, Real> sums;
+        sums.clear();
+        element_fit_sums<Real>(f, sums);
+        fit_to_model<D, Real>(sums, wedge_scale<D, Real>(g.r) * wmul, av, bv, acen, sh, q);
     }
+#pragma unroll
+    for (int k = 0; k < 5; k++) q[k] = group_sum<D>(q[k]);
+    if (!active || A != 0) return;
+    apply_step<Real>(L, xy, i, q, sh, separate, err);
+}
+
+// Two lanes per node (large 3D levels): issue slots and the FMA pipe set the pace (a node's 2 x 800
+// instructions against 287 bytes).  One depth-8 colour, float: 183 us (0.50 of the measured copy
+// bandwidth on 617 MB; 171 us without the float kernels' shear) against 600 us for a lane per element on a 12-point Gauss rule and 402 us for a lane
+// per element on the rule used now; double at depth 7: 1.06 ms against 3.5 ms, the FP64 pipe busy.  Lane s takes the four
+// elements on side s of axis 0 with the 18 grid points of its own and the node's plane in registers,
+// the stencil columns of its plane, and of the node's plane the A column (lane 0) or the B column
+// (lane 1), which the pair layout keeps as one run of 16-byte vectors per lane (PairLayout); one
+// exchange joins the two.  (Scalar stencil loads instead of the vectors: 281 us.)  Against a lane per element a node's neighbourhood is read twice instead of
+// eight times and its model summed in one shuffle round of five values instead of three.
+// stencils: the colour's block of the pair layout, the node being its jc-th of nc.
+template <typename Real>
+__device__ __forceinline__ void gs_update_pair3(const LevelPtrs<Real> &L, Real *xy, const Grid<3> &g, const int *I, bool active, int s,
+                                                unsigned int *err, int separate, const Real *stencils, int64_t jc, int64_t nc)
+{
+    using O = Ops<Real>;
+    using V = Real2<Real>;
+    using PL = PairLayout<Real>;
+    int64_t i = 0;
+    Real q[5] = {(Real)0, (Real)0, (Real)0, (Real)0, (Real)0};
+    const V zero = {(Real)0, (Real)0};
+    V P[9], Q[9], av = zero, bv = zero;
+    Real acen = (Real)0, sxy = (Real)0, sxx = (Real)0, syy = (Real)0;
+    Shear<Real> sh = {(Real)0, (Real)0};
+    const bool lo1 = I[1] > 0, hi1 = I[1] < g.r, lo2 = I[2] > 0, hi2 = I[2] < g.r;
+    const bool side = active && (s ? I[0] > 0 : I[0] < g.r);
+    if (active)
+    {
+        const int st1 = g.r + 1, st0 = st1 * st1;
+        const uint32_t iu = (uint32_t)I[0] * (uint32_t)st0 + (uint32_t)I[1] * (uint32_t)st1 + (uint32_t)I[2];
+        i = iu;
+        const V *own = reinterpret_cast<const V *>(xy) + iu;
+        const V *far = own + (s ? -st0 : st0);
+        typename PL::Vec cv[PL::G];
+        const typename PL::Vec *pc = reinterpret_cast<const typename PL::Vec *>(stencils) + 2 * jc + s;
+#pragma unroll
+        for (int v = 0; v < PL::G; v++) cv[v] = stream_load(pc + 2 * v * nc);
+        if (side && lo1 && hi1 && lo2 && hi2)
+        {
+#pragma unroll
+            for (int k = 0; k < 9; k++)
+            {
+                const int o = (k / 3 - 1) * st1 + k % 3 - 1;
+                P[k] = own[o];
+                Q[k] = far[o];
+            }
+        }
+        else
+        {
+#pragma unroll
+            for (int k = 0; k < 9; k++)
+            {
+                const int o1 = k / 3 - 1, o2 = k % 3 - 1, o = o1 * st1 + o2;
+                const bool in = (o1 < 0 ? lo1 : o1 > 0 ? hi1 : true) && (o2 < 0 ? lo2 : o2 > 0 ? hi2 : true);
+                P[k] = zero;
+                Q[k] = zero;
+                if (in) P[k] = own[o];
+                if (in && side) Q[k] = far[o];
+            }
+        }
+        // one partial sum per row of a plane: the columns cancel to a small gradient
+        V ev = zero;
+#pragma unroll
+        for (int o1 = 0; o1 < 3; o1++)
+        {
+            V ar = zero, br = zero, cr = zero;
+#pragma unroll
+            for (int o2 = 0; o2 < 3; o2++)
+            {
+                const int k = 3 * o1 + o2;
+                ar = O::fma(PL::at(cv, k), Q[k], ar);
+                br = O::fma(PL::at(cv, 9 + k), Q[k], br);
+                cr = O::fma(PL::at(cv, 18 + k), P[k], cr);
+            }
+            ev = O::add(ev, cr);
+            av = O::add(av, ar);
+            bv = O::add(bv, br);
+        }
+        if (s) bv = O::add(bv, ev);
+        else
+        {
+            av = O::add(av, ev);
+            acen = PL::at(cv, 18 + 4);
+        }
+        const V mid = P[4];
+#pragma unroll
+        for (int k = 0; k < 9; k++)
+        {
+            if (k != 4) P[k] = O::sub(P[k], mid);
+            Q[k] = O::sub(Q[k], mid);
+        }
+        if constexpr (shears<Real>())
+        {
+            const V d1 = hi1 ? P[7] : P[1], d2 = hi2 ? P[5] : P[3];
+            sxy = O::fma(d1.x, d1.y, O::mul(d2.x, d2.y));
+            sxx = O::fma(d1.x, d1.x, O::mul(d2.x, d2.x));
+            syy = O::fma(d1.y, d1.y, O::mul(d2.y, d2.y));
+            if (side)
+            {
+                sxy = O::fma(Q[4].x, Q[4].y, sxy);
+                sxx = O::fma(Q[4].x, Q[4].x, sxx);
+                syy = O::fma(Q[4].y, Q[4].y, syy);
+            }
+        }
+    }
+    if constexpr (shears<Real>())
+        if (!separate)
+        {
+            sxy = O::add(sxy, __shfl_xor_sync(0xffffffffu, sxy, 1));
+            sxx = O::add(sxx, __shfl_xor_sync(0xffffffffu, sxx, 1));
+            syy = O::add(syy, __shfl_xor_sync(0xffffffffu, syy, 1));
+            sh = shear_of(sxy, sxx, syy);
+        }
+    if (active)
+    {
+        if constexpr (shears<Real>())
+#pragma unroll
+            for (int k = 0; k < 9; k++)
+            {
+                if (k != 4) P[k] = sheared<Real>(sh, P[k]);
+                Q[k] = sheared<Real>(sh, Q[k]);
+            }
+        FitSums<3, Real> sums;
+        sums.clear();
+        if (side)
+#pragma unroll
+            for (int e = 0; e < 4; e++)
+            {
+                const int a1 = e >> 1, a2 = e & 1;  // the element lies on the lower side of axis 1, 2
+                if (!((a1 ? lo1 : hi1) && (a2 ? lo2 : hi2))) continue;
+                V d[8];
+#pragma unroll
+                for (int c = 0; c < 8; c++)
+                {
+                    const int k = 3 * (1 + (((c >> 1) & 1) ? (a1 ? -1 : 1) : 0)) + 1 + ((c & 1) ? (a2 ? -1 : 1) : 0);
+                    d[c] = (c & 4) ? Q[k] : P[k];
+                }
+                element_fit_sums<Real>(d, sums);
+            }
+        fit_to_model<3, Real>(sums, wedge_scale<3, Real>(g.r), av, bv, acen, sh, q);
+    }
+#pragma unroll
+    for (int k = 0; k < 5; k++) q[k] = O::add(q[k], __shfl_xor_sync(0xffffffffu, q[k], 1));
+    if (!active || s) return;
+    apply_step<Real>(L, xy, i, q, sh, separate, err);
 }
 
 // Warp-per-node variant for the coarsest 3D levels, where a colour has at most a few dozen nodes
@@ -774,7 +877,7 @@ __device__ __forceinline__ void gs_update_warp3(const LevelPtrs<Real> &L, Real *
     }
     if (!active || lane != 0) return;
     const Real ax = st5[0], ay = st5[1], bx = st5[2], by = st5[3], acen = st5[4];
-    const Real sc = (Real)wedge_scale<3>(g.r) * wmul;
+    const Real sc = wedge_scale<3, Real>(g.r) * wmul;
     Real q[5];
     q[0] = h[0] * sc + acen;
     q[1] = h[1] * sc + acen;
@@ -787,7 +890,7 @@ __device__ __forceinline__ void gs_update_warp3(const LevelPtrs<Real> &L, Real *
         Real2<Real> cur = ld2(xy, i);
         cur.x += p0;
         cur.y += p1;
-        if (!isfinite((double)cur.x) || !isfinite((double)cur.y)) atomicOr(err, (unsigned int)ERR_NONFINITE);
+        if (!finite_value<Real>(cur.x) || !finite_value<Real>(cur.y)) atomicOr(err, (unsigned int)ERR_NONFINITE);
         reinterpret_cast<Real2<Real> *>(xy)[i] = cur;
     }
 }
@@ -880,7 +983,7 @@ __device__ __forceinline__ void gs_update_split3(const LevelPtrs<Real> &L, Real 
 #pragma unroll
         for (int k = 0; k < 5; k++) h[k] = (part[0][k] + part[1][k]) + part[2][k];
         const Real ax = part[3][0], ay = part[3][1], bx = part[3][2], by = part[3][3], acen = part[3][4];
-        const Real sc = (Real)wedge_scale<3>(g.r) * wmul;
+        const Real sc = wedge_scale<3, Real>(g.r) * wmul;
         Real q[5];
         q[0] = h[0] * sc + acen;
         q[1] = h[1] * sc + acen;
@@ -938,138 +1041,91 @@ __global__ void __launch_bounds__(128 * NPB) gs_colour_split3_batch_kernel(const
     gs_split3_body<Real, NPB>(b.L, col, cbBase, b.err, b.separate, b.kexp, blockIdx.x);
 }
 
-template <int D, typename Real>
-__device__ __forceinline__ void gs_update_lanes(const LevelPtrs<Real> &L, const Grid<D> &g, const Colour<D> &col, int64_t j,
-                                                bool active, int A, unsigned int *err)
+// lanes per node of the colour kernels of the large levels
+template <int D, bool Pair>
+__host__ __device__ constexpr int lanes_per_node() { return Pair ? 2 : 1 << D; }
+
+// Resident blocks of 128 threads asked of the compiler.  Float pairs: 5 blocks (95 registers) 171 us a
+// depth-8 colour (before the shear), 4 blocks 178, 6 blocks 174; float lanes in 4D: 5 blocks 80 us a depth-5 colour, 2
+// blocks 137, 6 blocks 80.  Double is bound by the FP64 pipe at any occupancy.
+template <int D, typename Real, bool Pair>
+constexpr int lanes_min_blocks()
 {
-    int I[D];
-    if (active) col.node(j, I);
-    else
-        for (int d = 0; d < D; d++) I[d] = 0;
-    gs_update_lanes_at<D, Real>(L, L.xy, g, I, active, A, err);
+    if (sizeof(Real) == 8) return 2;
+    return D == 3 ? (Pair ? 5 : 6) : 5;
 }
 
-// Launch geometry without 64-bit index division: block = (128 >> D) nodes along the last axis
-// times 2^D lanes; grid.y = the colour's count on axis D-2; grid.z = the counts on the remaining
-// leading axes.
-// 3D float: cap registers at 48 (10 resident blocks, 40 warps per SM instead of 32 at 64 registers)
-template <int D, typename Real>
-constexpr int lanes_min_blocks() { return (D == 3 && sizeof(Real) == 4) ? 10 : 1; }
-
-template <int D, typename Real, bool Packed, int TPB, bool Stage = false>
-__device__ __forceinline__ void gs_lanes_body(const LevelPtrs<Real> &L, const Colour<D> &col, int64_t cbBase, unsigned int *err,
-                                              int separate, int bx, int by, int bz)
+template <int D, typename Real, bool Pair>
+__device__ __forceinline__ void gs_node_lanes(const LevelPtrs<Real> &L, const Grid<D> &g, const int *I, bool active, int lane, unsigned int *err,
+                                              int separate, const Colour<D> &col, int64_t cbBase, int64_t jc)
 {
+    if constexpr (Pair)
+    {
+        // a colour's block starts after 27 values per node of the colours before it
+        gs_update_pair3<Real>(L, L.xy, g, I, active, lane, err, separate, L.Acb + cbBase / 27 * PairLayout<Real>::kNode, jc, col.n);
+        return;
+    }
+    const Real *Ac = L.Acb ? L.Acb + cbBase : nullptr, *Bc = L.Bcb ? L.Bcb + cbBase : nullptr;
+    if constexpr (!Pair) gs_update_lanes_at<D, Real>(L, L.xy, g, I, active, lane, err, separate, Ac, Bc, jc, col.n);
+}
+
+// One colour, groups of lanes along the colour's nodes of the last two axes: grid.x = blocks of
+// TPB / lanes nodes over the cnt[D-2] x cnt[D-1] nodes of a plane (flat, so that only a plane's last
+// block is partly empty), by = the leading axes' node.
+template <int D, typename Real, bool Pair, int TPB>
+__device__ __forceinline__ void gs_lanes_body(const LevelPtrs<Real> &L, const Colour<D> &col, int64_t cbBase, unsigned int *err,
+                                              int separate, int bx, int by)
+{
+    constexpr int LPN = lanes_per_node<D, Pair>(), NPB = TPB / LPN;
     Grid<D> g(L.level);
-    constexpr int NPB = TPB >> D;
-    const int A = threadIdx.x & ((1 << D) - 1);
-    const int tl = bx * NPB + (threadIdx.x >> D);
+    const uint32_t plane = (uint32_t)(col.cnt[D - 2] * col.cnt[D - 1]), c1 = (uint32_t)col.cnt[D - 1];
+    const uint32_t p = (uint32_t)bx * NPB + threadIdx.x / LPN;
     int I[D];
-    I[D - 1] = 2 * tl + col.par[D - 1];
-    I[D - 2] = 2 * by + col.par[D - 2];
-    if constexpr (D == 3) I[0] = 2 * bz + col.par[0];
+    const uint32_t j1 = p / c1;
+    I[D - 1] = 2 * (int)(p - j1 * c1) + col.par[D - 1];
+    I[D - 2] = 2 * (int)j1 + col.par[D - 2];
+    if constexpr (D == 3) I[0] = 2 * by + col.par[0];
     else
     {
-        I[1] = 2 * (bz % col.cnt[1]) + col.par[1];
-        I[0] = 2 * (bz / col.cnt[1]) + col.par[0];
+        I[1] = 2 * (by % col.cnt[1]) + col.par[1];
+        I[0] = 2 * (by / col.cnt[1]) + col.par[0];
     }
-    // index of the node in the colour (axis 0 slowest)
-    const int64_t jc = ((int64_t)bz * col.cnt[D - 2] + by) * col.cnt[D - 1] + tl;
-    const Real *Ac = L.Acb ? L.Acb + cbBase : nullptr, *Bc = L.Bcb ? L.Bcb + cbBase : nullptr;
-    if constexpr (D == 3 && Stage)
-        if (Ac)
-        {
-            // stage the row's 3 x 3 x W neighbourhood and its nodes' stencil columns (every thread of
-            // the block takes part; Ac is the same for the whole block)
-            constexpr int W = 2 * NPB + 1, S = Dims<3>::S;
-            __shared__ Real2<Real> tile[9 * W];
-            __shared__ Real As[S * NPB], Bs[S * NPB];
-            const int x0 = 2 * bx * NPB + col.par[2] - 1, y0 = I[1] - 1, z0 = I[0] - 1;
-            for (int k = threadIdx.x; k < 9 * W; k += TPB)
-            {
-                const int lz = k / (3 * W), ly = (k / W) % 3, lx = k % W;
-                const int gz = z0 + lz, gy = y0 + ly, gx = x0 + lx;
-                if (gz >= 0 && gz <= g.r && gy >= 0 && gy <= g.r && gx >= 0 && gx <= g.r)
-                    tile[k] = ld2(L.xy, ((int64_t)gz * (g.r + 1) + gy) * (g.r + 1) + gx);
-            }
-            const int nrow = min(NPB, col.cnt[2] - bx * NPB);  // the block's nodes in the colour
-            const int64_t jc0 = ((int64_t)bz * col.cnt[1] + by) * col.cnt[2] + (int64_t)bx * NPB;
-            for (int k = threadIdx.x; k < S * NPB; k += TPB)
-            {
-                const int o = k / NPB, t = k - o * NPB;
-                if (t < nrow)
-                {
-                    As[k] = Ac[(int64_t)o * col.n + jc0 + t];
-                    Bs[k] = Bc[(int64_t)o * col.n + jc0 + t];
-                }
-            }
-            __syncthreads();
-            LaneStage<Real> stg;
-            stg.tile = tile;
-            stg.t = tl - bx * NPB;
-            stg.tcentre = 4 * W + 2 * stg.t + 1;
-            stg.As = As;
-            stg.Bs = Bs;
-            stg.npb = NPB;
-            gs_update_lanes_at<D, Real, Packed, true, W>(L, L.xy, g, I, tl < col.cnt[D - 1], A, err, separate, Ac, Bc, jc,
-                                                        col.n, (Real)1, stg);
-            return;
-        }
-    gs_update_lanes_at<D, Real, Packed>(L, L.xy, g, I, tl < col.cnt[D - 1], A, err, separate, Ac, Bc, jc, col.n);
+    gs_node_lanes<D, Real, Pair>(L, g, I, p < plane, threadIdx.x % LPN, err, separate, col, cbBase, (int64_t)by * plane + p);
 }
 
-template <int D, typename Real, int MinBlocks = lanes_min_blocks<D, Real>(), bool Packed = false, bool Stage = false>
-__global__ void __launch_bounds__(kThreads, MinBlocks) gs_colour_lanes_kernel(LevelPtrs<Real> L, Colour<D> col,
-                                                                              int64_t cbBase, unsigned int *err,
-                                                                              int separate)
+template <int D, typename Real, bool Pair>
+__global__ void __launch_bounds__(kThreads, lanes_min_blocks<D, Real, Pair>())
+    gs_colour_lanes_kernel(LevelPtrs<Real> L, Colour<D> col, int64_t cbBase, unsigned int *err, int separate)
 {
-    gs_lanes_body<D, Real, Packed, kThreads, Stage>(L, col, cbBase, err, separate, blockIdx.x, blockIdx.y, blockIdx.z);
+    gs_lanes_body<D, Real, Pair, kThreads>(L, col, cbBase, err, separate, blockIdx.x, blockIdx.y);
 }
 
 // One colour of an adaptive level: the colour's active nodes from its list (colour-local indices),
-// 2^Dim lanes per node as gs_colour_lanes_kernel, each node's update computed the same way
-template <int D, typename Real, int MinBlocks = lanes_min_blocks<D, Real>(), bool Packed = false>
-__global__ void __launch_bounds__(kThreads, MinBlocks) gs_colour_lanes_list_kernel(LevelPtrs<Real> L, Colour<D> col,
-                                                                                   int64_t cbBase, const int *list, int count,
-                                                                                   unsigned int *err, int separate)
+// each node's update computed the same way
+template <int D, typename Real, bool Pair>
+__global__ void __launch_bounds__(kThreads, lanes_min_blocks<D, Real, Pair>())
+    gs_colour_lanes_list_kernel(LevelPtrs<Real> L, Colour<D> col, int64_t cbBase, const int *list, int count, unsigned int *err,
+                                int separate)
 {
-    constexpr int NPB = kThreads >> D;
+    constexpr int LPN = lanes_per_node<D, Pair>(), NPB = kThreads / LPN;
     Grid<D> g(L.level);
-    const int A = threadIdx.x & ((1 << D) - 1);
-    const int k = blockIdx.x * NPB + (threadIdx.x >> D);
+    const int k = blockIdx.x * NPB + threadIdx.x / LPN;
     const bool active = k < count;
     const int64_t jc = active ? list[k] : 0;
     int I[D];
     col.node(jc, I);
-    const Real *Ac = L.Acb ? L.Acb + cbBase : nullptr, *Bc = L.Bcb ? L.Bcb + cbBase : nullptr;
-    gs_update_lanes_at<D, Real, Packed>(L, L.xy, g, I, active, A, err, separate, Ac, Bc, jc, col.n);
+    gs_node_lanes<D, Real, Pair>(L, g, I, active, threadIdx.x % LPN, err, separate, col, cbBase, jc);
 }
 
-// the same colour of every reconstruction of a lockstep batch (3D): block = TPB threads (TPB / 8
-// nodes along the last axis), grid.z = reconstruction x the colour's count on axis 0
-template <typename Real, int TPB, int MinBlocks, bool Packed>
-__global__ void __launch_bounds__(TPB, MinBlocks) gs_colour_lanes_batch_kernel(const BatchJob<Real> *jobs, Colour<3> col,
-                                                                               int64_t cbBase)
+// the same colour of every reconstruction of a lockstep batch (3D): block = TPB threads, grid.y =
+// reconstruction x the colour's count on axis 0
+template <typename Real, int TPB, bool Pair>
+__global__ void __launch_bounds__(TPB, lanes_min_blocks<3, Real, Pair>() * kThreads / TPB)
+    gs_colour_lanes_batch_kernel(const BatchJob<Real> *jobs, Colour<3> col, int64_t cbBase)
 {
-    const int m = blockIdx.z / col.cnt[0], bz = blockIdx.z - m * col.cnt[0];
+    const int m = blockIdx.y / col.cnt[0], by = blockIdx.y - m * col.cnt[0];
     const BatchJob<Real> &b = jobs[m];
-    gs_lanes_body<3, Real, Packed, TPB>(b.L, col, cbBase, b.err, b.separate, blockIdx.x, blockIdx.y, bz);
-}
-
-// Flat variant: consecutive groups of 2^D threads take consecutive nodes of the colour (32-bit
-// decomposition), so no block row is left partly empty.
-template <int D, typename Real>
-__global__ void __launch_bounds__(kThreads) gs_colour_flat_kernel(LevelPtrs<Real> L, Colour<D> col, unsigned int *err, int separate)
-{
-    Grid<D> g(L.level);
-    const int A = threadIdx.x & ((1 << D) - 1);
-    const int64_t j = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> D;
-    const bool active = j < col.n;
-    int I[D];
-    if (active) col.node(j, I);
-    else
-        for (int d = 0; d < D; d++) I[d] = 0;
-    gs_update_lanes_at<D, Real>(L, L.xy, g, I, active, A, err, separate);
+    gs_lanes_body<3, Real, Pair, TPB>(b.L, col, cbBase, b.err, b.separate, blockIdx.x, by);
 }
 
 // All sweeps of a small level in one thread block: the colours follow each other behind a block
@@ -1334,7 +1390,7 @@ __device__ __forceinline__ void gs_tiny_body(const LevelPtrs<Real> &L, int iters
             }
             if (apply)
             {
-                const Real sc = (Real)wedge_scale<3>(R) * wmul;
+                const Real sc = wedge_scale<3, Real>(R) * wmul;
                 Real q[5];
                 q[0] = h[0] * sc + sv[4];
                 q[1] = h[1] * sc + sv[4];
@@ -1475,7 +1531,7 @@ __device__ __forceinline__ void gs_tiny0_body(const LevelPtrs<Real> &L, int iter
                     h[k] = (part[0][k] + part[1][k]) + part[2][k];
                     sv[k] = part[3][k];
                 }
-                const Real sc = (Real)wedge_scale<3>(1) * wmul;
+                const Real sc = wedge_scale<3, Real>(1) * wmul;
                 Real q[5];
                 q[0] = h[0] * sc + sv[4];
                 q[1] = h[1] * sc + sv[4];
@@ -1658,7 +1714,7 @@ __device__ __forceinline__ void gs_tiny1_cluster_body(const LevelPtrs<Real> &L, 
                 for (int w2 = 1; w2 < incCnt[c][warp]; w2++)
 #pragma unroll
                     for (int k = 0; k < 5; k++) h[k] += part[warp + w2][k];
-                const Real sc = (Real)wedge_scale<3>(R) * wmul;
+                const Real sc = wedge_scale<3, Real>(R) * wmul;
                 Real q[5];
                 q[0] = h[0] * sc + sv[4];
                 q[1] = h[1] * sc + sv[4];
@@ -1894,7 +1950,7 @@ __device__ __forceinline__ void gs_cluster_body(const LevelPtrs<Real> &L, int it
                     }
                     const int ed = ((I[0] > 0 ? I[0] - 1 : 0) * R + (I[1] > 0 ? I[1] - 1 : 0)) * R + (I[2] > 0 ? I[2] - 1 : 0);
                     const Real *sv = part + 10 * ed + 5;
-                    const Real sc = (Real)wedge_scale<3>(R) * wmul;
+                    const Real sc = wedge_scale<3, Real>(R) * wmul;
                     Real q[5];
                     q[0] = h[0] * sc + sv[4];
                     q[1] = h[1] * sc + sv[4];
@@ -2016,7 +2072,7 @@ __global__ void __launch_bounds__(kThreads) gn_matvec_kernel(LevelPtrs<Real> L, 
         gather_element<D, Real>(g, nc, i, A, dxy, dx, dy);
         element_gn<D, Real>(x, y, dx, dy, A, s);
     }
-    const Real sc = (Real)wedge_scale<D>(g.r);
+    const Real sc = wedge_scale<D, Real>(g.r);
     Real ox = s[0] * sc, oy = s[1] * sc;
     constexpr int S = Dims<D>::S;
     for (int o = 0; o < S; o++)
@@ -2161,14 +2217,11 @@ __global__ void f2d_kernel(const float *in, double *out, int64_t n)
 
 inline unsigned int blocks_for(int64_t n, int t = kThreads) { return (unsigned int)((n + t - 1) / t); }
 
-int g_lanes_variant = 1;  // 0: scalar float element fit in the lane kernel, 1: packed
 int g_cluster_levels = 0;  // 1: 3D level 2 in double-float by gs_cluster_kernel (8 / 16: that cluster size)
 int g_cluster_blocks = 8;  // the cluster size chosen by prepare_cluster_kernels
 int g_tiny_levels = 1;    // 1: 3D levels 0-1 by gs_tiny0_kernel / gs_tiny1_kernel, 2: level 0 by the one-warp
                           // gs_tiny_kernel, 3: level 1 by the one-block gs_tiny_kernel, 0: by the block
                           // kernels of gs_level_kernel
-int g_gs_variant = 1;  // 0: one thread per node, 1: 2^D lanes per node (row grid), 2: 2^D lanes per node (flat grid),
-                       // 4: as 1 without the point-split update of the small 3D levels
 
 }  // namespace
 
@@ -2213,63 +2266,34 @@ void launch_gs_colour(const LevelPtrs<Real> &L, int colour, unsigned int *err, c
     Colour<D> col(g, colour);
     if (col.n == 0) return;
     if constexpr (D == 3)
-        if (g_gs_variant != 0 && g_gs_variant != 4 && col.n <= kSplitMaxColourNodes)
+        if (col.n <= kSplitMaxColourNodes)
         {
             // small levels: point-split update, 128 threads per node
             gs_colour_split3_kernel<Real><<<(unsigned)((col.n + kSplitNodes - 1) / kSplitNodes), 128 * kSplitNodes, 0, s>>>(
                 L, col, colour_block_base<D>(g, colour), err, separate);
             return;
         }
-    if (L.alist)
-    {
-        // adaptive level: only the colour's active nodes
-        const int count = L.aoff[colour + 1] - L.aoff[colour];
-        if (count == 0) return;
-        constexpr int NPB = kThreads >> D;
-        const unsigned nb = (unsigned)((count + NPB - 1) / NPB);
-        const int64_t cb = colour_block_base<D>(g, colour);
-        const int *list = L.alist + L.aoff[colour];
-        if constexpr (std::is_same<Real, float>::value)
-            if (g_lanes_variant != 0)
-            {
-                gs_colour_lanes_list_kernel<D, Real, D == 3 ? 9 : 1, true><<<nb, kThreads, 0, s>>>(L, col, cb, list, count, err, separate);
-                return;
-            }
-        gs_colour_lanes_list_kernel<D, Real><<<nb, kThreads, 0, s>>>(L, col, cb, list, count, err, separate);
-        return;
-    }
-    if (g_gs_variant == 0) gs_colour_kernel<D, Real><<<blocks_for(col.n), kThreads, 0, s>>>(L, col, err, separate);
-    else if (g_gs_variant == 2)
-        gs_colour_flat_kernel<D, Real><<<blocks_for(col.n << D), kThreads, 0, s>>>(L, col, err, separate);
-    else
-    {
-        constexpr int NPB = kThreads >> D;
-        dim3 grid((unsigned)((col.cnt[D - 1] + NPB - 1) / NPB), (unsigned)col.cnt[D - 2],
-                  (unsigned)(D == 3 ? col.cnt[0] : col.cnt[0] * col.cnt[1]));
-        const int64_t cb = colour_block_base<D>(g, colour);
-        // float: the element integrals on the packed two-wide FP32 instructions (3D: 0.614 against
-        // 0.680 ms per depth-8 colour; registers capped at 56, 9 resident blocks, where the
-        // scalar fit ran best at 48); EPR_LANES_VARIANT=0 selects the scalar fit
-        // (EPR_LANES_VARIANT 2 and 3: the block's row of nodes staged in shared memory, 9 or 8
-        // resident blocks: 0.741 and 0.785 against 0.601 ms per depth-8 colour -- the kernel is
-        // bound by instruction issue, and the staging adds instructions and a block barrier)
-        if constexpr (std::is_same<Real, float>::value)
-            if (g_lanes_variant != 0)
-            {
-                if (g_lanes_variant == 2)
-                    gs_colour_lanes_kernel<D, Real, D == 3 ? 9 : 1, true, true><<<grid, kThreads, 0, s>>>(L, col, cb, err, separate);
-                else if (g_lanes_variant == 3)
-                    gs_colour_lanes_kernel<D, Real, D == 3 ? 8 : 1, true, true><<<grid, kThreads, 0, s>>>(L, col, cb, err, separate);
-                else
-                    gs_colour_lanes_kernel<D, Real, D == 3 ? 9 : 1, true><<<grid, kThreads, 0, s>>>(L, col, cb, err, separate);
-                return;
-            }
-        gs_colour_lanes_kernel<D, Real><<<grid, kThreads, 0, s>>>(L, col, cb, err, separate);
-    }
+    const int64_t cb = colour_block_base<D>(g, colour);
+    auto launch = [&](auto pair) {
+        constexpr bool Pair = decltype(pair)::value;
+        constexpr int NPB = kThreads / lanes_per_node<D, Pair>();
+        if (L.alist)
+        {
+            // adaptive level: only the colour's active nodes
+            const int count = L.aoff[colour + 1] - L.aoff[colour];
+            if (count > 0)
+                gs_colour_lanes_list_kernel<D, Real, Pair><<<blocks_for(count, NPB), kThreads, 0, s>>>(L, col, cb, L.alist + L.aoff[colour],
+                                                                                                      count, err, separate);
+            return;
+        }
+        dim3 grid(blocks_for((int64_t)col.cnt[D - 2] * col.cnt[D - 1], NPB), (unsigned)(D == 3 ? col.cnt[0] : col.cnt[0] * col.cnt[1]));
+        gs_colour_lanes_kernel<D, Real, Pair><<<grid, kThreads, 0, s>>>(L, col, cb, err, separate);
+    };
+    if constexpr (D == 3)
+        if (pair_level<D>(L.level) && L.Acb) return launch(std::true_type{});
+    launch(std::false_type{});
 }
 
-void set_gs_variant(int v) { g_gs_variant = v; }
-void set_lanes_variant(int v) { g_lanes_variant = v; }
 void set_tiny_levels(int v) { g_tiny_levels = v; }
 void set_cluster_levels(int v) { g_cluster_levels = v; }
 bool cluster_level(int level, bool isDF) { return g_cluster_levels && isDF && level == 2; }
@@ -2387,7 +2411,7 @@ int launch_gs_sweeps(const LevelPtrs<Real> &L, int iters, unsigned int *err, cud
         // against 234 ms double for the level's 2560 sweeps at depth 8); resolution 2 takes a warp
         // per node (13 against 16 ms float, 145 against 182 ms double)
         if constexpr (D == 3)
-            if (g_gs_variant != 4 && colour0 == 1)
+            if (colour0 == 1)
             {
                 // 128 threads per node: the tiny levels, where the update latency sets the pace
                 const int threads = (int)colour0 * 128;
@@ -2638,22 +2662,25 @@ void launch_tiny_batch(const BatchJob<Real> *jobs, int level, int count, cudaStr
     else gs_tiny1_batch_kernel<Real><<<2 * count, 128, 0, s>>>(jobs);
 }
 
-template <typename Real, int TPB>
-static void launch_lanes_batch(const BatchJob<Real> *jobs, const Grid<3> &g, const Colour<3> &col, int64_t cb, int count,
-                               cudaStream_t s)
+template <typename Real, int TPB, bool Pair>
+static void launch_lanes_batch_as(const BatchJob<Real> *jobs, const Colour<3> &col, int64_t cb, int count, cudaStream_t s)
 {
-    constexpr bool kFloat = std::is_same<Real, float>::value;
-    // float: the packed fit with the solo kernel's register cap (9 blocks of 128 threads per SM)
-    constexpr int MinBlocks = kFloat ? (TPB == 64 ? 18 : TPB == 128 ? 9 : 4) : 1;
-    constexpr int NPB = TPB >> 3;
-    // grid.z = reconstruction x axis-0 count, at most 65,535: chunks of reconstructions
+    constexpr int NPB = TPB / lanes_per_node<3, Pair>();
+    // grid.y = reconstruction x axis-0 count, at most 65,535: chunks of reconstructions
     const int per = std::max(1, 65535 / col.cnt[0]);
     for (int m0 = 0; m0 < count; m0 += per)
     {
         const int cnt = std::min(per, count - m0);
-        dim3 grid((unsigned)((col.cnt[2] + NPB - 1) / NPB), (unsigned)col.cnt[1], (unsigned)(cnt * col.cnt[0]));
-        gs_colour_lanes_batch_kernel<Real, TPB, MinBlocks, kFloat><<<grid, TPB, 0, s>>>(jobs + m0, col, cb);
+        dim3 grid(blocks_for((int64_t)col.cnt[1] * col.cnt[2], NPB), (unsigned)(cnt * col.cnt[0]));
+        gs_colour_lanes_batch_kernel<Real, TPB, Pair><<<grid, TPB, 0, s>>>(jobs + m0, col, cb);
     }
+}
+template <typename Real, int TPB>
+static void launch_lanes_batch(const BatchJob<Real> *jobs, int level, const Colour<3> &col, int64_t cb, int count,
+                               cudaStream_t s)
+{
+    if (pair_level<3>(level)) launch_lanes_batch_as<Real, TPB, true>(jobs, col, cb, count, s);
+    else launch_lanes_batch_as<Real, TPB, false>(jobs, col, cb, count, s);
 }
 
 template <typename Real, int NPB>
@@ -2686,9 +2713,9 @@ void launch_colour_batch(const BatchJob<Real> *jobs, int level, int colour, int 
     if constexpr (std::is_same<Real, df>::value) return;  // double-float levels are 3D levels <= 3
     else
     {
-        if (tile == 0) launch_lanes_batch<Real, 64>(jobs, g, col, cb, count, s);
-        else if (tile == 2) launch_lanes_batch<Real, 256>(jobs, g, col, cb, count, s);
-        else launch_lanes_batch<Real, 128>(jobs, g, col, cb, count, s);
+        if (tile == 0) launch_lanes_batch<Real, 64>(jobs, level, col, cb, count, s);
+        else if (tile == 2) launch_lanes_batch<Real, 256>(jobs, level, col, cb, count, s);
+        else launch_lanes_batch<Real, 128>(jobs, level, col, cb, count, s);
     }
 }
 
