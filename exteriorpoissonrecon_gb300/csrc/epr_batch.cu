@@ -4,15 +4,14 @@
 // epr_batch_solve (epr_capi.cu) overlaps whole solves on host worker streams; each reconstruction
 // still issues its own ~10,000 launches, and the coarse levels of every one of them are latency
 // bound.  Here the cascadic schedule (ExteriorPoisson.h:315-409) of all members advances level by
-// level: the levels every member has (3D levels 0-1) run in one block per member, and from level 2
-// on each sweep's colour is one launch whose grid spans the colour's nodes of every member still
+// level: a small level (3D levels 0-3; 0-2 in double) is one launch of a block or cluster per member, and
+// above them each sweep's colour is one launch whose grid spans the colour's nodes of every member still
 // sweeping that level (members sorted by their sweep count, so the ones still sweeping are a
 // prefix of the table).  Every member's nodes see exactly the kernels and arithmetic of its own
 // solve (the same bodies, block shapes that change no node's arithmetic), so every member gets its
 // solo solve's bits.
 //
-// The block shapes of the colour kernels (nodes per block of the point-split kernel, threads per
-// block of the lane kernel) are the tiles an autotuner picks per level: epr_batch_tune times every
+// The block shapes of the colour kernels (threads per block) are the tiles an autotuner picks per level: epr_batch_tune times every
 // shape on the batch's own data and keeps the fastest.
 #include <algorithm>
 #include <atomic>
@@ -36,7 +35,7 @@ struct LevelPlan
     int level = 0;
     int type = kTypeFloat;
     int count = 0;             // members that relax this level
-    bool tiny = false;         // all sweeps in one launch per member (3D levels 0-1; 2 in double-float)
+    bool tiny = false;         // all sweeps of all members in one launch (the small levels)
     std::vector<int> iters;    // per job, non-increasing
     std::vector<int> members;  // per job
     size_t off = 0;            // byte offset of the BatchJob table in the image
@@ -156,9 +155,8 @@ bool make_plan(epr_batch &b)
         }
         std::stable_sort(act.begin(), act.end());
         P.count = (int)act.size();
-        // all sweeps in one launch per member: levels 0-1, and level 2 in double-float on a cluster
-        // per member (the solo solve's kernels)
-        P.tiny = b.ctxs[act[0].second]->levels[l].N <= 27 || cluster_level(l, P.type == kTypeDF);
+        // all sweeps in one launch: the small levels (the solo solve's kernels, a block or cluster per member)
+        P.tiny = P.type == kTypeDouble ? small_level<double>(l) : small_level<df>(l);
         for (auto &a : act)
         {
             P.iters.push_back(-a.first);
@@ -230,7 +228,7 @@ int64_t record(epr_batch &b)
             const BatchJob<Real> *jobs = reinterpret_cast<const BatchJob<Real> *>(b.dtab + P.off);
             if (P.tiny)
             {
-                launch_tiny_batch<Real>(jobs, l, P.count, s);
+                launch_small_level_batch<Real>(jobs, l, P.count, s);
                 launches++;
                 return;
             }
@@ -241,11 +239,6 @@ int64_t record(epr_batch &b)
                 for (int c = 0; c < 8; c++)
                 {
                     launch_colour_batch<Real>(jobs, l, c, cnt, b.tile[l], s);
-                    launches++;
-                }
-                if constexpr (std::is_same<Real, df>::value)
-                {
-                    launch_df_rescale_batch(jobs, cnt, s);
                     launches++;
                 }
             }

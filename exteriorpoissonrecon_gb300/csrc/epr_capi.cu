@@ -140,12 +140,12 @@ bool Context::sync_system32(int l)
     }
     if (lvlDF(l))
     {
-        // the point-split kernels of these levels read the stencils in natural order
+        // the small levels' kernels read the stencils in natural order
         launch_d2df(L.A64, L.Ad, (int64_t)S * L.N, stream);
         launch_d2df(L.B64, L.Bd, (int64_t)S * L.N, stream);
         return launch_ok("convert system");
     }
-    if (L.N > (dim == 3 ? 27 : 81))
+    if (dim == 3 ? !(lvl32(l) ? small_colour_level<float>(l) : small_colour_level<double>(l)) : L.N > 81)  // the levels below read the natural order
     {
         const size_t real = lvl32(l) ? sizeof(float) : sizeof(double);
         if (dim == 3 && pair_level<3>(l))
@@ -260,19 +260,23 @@ bool Context::energy(int l, double *out3)
     return true;
 }
 
-bool Context::gs(int l, int iters, int64_t persistentMaxNodes)
+bool Context::gs(int l, int iters)
 {
     bool fp32 = lvl32(l);
     if (lvlDF(l))
     {
-        launches += launch_gs_sweeps_df(level_ptrs<df>(this, l), iters, d_err, stream, P.separate, persistentMaxNodes, d_kexp);
+        if (iters > 0)
+        {
+            launch_small_level<df>(level_ptrs<df>(this, l), iters, d_err, stream, P.separate, d_kexp);
+            launches++;
+        }
         stats.node_updates += (int64_t)iters * levels[l].N;
         return launch_ok("gs");
     }
     launches += with_dim(this, [&](auto dd) {
         constexpr int D = decltype(dd)::value;
-        if (fp32) return launch_gs_sweeps<D, float>(level_ptrs<float>(this, l), iters, d_err, stream, P.separate, persistentMaxNodes);
-        return launch_gs_sweeps<D, double>(level_ptrs<double>(this, l), iters, d_err, stream, P.separate, persistentMaxNodes);
+        if (fp32) return launch_gs_sweeps<D, float>(level_ptrs<float>(this, l), iters, d_err, stream, P.separate);
+        return launch_gs_sweeps<D, double>(level_ptrs<double>(this, l), iters, d_err, stream, P.separate);
     });
     stats.node_updates += (int64_t)iters * levels[l].N;
     return launch_ok("gs");
@@ -411,12 +415,10 @@ bool Context::download_xy(int l, double *x, double *y, bool fromSolution)
 }
 
 // The relaxation sequence of the cascadic schedule (GS on every solve level, prolongation to the
-// next), captured once into a CUDA graph and replayed: it is a fixed sequence of ~2,500 launches
-// with no host interaction.  In the graph only the two coarsest levels run their sweeps inside one
-// block; the others launch one kernel per colour, which the graph issues back to back.
+// next), captured once into a CUDA graph and replayed: it is a fixed sequence of some 2,500 launches
+// (depth 8) with no host interaction, one for each small level and one for each colour of the others.
 bool Context::relax_levels(int minD, int maxD, bool useGraph)
 {
-    const int64_t graphPersistentMax = dim == 3 ? 27 : 81;
     if (useGraph && solve_graph)
     {
         launches += graph_launches;
@@ -434,9 +436,7 @@ bool Context::relax_levels(int minD, int maxD, bool useGraph)
     for (int l = minD; ok && l <= maxD; l++)
     {
         int iters = (int)std::ceil(std::pow(P.i_mult, depth - l) * P.gs_iters);
-        // the same launch configuration whether captured or not (one kernel per colour from level 2
-        // on), so that every solve of a context runs the same kernels and gives the same bits
-        ok = gs(l, iters, useGraph ? graphPersistentMax : kPersistentMaxNodes);
+        ok = gs(l, iters);
         if (ok && l < maxD) ok = prolong_add(l);
     }
     if (!capture) return ok;
@@ -668,8 +668,6 @@ epr_ctx *epr_create(int dim, int depth, const epr_params *params)
     }
     {
         std::lock_guard<std::mutex> lock(g_create_mutex);
-        if (const char *v = getenv("EPR_TINY_LEVELS")) epr::set_tiny_levels(atoi(v));
-        if (const char *v = getenv("EPR_CLUSTER_LEVELS")) epr::set_cluster_levels(atoi(v));
         static uint64_t prepared = 0;  // devices whose kernel attributes are set
         if (p.device >= 0 && p.device < 64 && !(prepared & (1ull << p.device)))
         {
@@ -1064,8 +1062,7 @@ int epr_time_kernel(epr_ctx *ctx, const char *kernel, int level, int reps, doubl
     auto run = [&]() {
         if (dfLevel)
         {
-            // one colour of a double-float level (its point-split kernel on pairs of floats)
-            epr::launch_gs_colour_df(epr::level_ptrs<epr::df>(ctx, level), 0, ctx->d_err, ctx->stream, ctx->d_kexp);
+            epr::launch_small_colour<epr::df>(epr::level_ptrs<epr::df>(ctx, level), 0, ctx->d_err, ctx->stream, 0, ctx->d_kexp);
             return;
         }
         epr::with_dim(ctx, [&](auto dd) {

@@ -123,7 +123,7 @@ struct Context
     bool push_xy(int l);
     bool pull_xy(int l);
     bool energy(int l, double *out3);
-    bool gs(int l, int iters, int64_t persistentMaxNodes = kPersistentMaxNodes);
+    bool gs(int l, int iters);
     bool relax_levels(int minD, int maxD, bool useGraph);
     bool check_errors();
     bool prolong_add(int l);

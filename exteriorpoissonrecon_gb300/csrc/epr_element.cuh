@@ -109,43 +109,6 @@ __device__ __forceinline__ void derivative_table(const Real *f, Real *out)
     }
 }
 
-// The two steps of derivative_table separately, for callers that evaluate the other-axis points
-// one at a time (fewer live registers in 4D): the A-differences interpolated along B ...
-template <int D, int K, bool AisP, typename Real>
-__device__ __forceinline__ void derivative_partial(const Real *f, Real (&t)[2][1 << (D - 2)])
-{
-    using Cp = Component<D, K>;
-    constexpr int NO = 1 << Cp::M;
-    Real dif[2][NO];
-#pragma unroll
-    for (int bB = 0; bB < 2; bB++)
-#pragma unroll
-        for (int bo = 0; bo < NO; bo++)
-        {
-            int c1 = AisP ? Cp::corner(1, bB, bo) : Cp::corner(bB, 1, bo);
-            int c0 = AisP ? Cp::corner(0, bB, bo) : Cp::corner(bB, 0, bo);
-            dif[bB][bo] = f[c1] - f[c0];
-        }
-#pragma unroll
-    for (int g = 0; g < 2; g++)
-#pragma unroll
-        for (int bo = 0; bo < NO; bo++) t[g][bo] = hat2<Real>(0, g) * dif[0][bo] + hat2<Real>(1, g) * dif[1][bo];
-}
-
-// ... and then at the other-axis Gauss point go (the same operations as derivative_table)
-template <int M, typename Real>
-__device__ __forceinline__ Real derivative_at(const Real *t, int go)
-{
-    if constexpr (M == 1) return hat3<Real>(0, go) * t[0] + hat3<Real>(1, go) * t[1];
-    else
-    {
-        const int g0 = go / 3, g1 = go % 3;
-        Real u0 = hat3<Real>(0, g0) * t[0] + hat3<Real>(1, g0) * t[2];
-        Real u1 = hat3<Real>(0, g0) * t[1] + hat3<Real>(1, g0) * t[3];
-        return hat3<Real>(0, g1) * u0 + hat3<Real>(1, g1) * u1;
-    }
-}
-
 template <int M>
 __device__ __forceinline__ double other_weight(int go)
 {
@@ -186,219 +149,6 @@ __device__ __forceinline__ Real element_wedge(const Real *x, const Real *y)
     Real s = component_wedge<D, 0>(x, y) + component_wedge<D, 1>(x, y) + component_wedge<D, 2>(x, y);
     if constexpr (D == 4) s += component_wedge<D, 3>(x, y) + component_wedge<D, 4>(x, y) + component_wedge<D, 5>(x, y);
     return s;
-}
-
-// ---------------------------------------------------------------------------------------------
-// Quadratic-fit integrals of corner A of the element, one component (reference units):
-//   h0 = sum |U|^2, h1 = sum |V|^2, h2 = sum <U,V>, h3 = sum <W,U>, h4 = sum <W,V>
-// with U = W(phi_A, y), V = W(x, phi_A) (the derivatives of W along x_A and y_A).
-// ---------------------------------------------------------------------------------------------
-template <int D, int K, typename Real>
-__device__ __forceinline__ void component_fit(const Real *x, const Real *y, int A, Real *h)
-{
-    using Cp = Component<D, K>;
-    constexpr int M = Cp::M;
-    constexpr int NG = ipow(3, M);
-    if constexpr (M == 2)
-    {
-        // 4D: derivatives evaluated per other-axis point (same values, same summation order)
-        Real txP[2][4], txQ[2][4], tyP[2][4], tyQ[2][4];
-        derivative_partial<D, K, true>(x, txP);
-        derivative_partial<D, K, false>(x, txQ);
-        derivative_partial<D, K, true>(y, tyP);
-        derivative_partial<D, K, false>(y, tyQ);
-        const int aP = cbit<D>(A, Cp::P), aQ = cbit<D>(A, Cp::Q);
-        const Real sP = aP ? (Real)1 : (Real)-1, sQ = aQ ? (Real)1 : (Real)-1;
-        const int ao0 = cbit<D>(A, Cp::other(0)), ao1 = cbit<D>(A, Cp::other(1));
-#pragma unroll
-        for (int go = 0; go < NG; go++)
-        {
-            const Real lo = hat3<Real>(ao0, go / 3) * hat3<Real>(ao1, go % 3);
-            const Real wo = (Real)other_weight<M>(go);
-            Real xPg[2], xQg[2], yPg[2], yQg[2];
-#pragma unroll
-            for (int g = 0; g < 2; g++)
-            {
-                xPg[g] = derivative_at<M, Real>(txP[g], go);
-                xQg[g] = derivative_at<M, Real>(txQ[g], go);
-                yPg[g] = derivative_at<M, Real>(tyP[g], go);
-                yQg[g] = derivative_at<M, Real>(tyQ[g], go);
-            }
-#pragma unroll
-            for (int gp = 0; gp < 2; gp++)
-#pragma unroll
-                for (int gq = 0; gq < 2; gq++)
-                {
-                    Real w = (Real)(Gauss::W2(gp) * Gauss::W2(gq)) * wo;
-                    Real phP = sP * hat2<Real>(aQ, gq) * lo;
-                    Real phQ = sQ * hat2<Real>(aP, gp) * lo;
-                    Real xp = xPg[gq], xq = xQg[gp];
-                    Real yp = yPg[gq], yq = yQg[gp];
-                    Real W = yp * xq - xp * yq;
-                    Real U = yp * phQ - phP * yq;
-                    Real V = phP * xq - xp * phQ;
-                    Real wU = w * U, wV = w * V;
-                    h[0] += wU * U;
-                    h[1] += wV * V;
-                    h[2] += wU * V;
-                    h[3] += wU * W;
-                    h[4] += wV * W;
-                }
-        }
-        return;
-    }
-    Real xP[2 * NG], xQ[2 * NG], yP[2 * NG], yQ[2 * NG];
-    derivative_table<D, K, true>(x, xP);
-    derivative_table<D, K, false>(x, xQ);
-    derivative_table<D, K, true>(y, yP);
-    derivative_table<D, K, false>(y, yQ);
-    const int aP = cbit<D>(A, Cp::P), aQ = cbit<D>(A, Cp::Q);
-    const Real sP = aP ? (Real)1 : (Real)-1, sQ = aQ ? (Real)1 : (Real)-1;
-    int ao[M > 0 ? M : 1];
-#pragma unroll
-    for (int m = 0; m < M; m++) ao[m] = cbit<D>(A, Cp::other(m));
-#pragma unroll
-    for (int go = 0; go < NG; go++)
-    {
-        Real lo;
-        if constexpr (M == 1) lo = hat3<Real>(ao[0], go);
-        else lo = hat3<Real>(ao[0], go / 3) * hat3<Real>(ao[1], go % 3);
-        Real wo = (Real)other_weight<M>(go);
-#pragma unroll
-        for (int gp = 0; gp < 2; gp++)
-#pragma unroll
-            for (int gq = 0; gq < 2; gq++)
-            {
-                Real w = (Real)(Gauss::W2(gp) * Gauss::W2(gq)) * wo;
-                Real phP = sP * hat2<Real>(aQ, gq) * lo;
-                Real phQ = sQ * hat2<Real>(aP, gp) * lo;
-                Real xp = xP[gq * NG + go], xq = xQ[gp * NG + go];
-                Real yp = yP[gq * NG + go], yq = yQ[gp * NG + go];
-                Real W = yp * xq - xp * yq;
-                Real U = yp * phQ - phP * yq;
-                Real V = phP * xq - xp * phQ;
-                Real wU = w * U, wV = w * V;
-                h[0] += wU * U;
-                h[1] += wV * V;
-                h[2] += wU * V;
-                h[3] += wU * W;
-                h[4] += wV * W;
-            }
-    }
-}
-
-// The two steps of component_fit_pq3 for callers that spread a pair's three other-axis points
-// over threads: the pair's derivative tables (setup) and one point's terms (point).
-template <typename Real>
-struct PairTables
-{
-    Real xP[2], xQ[2], yP[2], yQ[2], w2, hq, hp;
-};
-
-template <typename Real>
-__device__ __forceinline__ void component_setup_pq3(const Real *x, const Real *y, int gp, int gq, PairTables<Real> &t)
-{
-    using Cp = Component<3, 0>;
-    const Real q0 = gq ? hat2<Real>(0, 1) : hat2<Real>(0, 0), q1 = gq ? hat2<Real>(1, 1) : hat2<Real>(1, 0);
-    const Real p0 = gp ? hat2<Real>(0, 1) : hat2<Real>(0, 0), p1 = gp ? hat2<Real>(1, 1) : hat2<Real>(1, 0);
-#pragma unroll
-    for (int bo = 0; bo < 2; bo++)
-    {
-        // derivative along P interpolated at Q's point gq, and along Q at P's point gp
-        t.xP[bo] = q0 * (x[Cp::corner(1, 0, bo)] - x[Cp::corner(0, 0, bo)]) + q1 * (x[Cp::corner(1, 1, bo)] - x[Cp::corner(0, 1, bo)]);
-        t.yP[bo] = q0 * (y[Cp::corner(1, 0, bo)] - y[Cp::corner(0, 0, bo)]) + q1 * (y[Cp::corner(1, 1, bo)] - y[Cp::corner(0, 1, bo)]);
-        t.xQ[bo] = p0 * (x[Cp::corner(0, 1, bo)] - x[Cp::corner(0, 0, bo)]) + p1 * (x[Cp::corner(1, 1, bo)] - x[Cp::corner(1, 0, bo)]);
-        t.yQ[bo] = p0 * (y[Cp::corner(0, 1, bo)] - y[Cp::corner(0, 0, bo)]) + p1 * (y[Cp::corner(1, 1, bo)] - y[Cp::corner(1, 0, bo)]);
-    }
-    t.w2 = gp == gq ? (gp ? (Real)(Gauss::W2(1) * Gauss::W2(1)) : (Real)(Gauss::W2(0) * Gauss::W2(0)))
-                    : (Real)(Gauss::W2(0) * Gauss::W2(1));
-    t.hq = gq ? hat2<Real>(0, 1) : hat2<Real>(0, 0);
-    t.hp = p0;
-}
-
-template <typename Real>
-__device__ __forceinline__ void component_point_pq3(const PairTables<Real> &t, int go, Real *h)
-{
-    constexpr Real kLo[3] = {hat3c<Real>(0, 0), hat3c<Real>(0, 1), hat3c<Real>(0, 2)};
-    constexpr Real kHi[3] = {hat3c<Real>(1, 0), hat3c<Real>(1, 1), hat3c<Real>(1, 2)};
-    constexpr Real kW[3] = {(Real)Gauss::W3(0), (Real)Gauss::W3(1), (Real)Gauss::W3(2)};
-    const Real lo = go == 0 ? kLo[0] : go == 1 ? kLo[1] : kLo[2];
-    const Real hi = go == 0 ? kHi[0] : go == 1 ? kHi[1] : kHi[2];
-    const Real w = t.w2 * (go == 0 ? kW[0] : go == 1 ? kW[1] : kW[2]);
-    const Real phP = (Real)-1 * t.hq * lo;
-    const Real phQ = (Real)-1 * t.hp * lo;
-    const Real xp = lo * t.xP[0] + hi * t.xP[1], xq = lo * t.xQ[0] + hi * t.xQ[1];
-    const Real yp = lo * t.yP[0] + hi * t.yP[1], yq = lo * t.yQ[0] + hi * t.yQ[1];
-    const Real W = yp * xq - xp * yq;
-    const Real U = yp * phQ - phP * yq;
-    const Real V = phP * xq - xp * phQ;
-    const Real wU = w * U, wV = w * V;
-    h[0] += wU * U;
-    h[1] += wV * V;
-    h[2] += wU * V;
-    h[3] += wU * W;
-    h[4] += wV * W;
-}
-
-// Component 0 of a 3D element in the canonical orientation (corner 0), restricted to the Gauss
-// points with the given (gp, gq): the share of one of four threads that split a component's
-// integral (the values of the points are those of component_fit).  The pair is a run-time value:
-// the A-differences are interpolated along B with the hat values of the pair's own Gauss point
-// (scalars picked from two constants), so that threads with different pairs run one instruction
-// stream and the corner arrays stay constant-indexed in registers.
-template <typename Real>
-__device__ __forceinline__ void component_fit_pq3(const Real *x, const Real *y, int gp, int gq, Real *h)
-{
-    using Cp = Component<3, 0>;
-    const Real q0 = gq ? hat2<Real>(0, 1) : hat2<Real>(0, 0), q1 = gq ? hat2<Real>(1, 1) : hat2<Real>(1, 0);
-    const Real p0 = gp ? hat2<Real>(0, 1) : hat2<Real>(0, 0), p1 = gp ? hat2<Real>(1, 1) : hat2<Real>(1, 0);
-    Real xP[2], xQ[2], yP[2], yQ[2];
-#pragma unroll
-    for (int bo = 0; bo < 2; bo++)
-    {
-        // derivative along P interpolated at Q's point gq, and along Q at P's point gp
-        xP[bo] = q0 * (x[Cp::corner(1, 0, bo)] - x[Cp::corner(0, 0, bo)]) + q1 * (x[Cp::corner(1, 1, bo)] - x[Cp::corner(0, 1, bo)]);
-        yP[bo] = q0 * (y[Cp::corner(1, 0, bo)] - y[Cp::corner(0, 0, bo)]) + q1 * (y[Cp::corner(1, 1, bo)] - y[Cp::corner(0, 1, bo)]);
-        xQ[bo] = p0 * (x[Cp::corner(0, 1, bo)] - x[Cp::corner(0, 0, bo)]) + p1 * (x[Cp::corner(1, 1, bo)] - x[Cp::corner(1, 0, bo)]);
-        yQ[bo] = p0 * (y[Cp::corner(0, 1, bo)] - y[Cp::corner(0, 0, bo)]) + p1 * (y[Cp::corner(1, 1, bo)] - y[Cp::corner(1, 0, bo)]);
-    }
-    const Real w2 = gp == gq ? (gp ? (Real)(Gauss::W2(1) * Gauss::W2(1)) : (Real)(Gauss::W2(0) * Gauss::W2(0)))
-                             : (Real)(Gauss::W2(0) * Gauss::W2(1));
-    const Real hq = gq ? hat2<Real>(0, 1) : hat2<Real>(0, 0), hp = p0;
-    constexpr Real kLo[3] = {hat3c<Real>(0, 0), hat3c<Real>(0, 1), hat3c<Real>(0, 2)};
-    constexpr Real kHi[3] = {hat3c<Real>(1, 0), hat3c<Real>(1, 1), hat3c<Real>(1, 2)};
-    constexpr Real kW[3] = {(Real)Gauss::W3(0), (Real)Gauss::W3(1), (Real)Gauss::W3(2)};
-    auto point = [&](int go) {
-        const Real lo = go == 0 ? kLo[0] : go == 1 ? kLo[1] : kLo[2];
-        const Real hi = go == 0 ? kHi[0] : go == 1 ? kHi[1] : kHi[2];
-        const Real w = w2 * (go == 0 ? kW[0] : go == 1 ? kW[1] : kW[2]);
-        const Real phP = (Real)-1 * hq * lo;
-        const Real phQ = (Real)-1 * hp * lo;
-        const Real xp = lo * xP[0] + hi * xP[1], xq = lo * xQ[0] + hi * xQ[1];
-        const Real yp = lo * yP[0] + hi * yP[1], yq = lo * yQ[0] + hi * yQ[1];
-        const Real W = yp * xq - xp * yq;
-        const Real U = yp * phQ - phP * yq;
-        const Real V = phP * xq - xp * phQ;
-        const Real wU = w * U, wV = w * V;
-        h[0] += wU * U;
-        h[1] += wV * V;
-        h[2] += wU * V;
-        h[3] += wU * W;
-        h[4] += wV * W;
-    };
-    // the three other-axis points: in double-float a rolled loop (the hat values and weights
-    // picked from constants), a third of the code of the unrolled one, for the kernels that run
-    // this fit for thousands of dependent single-node updates and are bound by instruction fetch
-    if constexpr (std::is_same<Real, df>::value)
-    {
-#pragma unroll 1
-        for (int go = 0; go < 3; go++) point(go);
-    }
-    else
-    {
-#pragma unroll
-        for (int go = 0; go < 3; go++) point(go);
-    }
 }
 
 // ---------------------------------------------------------------------------------------------

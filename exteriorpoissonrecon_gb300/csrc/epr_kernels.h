@@ -3,6 +3,7 @@
 #pragma once
 #include <cstddef>
 #include <cstdint>
+#include <type_traits>
 #include <cuda_runtime.h>
 
 #include "epr_df.cuh"
@@ -49,29 +50,30 @@ void launch_quadfit(const LevelPtrs<Real> &L, const Real *xy, double *out, cudaS
 // separate != 0: the reference's SeparateGaussSeidelSolve update (x first, then y with the new x)
 template <int D, typename Real>
 void launch_gs_colour(const LevelPtrs<Real> &L, int colour, unsigned int *err, cudaStream_t s, int separate = 0);
-// 1 (default): 3D levels 0-1 relax in gs_tiny_kernel (one warp per node-element incidence of a
-// colour); 0: in the block kernels
-void set_tiny_levels(int v);
-// 3D level 2 in double-float on one cluster launch (1; 8 or 16 fix the cluster size) or a launch
-// per colour (0, the default)
-void set_cluster_levels(int v);
-bool cluster_level(int level, bool isDF);
 // double-float levels: pairs stored as x 2^-k with k = kexp[level] (epr_df.cuh)
 void launch_df_push(const double *in, df *out, int64_t n, int *kexp, int level, cudaStream_t s);
 void launch_df_pull(const df *in, double *out, int64_t n, const int *kexp, int level, cudaStream_t s);
 void launch_d2df(const double *in, df *out, int64_t n, cudaStream_t s);
-int launch_gs_sweeps_df(const LevelPtrs<df> &L, int iters, unsigned int *err, cudaStream_t s, int separate,
-                        int64_t persistentMaxNodes, int *kexp);
-void launch_gs_colour_df(const LevelPtrs<df> &L, int colour, unsigned int *err, cudaStream_t s, int *kexp);
-// iters full sweeps (all 2^D colours in order); levels of at most persistentMaxNodes nodes run all
-// sweeps inside one thread block, larger ones launch one kernel per colour.  Returns the number of
-// kernels launched.
-constexpr int64_t kPersistentMaxNodes = 729;
+// iters full sweeps (all 2^D colours in order); the small levels run all sweeps in one launch, larger
+// ones launch one kernel per colour.  Returns the number of kernels launched.
 template <int D, typename Real>
-int launch_gs_sweeps(const LevelPtrs<Real> &L, int iters, unsigned int *err, cudaStream_t s, int separate = 0,
-                     int64_t persistentMaxNodes = kPersistentMaxNodes);
-// sets the shared-memory carve-out of the single-block level kernels (once per process, before
-// any stream capture)
+int launch_gs_sweeps(const LevelPtrs<Real> &L, int iters, unsigned int *err, cudaStream_t s, int separate = 0);
+
+// The small 3D levels (epr_small.cu).  All sweeps in one launch: levels 0-2, and level 3 but in double;
+// levels 3 and 4 in double by its per-colour launches (a lane per element leaves three of four FP64
+// units without a warp there: level 4 14.5 us a colour).
+constexpr int kSmallLevels3 = 5;
+template <typename Real>
+constexpr bool small_level(int level) { return level < 3 || (level == 3 && !std::is_same<Real, double>::value); }
+template <typename Real>
+constexpr bool small_colour_level(int level) { return level < 4 || (level == 4 && std::is_same<Real, double>::value); }
+void prepare_small_kernels();
+template <typename Real>
+void launch_small_level(const LevelPtrs<Real> &L, int iters, unsigned int *err, cudaStream_t s, int separate, int *kexp);
+template <typename Real>
+void launch_small_colour(const LevelPtrs<Real> &L, int colour, unsigned int *err, cudaStream_t s, int separate, const int *kexp);
+// sets the kernels' shared-memory limits and uploads the small levels' tables (once per device, before any
+// stream capture)
 void prepare_gs_kernels();
 template <int D, typename Real>
 void launch_gn_matvec(const LevelPtrs<Real> &L, const Real *xy, const Real *dxy, Real *out, cudaStream_t s);
@@ -129,20 +131,18 @@ struct XferJob
     void *dst = nullptr;
     int *kexp = nullptr;
 };
-// the colour kernels' block shapes a batch may pick (none changes any node's arithmetic):
-// levels whose colours have at most 125 nodes: nodes per block of the point-split kernel;
-// larger levels: threads per block of the lane kernel (8 lanes per node)
-constexpr int kSplitTiles[3] = {1, 2, 4};
+// the block shapes a batch may pick for the large levels' colour kernels (none changes any node's
+// arithmetic): threads per block.  Level 3 in double has one shape.
 constexpr int kLanesTiles[3] = {64, 128, 256};
-constexpr int kDefaultTile = 1;  // index into the tables: the solo solve's shapes (2 nodes, 128 threads)
-// all sweeps of 3D level 0 or 1 of `count` reconstructions (jobs[0..count))
+constexpr int kDefaultTile = 1;  // index into the table: the solo solve's shape (128 threads)
+// all sweeps of a small level of `count` reconstructions (jobs[0..count))
 template <typename Real>
-void launch_tiny_batch(const BatchJob<Real> *jobs, int level, int count, cudaStream_t s);
-// one colour of a level >= 2 of jobs[0..count) with the block shape kSplitTiles / kLanesTiles[tile]
+void launch_small_level_batch(const BatchJob<Real> *jobs, int level, int count, cudaStream_t s);
+// one colour of a level of jobs[0..count)
+template <typename Real>
+void launch_small_colour_batch(const BatchJob<Real> *jobs, int level, int colour, int count, cudaStream_t s);
 template <typename Real>
 void launch_colour_batch(const BatchJob<Real> *jobs, int level, int colour, int count, int tile, cudaStream_t s);
-// a new exponent for each double-float level of jobs[0..count) (once per sweep)
-void launch_df_rescale_batch(const BatchJob<df> *jobs, int count, cudaStream_t s);
 // fine += P coarse for jobs[0..count) (src coarse, dst fine)
 template <typename Real>
 void launch_prolong_add_batch(const XferJob *jobs, int coarseLevel, int count, cudaStream_t s);
