@@ -151,7 +151,7 @@ bool Context::sync_system32(int l)
         if (dim == 3 && pair_level<3>(l))
         {
             if (!L.Acb && !alloc(&L.Acb, 56 * L.N * real, "alloc colour blocks")) return false;
-            if (lvl32(l)) launch_to_pair_blocks<float>(l, L.A64, L.B64, (float *)L.Acb, stream);
+            if (lvl32(l)) launch_to_pair_blocks<float>(l, L.A32, L.B32, (float *)L.Acb, stream);
             else launch_to_pair_blocks<double>(l, L.A64, L.B64, (double *)L.Acb, stream);
             return launch_ok("convert system");
         }

@@ -86,9 +86,12 @@ void launch_prolong(int coarseLevel, const Real *coarse, Real *fine, int add, cu
 template <int D, typename Real>
 void launch_restrict(int coarseLevel, const Real *fine, Real *coarse, cudaStream_t s);
 
-// coarse = P^T fine P of a column stencil (offset-major, double), fine level -> fineLevel - 1
+// coarse = P^T fine P of a column stencil (offset-major, double), fine level -> fineLevel - 1; scratch holds
+// galerkin_scratch(fineLevel) doubles (enough for every coarser level too)
 template <int D>
-void launch_galerkin(int fineLevel, const double *Mf, double *Mc, cudaStream_t s);
+size_t galerkin_scratch(int fineLevel);
+template <int D>
+void launch_galerkin(int fineLevel, const double *Mf, double *Mc, double *scratch, cudaStream_t s);
 
 // colour-blocked copy (Real) of a natural offset-major double stencil of `level`
 template <int D, typename Real>
@@ -96,7 +99,7 @@ void launch_to_colour_blocks(int level, const double *M, Real *out, cudaStream_t
 
 // both natural stencils of a 3D level (level >= kPairLevel) -> its pair layout (PairLayout, 56 values per node)
 template <typename Real>
-void launch_to_pair_blocks(int level, const double *A, const double *B, Real *out, cudaStream_t s);
+void launch_to_pair_blocks(int level, const Real *A, const Real *B, Real *out, cudaStream_t s);
 
 // elementwise helpers
 template <typename Real>

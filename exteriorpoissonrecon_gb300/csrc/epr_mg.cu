@@ -126,10 +126,10 @@ __global__ void to_colour_blocks_kernel(int level, const double *M, ColourBlocks
     for (int o = 0; o < Dims<D>::S; o++) dst[o * n] = (Real)M[(int64_t)o * g.N + i];
 }
 
-// both natural offset-major double stencils of a 3D level -> its pair layout; one thread per lane of a
+// both natural offset-major stencils of a 3D level -> its pair layout; one thread per lane of a
 // node, grid.y = colour
 template <typename Real>
-__global__ void to_pair_blocks_kernel(int level, const double *A, const double *B, ColourBlocks<3> cb, Real *out)
+__global__ void to_pair_blocks_kernel(int level, const Real *A, const Real *B, ColourBlocks<3> cb, Real *out)
 {
     using PL = PairLayout<Real>;
     const int c = blockIdx.y;
@@ -158,7 +158,7 @@ __global__ void to_pair_blocks_kernel(int level, const double *A, const double *
                 stencil_offset<3>(o, off);
                 for (int d = 0; d < 3; d++) in = in && I[d] + off[d] >= 0 && I[d] + off[d] <= g.r;
             }
-            r[w] = in ? (Real)(m ? B : A)[(int64_t)o * g.N + i] : (Real)0;
+            r[w] = in ? (m ? B : A)[(int64_t)o * g.N + i] : (Real)0;
         }
         typename PL::Vec vec;
         if constexpr (PL::W == 4) vec = make_float4(r[0], r[1], r[2], r[3]);
@@ -765,12 +765,12 @@ __global__ void biquad_finish_kernel(const double *partial, int nblocks, double 
 }  // namespace
 
 template <typename Real>
-void launch_to_pair_blocks(int level, const double *A, const double *B, Real *out, cudaStream_t s)
+void launch_to_pair_blocks(int level, const Real *A, const Real *B, Real *out, cudaStream_t s)
 {
     ColourBlocks<3> cb = colour_blocks<3>(level);
     to_pair_blocks_kernel<Real><<<dim3(blocks(2 * cb.count[0]), 8), kThreads, 0, s>>>(level, A, B, cb, out);
 }
-template void launch_to_pair_blocks<float>(int, const double *, const double *, float *, cudaStream_t);
+template void launch_to_pair_blocks<float>(int, const float *, const float *, float *, cudaStream_t);
 template void launch_to_pair_blocks<double>(int, const double *, const double *, double *, cudaStream_t);
 
 template <int D, typename Real>
@@ -809,6 +809,7 @@ struct MGHierarchy
     int mode = -1;  // precision and double band the levels were allocated for
     std::vector<MGLevel> L;
     double *x64 = nullptr, *b64 = nullptr;  // finest-level double vectors (solution, right-hand side)
+    double *scratch = nullptr;              // of the Galerkin products
 };
 
 void release_mg(Context &c)
@@ -820,6 +821,7 @@ void release_mg(Context &c)
     }
     c.release(c.mg->x64);
     c.release(c.mg->b64);
+    c.release(c.mg->scratch);
     delete c.mg;
     c.mg = nullptr;
 }
@@ -857,7 +859,9 @@ static bool mg_prepare(Context &c, int top)
             return false;
     }
     const int64_t N = h.L[top].N;
-    return c.alloc((void **)&h.x64, sizeof(double) * N, "alloc mg x64") && c.alloc((void **)&h.b64, sizeof(double) * N, "alloc mg b64");
+    const size_t scratch = top == 0 ? 0 : c.dim == 3 ? galerkin_scratch<3>(top) : galerkin_scratch<4>(top);
+    return c.alloc((void **)&h.x64, sizeof(double) * N, "alloc mg x64") && c.alloc((void **)&h.b64, sizeof(double) * N, "alloc mg b64") &&
+           c.alloc((void **)&h.scratch, sizeof(double) * scratch, "alloc mg scratch");
 }
 
 template <typename F>
@@ -883,7 +887,7 @@ static bool mg_build(Context &c, int top, int lo)
     mg_dim(c, [&](auto dd) {
         constexpr int D = decltype(dd)::value;
         if (lo < top)
-            for (int l = top; l > 0; l--) launch_galerkin<D>(l, h.L[l].M64, h.L[l - 1].M64, c.stream);
+            for (int l = top; l > 0; l--) launch_galerkin<D>(l, h.L[l].M64, h.L[l - 1].M64, h.scratch, c.stream);
         for (int l = std::max(lo, 1); l <= top; l++)
         {
             with_real(h.L[l].f32, [&](auto rv) {
@@ -894,7 +898,7 @@ static bool mg_build(Context &c, int top, int lo)
             });
             c.launches++;
         }
-        c.launches += (lo < top) ? top : 0;
+        c.launches += (lo < top) ? top * D : 0;
         return 0;
     });
     return c.launch_ok("mg hierarchy");

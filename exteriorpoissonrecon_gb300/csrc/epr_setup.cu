@@ -20,6 +20,7 @@
 // Splats are deterministic gathers: samples are sorted by the Morton key of their cell, so the
 // samples of any coarser cell are one contiguous range; every output vertex is reduced by one
 // warp in a fixed order.
+#include <algorithm>
 #include <cmath>
 #include <cstdio>
 #include <string>
@@ -576,7 +577,7 @@ __device__ double samples_per_cell(const DensityGrids<D> &G, int t, const double
 {
     double count;
     density_interp<D, 1>(G, t, p, &count);
-    return count / (double)(1u << ((t - 1) * (D - 2)));
+    return count * (1. / (double)(1u << ((t - 1) * (D - 2))));  // a power of two
 }
 
 template <int D>
@@ -605,29 +606,39 @@ __device__ double est_depth_raw(const DensityGrids<D> &G, int maxT, const double
     return d1 + log(tg / s1) / log(s2 / s1);
 }
 
-// ascending eigenvalues of a symmetric D x D matrix (cyclic Jacobi)
+// ascending eigenvalues of a symmetric D x D matrix (cyclic Jacobi, until what is left off the diagonal
+// cannot change a bit of it; every loop unrolled, so that the matrix stays in registers)
 template <int D>
 __device__ void sym_eigenvalues(double a[D][D], double *ev)
 {
     for (int sweep = 0; sweep < 64; sweep++)
     {
-        double off = 0;
+        double off = 0, diag = 0;
+#pragma unroll
         for (int i = 0; i < D; i++)
+        {
+            diag += a[i][i] * a[i][i];
+#pragma unroll
             for (int j = i + 1; j < D; j++) off += a[i][j] * a[i][j];
-        if (off == 0) break;
+        }
+        if (!(off > 1e-40 * diag)) break;
+#pragma unroll
         for (int p = 0; p < D; p++)
+#pragma unroll
             for (int q = p + 1; q < D; q++)
             {
                 if (a[p][q] == 0) continue;
                 double theta = (a[q][q] - a[p][p]) / (2 * a[p][q]);
                 double t = (theta >= 0 ? 1. : -1.) / (fabs(theta) + sqrt(theta * theta + 1));
                 double c = 1 / sqrt(t * t + 1), s = t * c;
+#pragma unroll
                 for (int k = 0; k < D; k++)
                 {
                     double akp = a[k][p], akq = a[k][q];
                     a[k][p] = c * akp - s * akq;
                     a[k][q] = s * akp + c * akq;
                 }
+#pragma unroll
                 for (int k = 0; k < D; k++)
                 {
                     double apk = a[p][k], aqk = a[q][k];
@@ -636,17 +647,23 @@ __device__ void sym_eigenvalues(double a[D][D], double *ev)
                 }
             }
     }
+#pragma unroll
     for (int i = 0; i < D; i++) ev[i] = a[i][i];
+#pragma unroll
     for (int i = 1; i < D; i++)
-        for (int j = i; j > 0 && ev[j - 1] > ev[j]; j--) { double t = ev[j]; ev[j] = ev[j - 1]; ev[j - 1] = t; }
+#pragma unroll
+        for (int j = i; j > 0; j--)
+            if (ev[j - 1] > ev[j]) { double t = ev[j]; ev[j] = ev[j - 1]; ev[j - 1] = t; }
 }
 
 template <int D>
-__global__ void estimator_kernel(DensityGrids<D> G, const double *pos, int64_t n, double *measure, double *noise, double *sdepth)
+__global__ void estimator_kernel(DensityGrids<D> G, const double *pos, const int *order, int64_t n, double *measure, double *noise,
+                                 double *sdepth)
 {
     constexpr int W = 1 + D + D * D;
     int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
     if (i >= n) return;
+    i = order[i];  // neighbours in space together: one depth search and one set of vertices for a warp
     double p[D];
     for (int d = 0; d < D; d++) p[d] = pos[i * D + d];
     int maxT = G.depth + 1;
@@ -745,45 +762,78 @@ __device__ void project_blade(double *p)
         for (int j = 0; j < i; j++, idx++) p[idx] = ((v1[j] * scale) * (v2[i] * scale) - (v1[i] * scale) * (v2[j] * scale)) / 2.;
 }
 
+// sum[v] = own[v] + the prolongation of the coarser level's sums: the vertex values accumulated over the tree
+// depths, of which element_frame_kernel reads one depth (reading all nine of a depth-8 tree took 10.7 ms)
+template <int D>
+__global__ void accumulate_frames_kernel(int level, const double *own, const double *coarse, double *sum)
+{
+    constexpr int K = D * (D - 1) / 2;
+    Grid<D> g(level), gc(level - 1);
+    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (i >= g.N) return;
+    int I[D];
+    g.node(i, I);
+    double acc[K];
+#pragma unroll
+    for (int k = 0; k < K; k++) acc[k] = 0;
+    for (int c = 0; c < (1 << D); c++)
+    {
+        int J[D];
+        bool use = true;
+        double w = 1.;
+#pragma unroll
+        for (int d = 0; d < D; d++)
+        {
+            const int b = (c >> d) & 1;
+            if (I[d] & 1) { J[d] = (I[d] >> 1) + b; w *= 0.5; }
+            else { J[d] = I[d] >> 1; use = use && !b; }
+        }
+        if (!use) continue;
+        const double *v = coarse + gc.node(J) * K;
+#pragma unroll
+        for (int k = 0; k < K; k++) acc[k] += w * v[k];
+    }
+#pragma unroll
+    for (int k = 0; k < K; k++) sum[i * K + k] = own[i * K + k] + acc[k];
+}
+
 template <int D>
 __global__ void element_frame_kernel(SkewGrids<D> G, double *S, int *leaf, int project)
 {
     constexpr int K = D * (D - 1) / 2;
-    int r = 1 << G.depth;
-    int64_t NE = 1;
-    for (int d = 0; d < D; d++) NE *= r;
     int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (e >= NE) return;
+    const Grid<D> grid(G.depth);
+    if (e >= grid.NE) return;
     int E[D];
-    Grid<D>(G.depth).elem(e, E);
-    double p[D];
-    for (int d = 0; d < D; d++) p[d] = (E[d] + 0.5) / r;
+    grid.elem(e, E);
+    // the element centre (E + 1/2) / r lies inside a cell of every depth (its coordinate there is an odd
+    // multiple of a power of two), so the cells are E's leading bits and its place in them the others
     int L = 1;
     while (L <= G.depth)
     {
-        int side = 1 << L, res = 1 << (L - 1);
+        int side = 1 << L;
         int64_t li = 0;
-        for (int d = 0; d < D; d++) li = li * side + tree_cell(p[d], res);
+        for (int d = 0; d < D; d++) li = li * side + (E[d] >> (G.depth + 1 - L));
         if (!G.refined[L][li]) break;
         L++;
     }
+    // the sum over the tree depths 1..L of the splats' multilinear interpolants, which on a depth-L cell is
+    // the interpolant of their accumulated vertex values
     double acc[K];
     for (int k = 0; k < K; k++) acc[k] = 0;
-    for (int t = 1; t <= L; t++)
     {
-        int res = 1 << (t - 1), nv = res + 1;
+        const int res = 1 << (L - 1), nv = res + 1, below = G.depth + 1 - L;
+        const double unit = 1. / (double)(1 << below);
         int c[D];
         double lv[D][2];
         for (int d = 0; d < D; d++)
         {
-            double s = p[d] * res;
-            int f = (int)floor(s);
-            double x = s - f;
+            const double x = ((E[d] & ((1 << below) - 1)) + 0.5) * unit;
             lv[d][0] = 1. - x;
             lv[d][1] = x;
-            c[d] = tree_cell(p[d], res);
+            c[d] = E[d] >> below;
         }
-        const double *g = G.g[t - 1];
+        const double *g = G.g[L - 1];
         for (int cc = 0; cc < (1 << D); cc++)
         {
             double w = 1.;
@@ -837,11 +887,78 @@ __host__ __device__ inline double mass1(int a, int b) { return a == b ? 1. / 3. 
 __host__ __device__ inline double stiff1(int a, int b) { return a == b ? 1. : -1.; }
 __host__ __device__ inline double mixed1(int a) { return (a ? 1. : -1.) * 0.5; }
 
-// R = sWeight * mean(measure) * sum_samples w phi_a phi_b, gathered per column node a
+// R = sWeight * mean(measure) * sum_samples w phi_a phi_b.  First per occupied cell, a warp each: the sums
+// over the cell's samples (in their order) of w phi_a phi_b for every pair of corners a <= b; 32 samples at
+// a time put their weighted and plain hat values in shared memory, then every lane sums its pairs.  A
+// sample's exponential and hats are formed once (a thread per node and its eight cells formed them eight
+// times, in a loop as long as the densest cell: 6.9 ms at depth 7 with 200,000 samples).
 template <int D>
-__global__ void screening_kernel(const double *pos, const double *noise, const int *order, const int *cellStart,
-                                 const int *cellOfFinest, int depth, double nSigma, const double *scaleDev, double *A)
+struct CellPairs
 {
+    static constexpr int C = 1 << D, N = C * (C + 1) / 2;
+    static __host__ __device__ constexpr int index(int a, int b) { return a <= b ? a * C - a * (a - 1) / 2 + (b - a) : index(b, a); }
+};
+template <int D>
+__global__ void __launch_bounds__(128) cell_mass_kernel(const double *pos, const double *noise, const int *order, const int *cellStart,
+                                                         const int64_t *cellKey, int64_t ncells, int depth, double nSigma, double *mass)
+{
+    using CP = CellPairs<D>;
+    constexpr int C = CP::C, NP = (CP::N + 31) / 32;
+    __shared__ double hats[4][32][C + 1];  // the last value of a row: the sample's weight
+    const int wp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int64_t k = blockIdx.x * (int64_t)4 + wp;
+    if (k >= ncells) return;  // whole warps
+    const int r = 1 << depth;
+    int E[D];
+    demorton<D>(cellKey[k], depth, E);
+    int pa[NP], pb[NP];
+    double acc[NP];
+#pragma unroll
+    for (int n = 0; n < NP; n++)
+    {
+        int p = lane + 32 * n, a = 0;
+        while (a < C - 1 && p >= C - a) { p -= C - a; a++; }
+        pa[n] = a;
+        pb[n] = min(a + p, C - 1);
+        acc[n] = 0;
+    }
+    const int first = cellStart[k], last = cellStart[k + 1];
+    for (int j0 = first; j0 < last; j0 += 32)
+    {
+        const int j = j0 + lane;
+        if (j < last)
+        {
+            const int s = order[j];
+            const double nz = noise[s];
+            double lv[D][2];
+#pragma unroll
+            for (int d = 0; d < D; d++) { const double x = pos[(int64_t)s * D + d] * r - E[d]; lv[d][0] = 1. - x; lv[d][1] = x; }
+#pragma unroll
+            for (int c = 0; c < C; c++)
+            {
+                double h = 1.;
+#pragma unroll
+                for (int d = 0; d < D; d++) h *= lv[d][(c >> (D - 1 - d)) & 1];
+                hats[wp][lane][c] = h;
+            }
+            hats[wp][lane][C] = exp(-nz * nz / (2. * nSigma * nSigma));
+        }
+        __syncwarp();
+        const int cnt = min(32, last - j0);
+        for (int t = 0; t < cnt; t++)
+#pragma unroll
+            for (int n = 0; n < NP; n++) acc[n] += hats[wp][t][pa[n]] * hats[wp][t][pb[n]] * hats[wp][t][C];
+        __syncwarp();
+    }
+#pragma unroll
+    for (int n = 0; n < NP; n++)
+        if (lane + 32 * n < CP::N) mass[k * CP::N + lane + 32 * n] = acc[n];
+}
+// ... then gathered per column node from its cells
+template <int D>
+__global__ void screening_kernel(const double *mass, const int *cellOfFinest, int depth, const double *scaleDev, double *A)
+{
+    using CP = CellPairs<D>;
     constexpr int S = Dims<D>::S;
     Grid<D> g(depth);
     int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
@@ -849,42 +966,33 @@ __global__ void screening_kernel(const double *pos, const double *noise, const i
     int I[D];
     g.node(i, I);
     double acc[S];
+#pragma unroll
     for (int o = 0; o < S; o++) acc[o] = 0;
     bool any = false;
+#pragma unroll
     for (int a = 0; a < (1 << D); a++)
     {
         int E[D];
         bool ok = true;
+#pragma unroll
         for (int d = 0; d < D; d++) { E[d] = I[d] - ((a >> (D - 1 - d)) & 1); if (E[d] < 0 || E[d] >= g.r) ok = false; }
         if (!ok) continue;
-        int k = cellOfFinest[g.elem(E)];
+        const int k = cellOfFinest[g.elem(E)];
         if (k < 0) continue;
         any = true;
-        for (int j = cellStart[k]; j < cellStart[k + 1]; j++)
+        const double *m = mass + (int64_t)k * CP::N;
+#pragma unroll
+        for (int b = 0; b < (1 << D); b++)
         {
-            int s = order[j];
-            double nz = noise[s];
-            double w = exp(-nz * nz / (2. * nSigma * nSigma));
-            double lv[D][2];
-            for (int d = 0; d < D; d++) { double x = pos[(int64_t)s * D + d] * g.r - E[d]; lv[d][0] = 1. - x; lv[d][1] = x; }
-            double pa = 1.;
-            for (int d = 0; d < D; d++) pa *= lv[d][(a >> (D - 1 - d)) & 1];
-            for (int b = 0; b < (1 << D); b++)
-            {
-                double pb = 1.;
-                int o = 0;
-                for (int d = 0; d < D; d++)
-                {
-                    int cb = (b >> (D - 1 - d)) & 1, ca = (a >> (D - 1 - d)) & 1;
-                    pb *= lv[d][cb];
-                    o = o * 3 + (cb - ca + 1);
-                }
-                acc[o] += pa * pb * w;
-            }
+            int o = 0;
+#pragma unroll
+            for (int d = 0; d < D; d++) o = o * 3 + (((b >> (D - 1 - d)) & 1) - ((a >> (D - 1 - d)) & 1) + 1);
+            acc[o] += m[CP::index(a, b)];
         }
     }
     if (!any) return;
-    double sc = *scaleDev;
+    const double sc = *scaleDev;
+#pragma unroll
     for (int o = 0; o < S; o++) A[(int64_t)o * g.N + i] = acc[o] * sc;
 }
 
@@ -1002,102 +1110,97 @@ __global__ void dirichlet_kernel(int level, double w, double *dst)
     }
 }
 
-// 3D Galerkin with every index compile-time: for a coarse node J and fine offsets (go, fo) the
-// parity of F = 2 J + go + fo, hence the coarse parents of F relative to J, depend on go and fo
-// only, so the 27 accumulators stay in registers.  Same sums, same order as the generic kernel.
-__global__ void __launch_bounds__(64) galerkin3_kernel(int fineLevel, const double *Mf, double *Mc)
+// Galerkin coarsening P^T M P of a column stencil along one axis (P is a tensor product, so the axes follow
+// each other; offsets along the other axes stay what they are).  One thread per node of the coarsened
+// grid and offset along the other axes: the 9 entries of the up to three fine nodes 2J + g along the axis,
+// weights 1 and 1/2, three entries out.  Memory-bound, and entries far from the samples are zero: a warp
+// whose entries all are skips the arithmetic.  13 products per thread and axis, against 27 x 27 x 3 per
+// coarse node for all axes at once (depth 8: two stencils 35 ms; on the small levels one thread's chain of
+// dependent FP64 sums took 190 us a level).
+// inner: nodes after the axis, nin / nout: nodes along it, digit: 3^(axes after it)
+__global__ void __launch_bounds__(256) galerkin_axis_kernel(const double *__restrict__ in, double *__restrict__ out, uint32_t totalIn, uint32_t totalOut,
+                                                             uint32_t inner, uint32_t nin, uint32_t nout, int digit)
 {
-    constexpr int D = 3, S = 27;
-    Grid<D> gf(fineLevel), gc(fineLevel - 1);
-    int64_t J = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (J >= gc.N) return;
-    int Jc[D];
-    gc.node(J, Jc);
-    double acc[S];
+    const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
+    if (j >= totalOut) return;  // the last block's tail; the rest of the warp votes with the active mask
+    const int other = blockIdx.y, hi = other / digit, lo = other - hi * digit;
+    const uint32_t t = j / inner, k = j - t * inner, outer = t / nout, J = t - outer * nout;
+    const uint32_t at = (outer * nin + 2 * J) * inner + k;
+    double v[3][3];  // [fine node g + 1][offset f + 1]
+    bool any = false;
 #pragma unroll
-    for (int o = 0; o < S; o++) acc[o] = 0;
-#pragma unroll
-    for (int go = 0; go < S; go++)
+    for (int g = 0; g < 3; g++)
     {
-        const int g0 = go / 9 - 1, g1 = (go / 3) % 3 - 1, g2 = go % 3 - 1;
-        const int G0 = 2 * Jc[0] + g0, G1 = 2 * Jc[1] + g1, G2 = 2 * Jc[2] + g2;
-        if (G0 < 0 || G0 > gf.r || G1 < 0 || G1 > gf.r || G2 < 0 || G2 > gf.r) continue;
-        const double wg = (g0 ? 0.5 : 1.) * (g1 ? 0.5 : 1.) * (g2 ? 0.5 : 1.);
-        const int64_t gi = ((int64_t)G0 * (gf.r + 1) + G1) * (gf.r + 1) + G2;
+        const bool ok = g == 1 || (g == 0 ? J > 0 : J + 1 < nout);
 #pragma unroll
-        for (int fo = 0; fo < S; fo++)
+        for (int f = 0; f < 3; f++)
         {
-            const double v = Mf[(int64_t)fo * gf.N + gi];
-            if (v == 0) continue;
-            const int f[3] = {g0 + fo / 9 - 1, g1 + (fo / 3) % 3 - 1, g2 + fo % 3 - 1};  // F - 2 J
-            const int n1 = (f[0] & 1) + (f[1] & 1) + (f[2] & 1);
-#pragma unroll
-            for (int c = 0; c < (1 << n1); c++)
-            {
-                double w = wg * v;
-                int o = 0, bit = 0;
-#pragma unroll
-                for (int d = 0; d < D; d++)
-                {
-                    int rel;  // coarse parent of F minus J, + 1
-                    if (f[d] & 1) { rel = ((f[d] - 1) >> 1) + ((c >> bit) & 1) + 1; bit++; w *= 0.5; }
-                    else rel = (f[d] >> 1) + 1;
-                    o = o * 3 + rel;
-                }
-                acc[o] += w;
-            }
+            const int64_t o = (int64_t)(hi * 3 + f) * digit + lo;
+            v[g][f] = ok ? __ldcs(in + o * totalIn + (uint32_t)(at + (g - 1) * (int)inner)) : 0.;
+            any = any || v[g][f] != 0.;
         }
     }
+    double r[3] = {0., 0., 0.};
+    if (__any_sync(__activemask(), any))
+    {
+        // row weight (1/2 for the outer nodes) times the parent weights of node g + f
+        r[0] = 0.5 * v[0][0] + 0.25 * v[0][1] + 0.5 * v[1][0];
+        r[1] = 0.25 * v[0][1] + 0.5 * v[0][2] + 0.5 * v[1][0] + v[1][1] + 0.5 * v[1][2] + 0.5 * v[2][0] + 0.25 * v[2][1];
+        r[2] = 0.5 * v[1][2] + 0.25 * v[2][1] + 0.5 * v[2][2];
+    }
 #pragma unroll
-    for (int o = 0; o < S; o++) Mc[(int64_t)o * gc.N + J] = acc[o];
+    for (int f = 0; f < 3; f++) out[((int64_t)(hi * 3 + f) * digit + lo) * totalOut + j] = r[f];
 }
 
-// Galerkin P^T M P of a column stencil, one coarse column per thread
-template <int D>
-__global__ void galerkin_kernel(int fineLevel, const double *Mf, double *Mc)
+// 3D, resolution >= 2: an entry depends on its offset and, per axis, on whether the node is on the lower
+// boundary, inside or on the upper one, so each block tabulates the 27 x 27 entries once (dirichlet_kernel's
+// own sums) and streams through the nodes: one addition an entry, bound by the two passes over the stencil.
+__global__ void __launch_bounds__(256) dirichlet3_kernel(int level, double w, double *dst)
 {
-    constexpr int S = Dims<D>::S;
-    Grid<D> gf(fineLevel), gc(fineLevel - 1);
-    int64_t J = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
-    if (J >= gc.N) return;
-    int Jc[D];
-    gc.node(J, Jc);
-    double acc[S];
-    for (int o = 0; o < S; o++) acc[o] = 0;
-    for (int go = 0; go < S; go++)
+    constexpr int D = 3, S = 27;
+    __shared__ double table[27][S];
+    Grid<D> g(level);
+    const double h = 1. / g.r;
+    for (int k = threadIdx.x; k < 27 * S; k += blockDim.x)
     {
-        int goff[D], G[D];
-        stencil_offset<D>(go, goff);
+        const int cls = k / S, o = k - cls * S;
+        const int cd[D] = {cls / 9, (cls / 3) % 3, cls % 3}, off[D] = {o / 9 - 1, (o / 3) % 3 - 1, o % 3 - 1};
+        double sd[D], md[D];
         bool ok = true;
-        double wg = 1.;
-        for (int d = 0; d < D; d++) { G[d] = 2 * Jc[d] + goff[d]; if (G[d] < 0 || G[d] > gf.r) ok = false; if (goff[d]) wg *= 0.5; }
-        if (!ok) continue;
-        int64_t gi = gf.node(G);
-        for (int fo = 0; fo < S; fo++)
+        for (int d = 0; d < D; d++)
         {
-            double v = Mf[(int64_t)fo * gf.N + gi];
-            if (v == 0) continue;
-            int foff[D], F[D];
-            stencil_offset<D>(fo, foff);
-            for (int d = 0; d < D; d++) F[d] = G[d] + foff[d];
-            int n1 = 0;
-            for (int d = 0; d < D; d++) n1 += F[d] & 1;
-            for (int c = 0; c < (1 << n1); c++)
+            const int I = cd[d] == 0 ? 0 : cd[d] == 2 ? g.r : 1, J = I + off[d];
+            ok = ok && J >= 0 && J <= g.r;
+            double sv = 0, mv = 0;
+            const int lo = max(max(I, J) - 1, 0), hi = min(min(I, J), g.r - 1);
+            for (int e = lo; e <= hi; e++)
             {
-                double w = wg * v;
-                int o = 0, bit = 0;
-                for (int d = 0; d < D; d++)
-                {
-                    int Ic;
-                    if (F[d] & 1) { Ic = ((F[d] - 1) >> 1) + ((c >> bit) & 1); bit++; w *= 0.5; }
-                    else Ic = F[d] >> 1;
-                    o = o * 3 + (Ic - Jc[d] + 1);
-                }
-                acc[o] += w;
+                sv += stiff1(I - e, J - e) / h;
+                mv += mass1(I - e, J - e) * h;
             }
+            sd[d] = sv;
+            md[d] = mv;
         }
+        double sum = 0;
+        for (int q = 0; q < D; q++)
+        {
+            double v = 1.;
+            for (int d = 0; d < D; d++) v *= d == q ? sd[d] : md[d];
+            sum += v;
+        }
+        table[cls][o] = ok ? w * sum : 0.;
     }
-    for (int o = 0; o < S; o++) Mc[(int64_t)o * gc.N + J] = acc[o];
+    __syncthreads();
+    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < g.N; i += (int64_t)gridDim.x * blockDim.x)
+    {
+        int I[D];
+        g.node(i, I);
+        int cls = 0;
+#pragma unroll
+        for (int d = 0; d < D; d++) cls = cls * 3 + (I[d] == 0 ? 0 : I[d] == g.r ? 2 : 1);
+#pragma unroll
+        for (int o = 0; o < S; o++) dst[(int64_t)o * g.N + i] += table[cls][o];
+    }
 }
 
 __global__ void scale_by_kernel(double *v, const double *num, double mult, int64_t den)
@@ -1300,7 +1403,7 @@ bool build_impl(Context &c, Setup &st)
         DensityGrids<D> G;
         for (int l = 0; l <= depth; l++) G.g[l] = st.density[l];
         G.depth = depth;
-        estimator_kernel<D><<<nblocks(n, 128), 128, 0, s>>>(G, st.pos, n, st.measure, st.noise, st.sdepth);
+        estimator_kernel<D><<<nblocks(n, 128), 128, 0, s>>>(G, st.pos, st.order, n, st.measure, st.noise, st.sdepth);
     }
     if (!c.launch_ok("estimator")) return false;
 
@@ -1333,10 +1436,19 @@ bool build_impl(Context &c, Setup &st)
     if (!dalloc(c, &st.S, gfine.NE * K, "S") || !dalloc(c, &st.leaf, gfine.NE, "leaf")) return false;
     {
         SkewGrids<D> G;
-        for (int l = 0; l <= depth; l++) G.g[l] = st.skewGrid[l];
+        std::vector<double *> sums(depth + 1, nullptr);
+        G.g[0] = st.skewGrid[0];
+        for (int l = 1; l <= depth; l++)
+        {
+            Grid<D> gl(l);
+            if (!dalloc(c, &sums[l], gl.N * K, "frame sums")) return false;
+            accumulate_frames_kernel<D><<<nblocks(gl.N, 256), 256, 0, s>>>(l, st.skewGrid[l], G.g[l - 1], sums[l]);
+            G.g[l] = sums[l];
+        }
         for (int t = 0; t <= depth + 1 && t < 12; t++) G.refined[t] = st.refinedS[t];
         G.depth = depth;
         element_frame_kernel<D><<<nblocks(gfine.NE, 128), 128, 0, s>>>(G, st.S, st.leaf, c.P.project);
+        for (double *p : sums) c.release(p);
     }
     // the adaptive indexer: its tables, and the frame field restricted to its elements for c and B
     const double *Sfit = st.S;
@@ -1364,19 +1476,26 @@ bool build_impl(Context &c, Setup &st)
     {
         if (!device_sum(c, st.measure, n, 1, dsum + 1)) return false;
         scale_by_kernel<<<1, 32, 0, s>>>(dsum + 2, dsum + 1, c.P.s_weight, n);
-        screening_kernel<D><<<nblocks(Lf.N, 128), 128, 0, s>>>(st.pos, st.noise, st.order, st.cellStart, st.cellOfFinest, depth,
-                                                               c.P.n_sigma, dsum + 2, Lf.A64);
+        double *mass = nullptr;
+        if (!dalloc(c, &mass, (size_t)nc * CellPairs<D>::N, "cell masses")) return false;
+        cell_mass_kernel<D><<<nblocks(nc, 4), 128, 0, s>>>(st.pos, st.noise, st.order, st.cellStart, st.cellKey, nc, depth, c.P.n_sigma, mass);
+        screening_kernel<D><<<nblocks(Lf.N, 128), 128, 0, s>>>(mass, st.cellOfFinest, depth, dsum + 2, Lf.A64);
+        c.release(mass);
     }
     constraint_kernel<D><<<nblocks(Lf.N, 128), 128, 0, s>>>(Sfit, depth, Lf.B64);
     c.release(Smasked);
     if (!c.launch_ok("finest stencils")) return false;
 
     // ---- Galerkin hierarchy of R and B, then A = R + dWeight K on every level ----
-    for (int l = depth; l > 0; l--)
     {
-        Grid<D> gc(l - 1);
-        launch_galerkin<D>(l, c.levels[l].A64, c.levels[l - 1].A64, s);
-        launch_galerkin<D>(l, c.levels[l].B64, c.levels[l - 1].B64, s);
+        double *scratch = nullptr;
+        if (!dalloc(c, &scratch, galerkin_scratch<D>(depth), "galerkin scratch")) return false;
+        for (int l = depth; l > 0; l--)
+        {
+            launch_galerkin<D>(l, c.levels[l].A64, c.levels[l - 1].A64, scratch, s);
+            launch_galerkin<D>(l, c.levels[l].B64, c.levels[l - 1].B64, scratch, s);
+        }
+        c.release(scratch);
     }
     if (!c.launch_ok("galerkin")) return false;
     for (int l = 0; l <= depth; l++)
@@ -1399,7 +1518,8 @@ bool build_impl(Context &c, Setup &st)
 bool add_dirichlet_to(Context &c, int level, double *dst, double w)
 {
     int64_t N = c.levels[level].N;
-    if (c.dim == 3) dirichlet_kernel<3><<<nblocks(N, 128), 128, 0, c.stream>>>(level, w, dst);
+    if (c.dim == 3 && level > 0) dirichlet3_kernel<<<std::min(nblocks(N, 256), 1216u), 256, 0, c.stream>>>(level, w, dst);
+    else if (c.dim == 3) dirichlet_kernel<3><<<nblocks(N, 128), 128, 0, c.stream>>>(level, w, dst);
     else dirichlet_kernel<4><<<nblocks(N, 128), 128, 0, c.stream>>>(level, w, dst);
     return c.launch_ok("dirichlet");
 }
@@ -1463,16 +1583,43 @@ bool Setup::get(Context &c, const std::string &name, double *out, size_t cap, si
     return false;
 }
 
-// Galerkin coarsening of any column stencil (used by the linear multigrid of epr_mg.cu)
+// Galerkin coarsening of any column stencil (also for the linear multigrid of epr_mg.cu)
 template <int D>
-void launch_galerkin(int fineLevel, const double *Mf, double *Mc, cudaStream_t s)
+size_t galerkin_scratch(int fineLevel)
 {
-    Grid<D> gc(fineLevel - 1);
-    if constexpr (D == 3) galerkin3_kernel<<<nblocks(gc.N, 64), 64, 0, s>>>(fineLevel, Mf, Mc);
-    else galerkin_kernel<D><<<nblocks(gc.N, 64), 64, 0, s>>>(fineLevel, Mf, Mc);
+    // the grids with one and two axes coarsened
+    size_t n = (size_t)((1 << fineLevel) + 1), c = (size_t)((1 << (fineLevel - 1)) + 1), first = c, second = c * c;
+    for (int d = 1; d < D; d++) first *= n;
+    for (int d = 2; d < D; d++) second *= n;
+    return (size_t)Dims<D>::S * (first + second);
 }
-template void launch_galerkin<3>(int, const double *, double *, cudaStream_t);
-template void launch_galerkin<4>(int, const double *, double *, cudaStream_t);
+template <int D>
+void launch_galerkin(int fineLevel, const double *Mf, double *Mc, double *scratch, cudaStream_t s)
+{
+    uint32_t ext[D];
+    for (int d = 0; d < D; d++) ext[d] = (1u << fineLevel) + 1;
+    auto total = [&]() { uint32_t t = 1; for (int d = 0; d < D; d++) t *= ext[d]; return t; };
+    const double *in = Mf;
+    double *buf[2] = {scratch, nullptr};
+    uint32_t inner = 1;
+    int digit = 1;
+    for (int d = D - 1; d >= 0; d--)
+    {
+        const uint32_t nin = ext[d], totalIn = total();
+        ext[d] = (nin - 1) / 2 + 1;
+        const uint32_t totalOut = total();
+        if (d == D - 1) buf[1] = scratch + (size_t)Dims<D>::S * totalOut;
+        double *out = d == 0 ? Mc : buf[(D - 1 - d) & 1];
+        galerkin_axis_kernel<<<dim3(nblocks(totalOut, 256), Dims<D>::S / 3), 256, 0, s>>>(in, out, totalIn, totalOut, inner, nin, ext[d], digit);
+        in = out;
+        inner *= ext[d];
+        digit *= 3;
+    }
+}
+template size_t galerkin_scratch<3>(int);
+template size_t galerkin_scratch<4>(int);
+template void launch_galerkin<3>(int, const double *, double *, double *, cudaStream_t);
+template void launch_galerkin<4>(int, const double *, double *, double *, cudaStream_t);
 
 // the products of a build (everything but the samples), so that a context can be built again
 void Setup::release_built(Context &c)
