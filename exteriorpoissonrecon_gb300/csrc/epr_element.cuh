@@ -143,14 +143,6 @@ __device__ __forceinline__ Real component_wedge(const Real *x, const Real *y)
     return s;
 }
 
-template <int D, typename Real>
-__device__ __forceinline__ Real element_wedge(const Real *x, const Real *y)
-{
-    Real s = component_wedge<D, 0>(x, y) + component_wedge<D, 1>(x, y) + component_wedge<D, 2>(x, y);
-    if constexpr (D == 4) s += component_wedge<D, 3>(x, y) + component_wedge<D, 4>(x, y) + component_wedge<D, 5>(x, y);
-    return s;
-}
-
 // ---------------------------------------------------------------------------------------------
 // Quadratic-fit integrals of corner 0 (every node's elements are taken in the canonical
 // orientation, mirrored so that the node is their corner 0: mirroring along axis d flips the sign
@@ -294,13 +286,13 @@ __device__ __forceinline__ void fit_square(FitSums<D, Real> &s, double w, const 
     s.h2 = O::fma(wz.x, z.y, s.h2);
 }
 
-// the fit sums of corner 0 from the corner differences d[c] = f_c - f_0 (d[0] unused)
+// The signed sums of the corner differences d[c] = f_c - f_0 (d[0] unused), one axis at a time (corner
+// bits: axis 0 = 4, axis 1 = 2, axis 2 = 1): D_i, E_i = D of the two other axes, Fn = - D_012
 template <typename Real>
-__device__ __forceinline__ void element_fit_sums(const Real2<Real> (&d)[8], FitSums<3, Real> &s)
+__device__ __forceinline__ void signed_sums(const Real2<Real> (&d)[8], Real2<Real> (&Dm)[3], Real2<Real> (&E)[3], Real2<Real> &Fn)
 {
     using O = Ops<Real>;
     using V = Real2<Real>;
-    // signed sums, one axis at a time (corner bits: axis 0 = 4, axis 1 = 2, axis 2 = 1)
     const V s01 = O::add(d[2], d[3]), t01 = O::sub(d[2], d[3]);
     const V s10 = O::add(d[4], d[5]), t10 = O::sub(d[4], d[5]);
     const V s11 = O::add(d[6], d[7]), t11 = O::sub(d[6], d[7]);
@@ -308,14 +300,42 @@ __device__ __forceinline__ void element_fit_sums(const Real2<Real> (&d)[8], FitS
     const V ss1 = O::add(s10, s11), st1 = O::sub(s10, s11);
     const V ts0 = O::sub(t01, d[1]), tt0 = O::add(d[1], t01);  // tt0 with the opposite sign
     const V ts1 = O::add(t10, t11), tt1 = O::sub(t10, t11);
-    V Dm[3], E[3];
     Dm[0] = O::sub(ss0, ss1);
     Dm[1] = O::add(st0, st1);
     Dm[2] = O::add(ts0, ts1);
     E[2] = O::sub(st0, st1);
     E[1] = O::sub(ts0, ts1);
     E[0] = O::sub(tt1, tt0);
-    const V Fn = O::add(tt0, tt1);  // - D_012
+    Fn = O::add(tt0, tt1);
+}
+template <typename Real>
+__device__ __forceinline__ void signed_sums(const Real2<Real> (&d)[16], Real2<Real> (&D)[16])
+{
+    using O = Ops<Real>;
+    using V = Real2<Real>;
+    D[0] = V{(Real)0, (Real)0};
+#pragma unroll
+    for (int c = 1; c < 16; c++) D[c] = d[c];
+#pragma unroll
+    for (int b = 1; b < 16; b <<= 1)
+#pragma unroll
+        for (int c = 0; c < 16; c++)
+            if (!(c & b))
+            {
+                const V u = D[c], v = D[c | b];
+                D[c] = (c == 0 && b == 1) ? v : O::add(u, v);
+                D[c | b] = (c == 0 && b == 1) ? V{-v.x, -v.y} : O::sub(u, v);
+            }
+}
+
+// the fit sums of corner 0
+template <typename Real>
+__device__ __forceinline__ void element_fit_sums(const Real2<Real> (&d)[8], FitSums<3, Real> &s)
+{
+    using O = Ops<Real>;
+    using V = Real2<Real>;
+    V Dm[3], E[3], Fn;
+    signed_sums<Real>(d, Dm, E, Fn);
     // |U|^2, |V|^2, <U,V>: squares of the axis-symmetric and the two axis-antisymmetric combinations
     {
         constexpr double kappa = 4.0 / 11.0;
@@ -349,19 +369,7 @@ __device__ __forceinline__ void element_fit_sums(const Real2<Real> (&d)[16], Fit
     using O = Ops<Real>;
     using V = Real2<Real>;
     V D[16];
-    D[0] = V{(Real)0, (Real)0};
-#pragma unroll
-    for (int c = 1; c < 16; c++) D[c] = d[c];
-#pragma unroll
-    for (int b = 1; b < 16; b <<= 1)
-#pragma unroll
-        for (int c = 0; c < 16; c++)
-            if (!(c & b))
-            {
-                const V u = D[c], v = D[c | b];
-                D[c] = (c == 0 && b == 1) ? v : O::add(u, v);
-                D[c | b] = (c == 0 && b == 1) ? V{-v.x, -v.y} : O::sub(u, v);
-            }
+    signed_sums<Real>(d, D);
 #pragma unroll
     for (int P = 1; P < 4; P++)
 #pragma unroll
@@ -392,82 +400,137 @@ __device__ __forceinline__ void element_fit_sums(const Real2<Real> (&d)[16], Fit
         }
 }
 
-// h += the fit integrals of corner 0 of the element with corner values f (canonical orientation)
+// sum over the Gauss points of |W|^2 (reference units).  3D: along the axis R that is neither P nor Q the
+// coefficient of each of the monomials 1, t_P, t_Q is a quadratic W0 + W1 t + W2 t^2 of minors of the signed
+// sums, whose mean square is (W0 + W2 / 3)^2 + W1^2 / 3 + 4/45 W2^2: the 21 minors once, 150 multiplies and
+// adds an element (432 on the 12-point rule).
 template <int D, typename Real>
-__device__ __forceinline__ void element_fit(const Real2<Real> (&f)[1 << D], Real *h)
+__device__ __forceinline__ Real element_wedge(const Real2<Real> (&f)[1 << D])
 {
-    Real2<Real> d[1 << D];
-    d[0] = f[0];
+    using O = Ops<Real>;
+    using V = Real2<Real>;
+    if constexpr (D == 3)
+    {
+        V d[8], Dm[3], E[3], Fn;
 #pragma unroll
-    for (int c = 1; c < (1 << D); c++) d[c] = Ops<Real>::sub(f[c], f[0]);
-    FitSums<D, Real> s;
-    s.clear();
-    element_fit_sums<Real>(d, s);
-    s.add_to(h);
+        for (int c = 1; c < 8; c++) d[c] = O::sub(f[c], f[0]);
+        signed_sums<Real>(d, Dm, E, Fn);
+        Real DE[3][3], DF[3], EF[3];
+#pragma unroll
+        for (int i = 0; i < 3; i++)
+        {
+#pragma unroll
+            for (int j = 0; j < 3; j++) DE[i][j] = minor2<Real>(Dm[i], E[j]);
+            DF[i] = minor2<Real>(Dm[i], Fn);
+            EF[i] = minor2<Real>(E[i], Fn);
+        }
+        const Real third = (Real)(1.0 / 3.0);
+        // mean squares of the monomial 1 (a) and of t_P, t_Q (b), by the three terms above
+        Real a0 = 0, a1 = 0, a2 = 0, b0 = 0, b1 = 0, b2 = 0;
+#pragma unroll
+        for (int P = 1; P < 3; P++)
+#pragma unroll
+            for (int Q = 0; Q < P; Q++)
+            {
+                const int R = 3 - P - Q;
+                auto add = [&](Real W0, Real W1, Real W2, Real &s0, Real &s1, Real &s2) {
+                    const Real m = O::fma(third, W2, W0);
+                    s0 = O::fma(m, m, s0);
+                    s1 = O::fma(W1, W1, s1);
+                    s2 = O::fma(W2, W2, s2);
+                };
+                const Real EPR = minor2<Real>(E[P], E[R]), EQR = minor2<Real>(E[Q], E[R]);
+                // [D_Q + E_P t, D_P + E_Q t], [E_R + F t, D_P + E_Q t], [D_Q + E_P t, E_R + F t] with F = -Fn
+                add(minor2<Real>(Dm[Q], Dm[P]), O::sub(DE[Q][Q], DE[P][P]), minor2<Real>(E[P], E[Q]), a0, a1, a2);
+                add(-DE[P][R], O::sub(DF[P], EQR), EF[Q], b0, b1, b2);
+                add(DE[Q][R], O::sub(EPR, DF[Q]), -EF[P], b0, b1, b2);
+            }
+        const Real p0 = O::fma(third, b0, a0), p1 = O::fma(third, b1, a1), p2 = O::fma(third, b2, a2);
+        // each W carries 1/16 of the signed sums' minors
+        return O::mul((Real)(1.0 / 256.0), O::fma((Real)(4.0 / 45.0), p2, O::fma(third, p1, p0)));
+    }
+    else
+    {
+        Real x[16], y[16];
+#pragma unroll
+        for (int c = 0; c < 16; c++) { x[c] = f[c].x; y[c] = f[c].y; }
+        Real s = component_wedge<D, 0>(x, y) + component_wedge<D, 1>(x, y) + component_wedge<D, 2>(x, y);
+        s += component_wedge<D, 3>(x, y) + component_wedge<D, 4>(x, y) + component_wedge<D, 5>(x, y);
+        return s;
+    }
 }
 
 // ---------------------------------------------------------------------------------------------
-// Gauss-Newton products for corner A: J(d) = W(dx, y) + W(x, dy);
-//   s[0] = sum <J(d), U>,  s[1] = sum <J(d), V>   (reference units)
+// Gauss-Newton products for corner 0 (canonical orientation): J = W(dx, y) + W(x, dy), acc += the sums
+// (<J, V>, -<J, U>) in units of 4^D (the fit's linear part with J in the place of W)
 // ---------------------------------------------------------------------------------------------
-template <int D, int K, typename Real>
-__device__ __forceinline__ void component_gn(const Real *x, const Real *y, const Real *dx, const Real *dy, int A, Real *s)
+template <typename Real>
+__device__ __forceinline__ Real minor_derivative(const Real2<Real> &u, const Real2<Real> &v, const Real2<Real> &du, const Real2<Real> &dv)
 {
-    using Cp = Component<D, K>;
-    constexpr int M = Cp::M;
-    constexpr int NG = ipow(3, M);
-    Real xP[2 * NG], xQ[2 * NG], yP[2 * NG], yQ[2 * NG];
-    Real dxP[2 * NG], dxQ[2 * NG], dyP[2 * NG], dyQ[2 * NG];
-    derivative_table<D, K, true>(x, xP);
-    derivative_table<D, K, false>(x, xQ);
-    derivative_table<D, K, true>(y, yP);
-    derivative_table<D, K, false>(y, yQ);
-    derivative_table<D, K, true>(dx, dxP);
-    derivative_table<D, K, false>(dx, dxQ);
-    derivative_table<D, K, true>(dy, dyP);
-    derivative_table<D, K, false>(dy, dyQ);
-    const int aP = cbit<D>(A, Cp::P), aQ = cbit<D>(A, Cp::Q);
-    const Real sP = aP ? (Real)1 : (Real)-1, sQ = aQ ? (Real)1 : (Real)-1;
-    int ao[M > 0 ? M : 1];
+    using O = Ops<Real>;
+    return O::sub(O::fma(du.x, v.y, O::mul(u.x, dv.y)), O::fma(du.y, v.x, O::mul(u.y, dv.x)));
+}
+template <typename Real>
+__device__ __forceinline__ void gn_point(Real w, const Real2<Real> &q, const Real2<Real> &p, const Real2<Real> &m, const Real2<Real> &dq,
+                                         const Real2<Real> &dp, const Real2<Real> &dm, Real2<Real> &acc)
+{
+    using O = Ops<Real>;
+    const Real third = (Real)(1.0 / 3.0);
+    const Real J1 = O::mul(w, minor_derivative<Real>(q, p, dq, dp));
+    const Real JP = O::mul((Real)(w * third), minor_derivative<Real>(m, p, dm, dp)), JQ = O::mul((Real)(w * third), minor_derivative<Real>(q, m, dq, dm));
+    acc = O::fma(J1, O::sub(q, p), acc);
+    acc = O::fma(JQ, O::sub(q, m), acc);
+    acc = O::fma(JP, O::sub(m, p), acc);
+}
+template <typename Real>
+__device__ __forceinline__ void element_gn(const Real2<Real> (&d)[8], const Real2<Real> (&dd)[8], Real2<Real> &acc)
+{
+    using O = Ops<Real>;
+    using V = Real2<Real>;
+    V D[3], E[3], F, dD[3], dE[3], dF;
+    signed_sums<Real>(d, D, E, F);
+    signed_sums<Real>(dd, dD, dE, dF);
 #pragma unroll
-    for (int m = 0; m < M; m++) ao[m] = cbit<D>(A, Cp::other(m));
-#pragma unroll
-    for (int go = 0; go < NG; go++)
+    for (int k = 0; k < 2; k++)
     {
-        Real lo;
-        if constexpr (M == 1) lo = hat3<Real>(ao[0], go);
-        else lo = hat3<Real>(ao[0], go / 3) * hat3<Real>(ao[1], go % 3);
-        Real wo = (Real)other_weight<M>(go);
+        const Real t = (Real)Jacobi::S(k);
 #pragma unroll
-        for (int gp = 0; gp < 2; gp++)
+        for (int P = 1; P < 3; P++)
 #pragma unroll
-            for (int gq = 0; gq < 2; gq++)
+            for (int Q = 0; Q < P; Q++)
             {
-                Real w = (Real)(Gauss::W2(gp) * Gauss::W2(gq)) * wo;
-                Real phP = sP * hat2<Real>(aQ, gq) * lo;
-                Real phQ = sQ * hat2<Real>(aP, gp) * lo;
-                int ip = gq * NG + go, iq = gp * NG + go;
-                Real J = (yP[ip] * dxQ[iq] - dxP[ip] * yQ[iq]) + (dyP[ip] * xQ[iq] - xP[ip] * dyQ[iq]);
-                Real U = yP[ip] * phQ - phP * yQ[iq];
-                Real V = phP * xQ[iq] - xP[ip] * phQ;
-                s[0] += w * J * U;
-                s[1] += w * J * V;
+                const int R = 3 - P - Q;
+                gn_point<Real>((Real)Jacobi::W(k), O::fma(t, E[P], D[Q]), O::fma(t, E[Q], D[P]), O::fma(-t, F, E[R]), O::fma(t, dE[P], dD[Q]),
+                               O::fma(t, dE[Q], dD[P]), O::fma(-t, dF, dE[R]), acc);
             }
     }
 }
-
-template <int D, typename Real>
-__device__ __forceinline__ void element_gn(const Real *x, const Real *y, const Real *dx, const Real *dy, int A, Real *s)
+template <typename Real>
+__device__ __forceinline__ void element_gn(const Real2<Real> (&d)[16], const Real2<Real> (&dd)[16], Real2<Real> &acc)
 {
-    component_gn<D, 0>(x, y, dx, dy, A, s);
-    component_gn<D, 1>(x, y, dx, dy, A, s);
-    component_gn<D, 2>(x, y, dx, dy, A, s);
-    if constexpr (D == 4)
-    {
-        component_gn<D, 3>(x, y, dx, dy, A, s);
-        component_gn<D, 4>(x, y, dx, dy, A, s);
-        component_gn<D, 5>(x, y, dx, dy, A, s);
-    }
+    using O = Ops<Real>;
+    using V = Real2<Real>;
+    V D[16], dD[16];
+    signed_sums<Real>(d, D);
+    signed_sums<Real>(dd, dD);
+#pragma unroll
+    for (int P = 1; P < 4; P++)
+#pragma unroll
+        for (int Q = 0; Q < P; Q++)
+        {
+            constexpr int ax[4] = {8, 4, 2, 1};
+            const int R = Q > 0 ? 0 : (P > 1 ? 1 : 2), S = 6 - P - Q - R;
+            const int p = ax[P], q = ax[Q], r = ax[R], t = ax[S];
+#pragma unroll
+            for (int i = 0; i < 2; i++)
+#pragma unroll
+                for (int j = 0; j < 2; j++)
+                {
+                    const Real si = (Real)Jacobi::S(i), sj = (Real)Jacobi::S(j);
+                    auto at = [&](const V *T, int a) { return O::fma(sj, O::fma(si, T[a | r | t], T[a | t]), O::fma(si, T[a | r], T[a])); };
+                    gn_point<Real>((Real)(Jacobi::W(i) * Jacobi::W(j)), at(D, q), at(D, p), at(D, p | q), at(dD, q), at(dD, p), at(dD, p | q), acc);
+                }
+        }
 }
 
 }  // namespace epr

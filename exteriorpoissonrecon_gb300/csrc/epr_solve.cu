@@ -38,30 +38,6 @@ struct NodeCtx
     int64_t stride[D];
 };
 
-// Gather the corners of the element whose local corner A is the node I.
-template <int D, typename Real>
-__device__ __forceinline__ bool gather_element(const Grid<D> &g, const NodeCtx<D> &nc, int64_t i, int A, const Real *xy,
-                                               Real *x, Real *y)
-{
-#pragma unroll
-    for (int d = 0; d < D; d++)
-    {
-        int e = nc.I[d] - cbit<D>(A, d);
-        if (e < 0 || e >= g.r) return false;
-    }
-#pragma unroll
-    for (int c = 0; c < (1 << D); c++)
-    {
-        int64_t j = i;
-#pragma unroll
-        for (int d = 0; d < D; d++) j += (int64_t)(cbit<D>(c, d) - cbit<D>(A, d)) * nc.stride[d];
-        Real2<Real> v = ld2(xy, j);
-        x[c] = v.x;
-        y[c] = v.y;
-    }
-    return true;
-}
-
 // Wedge part of the quadratic model of node i, elements in canonical orientation.
 template <int D, typename Real>
 __device__ __forceinline__ void node_wedge_fit(const Grid<D> &g, const NodeCtx<D> &nc, int64_t i, const Real *xy, Real *h)
@@ -208,11 +184,9 @@ __global__ void __launch_bounds__(kThreads) energy_kernel(LevelPtrs<Real> L, con
                 int64_t j = base;
 #pragma unroll
                 for (int d = 0; d < D; d++) j += cbit<D>(c, d) * g.stride(d);
-                Real2<Real> v = ld2(xy, j);
-                x[c] = v.x;
-                y[c] = v.y;
+                f[c] = ld2(xy, j);
             }
-            acc[0] += (double)element_wedge<D, Real>(x, y);
+            acc[0] += (double)element_wedge<D, Real>(f);
         }
         if (t < g.N)
         {
@@ -237,11 +211,12 @@ __global__ void __launch_bounds__(kThreads) energy_kernel(LevelPtrs<Real> L, con
                 if (!ok) continue;
                 Real2<Real> v = ld2(xy, j);
                 double a = (double)L.A[(int64_t)o * L.N + t], b = (double)L.B[(int64_t)o * L.N + t];
-                xb += b * (double)v.y;
-                xa += a * ((double)me.x * (double)v.x + (double)me.y * (double)v.y);
+                by += b * (double)v.y;
+                ax += a * (double)v.x;
+                ay += a * (double)v.y;
             }
-            acc[1] += (double)me.x * xb;
-            acc[2] += xa;
+            acc[1] += (double)me.x * by;
+            acc[2] += (double)me.x * ax + (double)me.y * ay;
         }
     }
     block_sum_store<3>(acc, partial + 4 * blockIdx.x);
@@ -775,13 +750,33 @@ __global__ void __launch_bounds__(kThreads) gn_matvec_kernel(LevelPtrs<Real> L, 
 #pragma unroll 1
     for (int A = 0; A < (1 << D); A++)
     {
-        Real x[1 << D], y[1 << D], dx[1 << D], dy[1 << D];
-        if (!gather_element<D, Real>(g, nc, i, A, xy, x, y)) continue;
-        gather_element<D, Real>(g, nc, i, A, dxy, dx, dy);
-        element_gn<D, Real>(x, y, dx, dy, A, s);
+        bool ok = true;
+        int64_t sd[D];
+#pragma unroll
+        for (int d = 0; d < D; d++)
+        {
+            const int e = nc.I[d] - cbit<D>(A, d);
+            ok = ok && e >= 0 && e < g.r;
+            sd[d] = cbit<D>(A, d) ? -nc.stride[d] : nc.stride[d];
+        }
+        if (!ok) continue;
+        Real2<Real> df[1 << D], dd[1 << D];
+        df[0] = own;
+        dd[0] = down;
+#pragma unroll
+        for (int cc = 1; cc < (1 << D); cc++)
+        {
+            int64_t j = i;
+#pragma unroll
+            for (int d = 0; d < D; d++)
+                if (cbit<D>(cc, d)) j += sd[d];
+            df[cc] = Ops<Real>::sub(ld2(xy, j), own);
+            dd[cc] = Ops<Real>::sub(ld2(dxy, j), down);
+        }
+        element_gn<Real>(df, dd, acc);
     }
-    const Real sc = wedge_scale<D, Real>(g.r);
-    Real ox = s[0] * sc, oy = s[1] * sc;
+    const Real sc = wedge_scale<D, Real>(g.r) * (Real)(D == 3 ? 1.0 / 256.0 : 1.0 / 4096.0);
+    Real ox = -acc.y * sc, oy = acc.x * sc;
     constexpr int S = Dims<D>::S;
     for (int o = 0; o < S; o++)
     {
