@@ -67,6 +67,10 @@ template <typename Real>
 constexpr bool small_level(int level) { return level < 3 || (level == 3 && !std::is_same<Real, double>::value); }
 template <typename Real>
 constexpr bool small_colour_level(int level) { return level < 4 || (level == 4 && std::is_same<Real, double>::value); }
+// 4D in double: levels 0 and 1 in one launch, 2 and 3 by per-colour launches of the same lanes
+constexpr bool small4_colour_level(int level) { return level == 2 || level == 3; }
+bool launch_small4(const LevelPtrs<double> &L, int iters, unsigned int *err, cudaStream_t s, int separate);  // false: not a level it takes
+void launch_small4_colour(const LevelPtrs<double> &L, int colour, unsigned int *err, cudaStream_t s, int separate);
 void prepare_small_kernels();
 template <typename Real>
 void launch_small_level(const LevelPtrs<Real> &L, int iters, unsigned int *err, cudaStream_t s, int separate, int *kexp);

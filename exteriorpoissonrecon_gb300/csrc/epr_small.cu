@@ -542,6 +542,276 @@ __global__ void __launch_bounds__(128) small_colour_batch_kernel(const BatchJob<
     small_colour_body<Store, LEVEL>(b.L, colour, b.err, b.separate, b.kexp);
 }
 
+// ---------------------------------------------------------------------------------------------
+// 4D levels 0-3 in double: a warp per incidence, lane = (wedge component, Gauss-Jacobi point of the two
+// other axes).  The four lanes of a component form one (P, Q) face each and combine them along R and S by two
+// exchanges, so a lane's chain is some 85 FP64 instructions against 850 for a lane per element, with every
+// SM sub-partition on an incidence of its own.  16 incidences (a node has up to 16) go to a cluster of four
+// blocks of four warps and meet in the block of the node's first one.  Level 1, with 16 incidences a colour,
+// runs all sweeps on one such cluster, level 0 on one warp; levels 2 and 3 take a launch per colour, and from
+// level 4 on a lane per element fills the device.
+// ---------------------------------------------------------------------------------------------
+constexpr int kSmallLevels4 = 4;
+__host__ __device__ constexpr int small_base4(int level) { return 16 * ((ipow(16, level) - 1) / 15); }
+// entry: node (13 bits), corner of the element at the node (4 bits), the node's incidences on its first (5 bits)
+__device__ uint32_t g_incidences4[small_base4(kSmallLevels4)];
+
+void host_incidences4(uint32_t *out)
+{
+    for (int level = 0; level < kSmallLevels4; level++)
+    {
+        const Grid<4> g(level);
+        for (int c = 0; c < 16; c++)
+        {
+            const Colour<4> col(g, c);
+            uint32_t *dst = out + small_base4(level) + c * ipow(16, level);
+            for (int want = 16; want > 0; want >>= 1)
+                for (int64_t j = 0; j < col.n; j++)
+                {
+                    int I[4], cnt = 0, corner[16];
+                    col.node(j, I);
+                    for (int A = 0; A < 16; A++)
+                    {
+                        bool ok = true;
+                        for (int d = 0; d < 4; d++) { const int e = I[d] - cbit<4>(A, d); ok = ok && e >= 0 && e < g.r; }
+                        if (ok) corner[cnt++] = A;
+                    }
+                    if (cnt != want) continue;
+                    const uint32_t node = (uint32_t)g.node(I);
+                    for (int k = 0; k < cnt; k++) *dst++ = node | (uint32_t)corner[k] << 13 | (uint32_t)(k == 0 ? cnt : 0) << 17;
+                }
+        }
+    }
+}
+
+// owned_entry in 4D
+__device__ __forceinline__ void owned_entry4(const LevelPtrs<double> &L, int n1, int node, int A, int cc, double &a, double &b)
+{
+    int first = 0, o = 40, rest = node, three = 1;
+#pragma unroll
+    for (int d = 3; d >= 0; d--)
+    {
+        const int bit = 8 >> d, I = rest % n1;
+        rest /= n1;
+        if (I == n1 - 1) first |= bit;
+        if (cc & bit) o += (A & bit) ? -three : three;
+        three *= 3;
+    }
+    const bool own = ((A ^ first) & ~cc & 15) == 0;
+    a = own ? L.A[(int64_t)o * L.N + node] : 0.;
+    b = own && cc ? L.B[(int64_t)o * L.N + node] : 0.;
+}
+
+struct Lane4D
+{
+    int bp, bq, br, bs;       // corner bits of the component's axes P, Q and the others R, S
+    double coR, cxR, coS, cxS;  // weights of the own and the other face along R and S
+    double s1, s2, l1, l3;    // weights of the squares and the linear part (0 on idle lanes)
+    __device__ __forceinline__ void init(int lane, double sc)
+    {
+        const int comp = lane >> 2, i = lane & 1, j = (lane >> 1) & 1;
+        const int P = comp == 0 ? 1 : comp < 3 ? 2 : 3, Q = comp == 0 ? 0 : comp < 3 ? comp - 1 : comp < 6 ? comp - 3 : 2;
+        int R = 0;
+        while (R == P || R == Q) R++;
+        const int S = 6 - P - Q - R;
+        bp = 8 >> P;
+        bq = 8 >> Q;
+        br = 8 >> R;
+        bs = 8 >> S;
+        const double cp[2] = {1.0 + Jacobi::S(0), 1.0 + Jacobi::S(1)}, cm[2] = {1.0 - Jacobi::S(0), 1.0 - Jacobi::S(1)};
+        coR = i ? cm[1] : cp[0];
+        cxR = i ? cp[1] : cm[0];
+        coS = j ? cm[1] : cp[0];
+        cxS = j ? cp[1] : cm[0];
+        const double w = comp < 6 ? (i ? Jacobi::W(1) : Jacobi::W(0)) * (j ? Jacobi::W(1) : Jacobi::W(0)) * sc : 0.;
+        const double wv = w * (i ? cp[1] : cp[0]) * (j ? cp[1] : cp[0]);
+        s1 = wv * (7.0 / 6.0);
+        s2 = wv / 6.0;
+        l1 = w;
+        l3 = w / 3.0;
+    }
+};
+
+// the incidence's sums on every lane: v = (Q20, Q02, -Q11 / 2, Q10 / 2, Q01 / 2); at(offset) reads the pair
+// that many nodes from the node, (a, b) the lane's stencil entry (corner lane % 16 on lanes 0-15)
+template <typename At>
+__device__ __forceinline__ void incidence4d(const Lane4D &ln, const int *stride, int A, int lane, double a, double b, At at, double *v)
+{
+    using O = Ops<double>;
+    using V = double2;
+    auto step = [&](int bits) {  // node offset along the mirrored element's edges
+        int o = 0;
+#pragma unroll
+        for (int d = 0; d < 4; d++)
+            if (bits & (8 >> d)) o += (A & (8 >> d)) ? -stride[d] : stride[d];
+        return o;
+    };
+    {
+        const V n = at(step(lane & 15));
+        v[0] = v[1] = lane == 0 ? a : 0.;
+        v[2] = 0.;
+        v[3] = O::fma(a, n.x, -O::mul(b, n.y));
+        v[4] = O::fma(a, n.y, O::mul(b, n.x));
+    }
+    const int base = step((lane & 1 ? ln.br : 0) | (lane & 2 ? ln.bs : 0)), sp = step(ln.bp), sq = step(ln.bq);
+    const V c00 = at(base), c01 = at(base + sq), c10 = at(base + sp), c11 = at(base + sp + sq);
+    const V u0 = O::sub(c00, c01), u1 = O::sub(c10, c11);
+    V q = O::add(u0, u1), m = O::sub(u0, u1), p = O::add(O::sub(c00, c10), O::sub(c01, c11));
+    auto other = [](V x, int o) { return V{__shfl_xor_sync(0xffffffffu, x.x, o), __shfl_xor_sync(0xffffffffu, x.y, o)}; };
+    auto combine = [&](V x, double co, double cx, int o) { return O::fma(co, x, O::scale(cx, other(x, o))); };
+    q = combine(combine(q, ln.coR, ln.cxR, 1), ln.coS, ln.cxS, 2);
+    p = combine(combine(p, ln.coR, ln.cxR, 1), ln.coS, ln.cxS, 2);
+    m = combine(combine(m, ln.coR, ln.cxR, 1), ln.coS, ln.cxS, 2);
+    const double W1 = O::mul(ln.l1, minor2<double>(q, p)), WP = O::mul(ln.l3, minor2<double>(m, p)), WQ = O::mul(ln.l3, minor2<double>(q, m));
+    const V a1 = O::sub(q, m), a2 = O::sub(m, p), u = O::add(a1, a2), e = O::sub(a2, a1);
+    v[4] = O::fma(u.x, W1, O::fma(a1.x, WQ, O::fma(a2.x, WP, v[4])));
+    v[3] = O::fma(-u.y, W1, O::fma(-a1.y, WQ, O::fma(-a2.y, WP, v[3])));
+    const V us = O::scale(ln.s1, u), es = O::scale(ln.s2, e);
+    v[0] = O::fma(us.y, u.y, O::fma(es.y, e.y, v[0]));
+    v[1] = O::fma(us.x, u.x, O::fma(es.x, e.x, v[1]));
+    v[2] = O::fma(us.x, u.y, O::mul(es.x, e.y));
+    // four values halved with the lanes (lane's value: 2 (lane / 16) + (lane / 8) % 2), the fifth on every lane
+    const bool h16 = (lane & 16) != 0, h8 = (lane & 8) != 0;
+    double k0 = O::add(h16 ? v[2] : v[0], __shfl_xor_sync(0xffffffffu, h16 ? v[0] : v[2], 16));
+    const double k1 = O::add(h16 ? v[3] : v[1], __shfl_xor_sync(0xffffffffu, h16 ? v[1] : v[3], 16));
+    k0 = O::add(h8 ? k1 : k0, __shfl_xor_sync(0xffffffffu, h8 ? k0 : k1, 8));
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) k0 = O::add(k0, __shfl_xor_sync(0xffffffffu, k0, o));
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v[4] = O::add(v[4], __shfl_xor_sync(0xffffffffu, v[4], o));
+#pragma unroll
+    for (int n = 0; n < 4; n++) v[n] = __shfl_sync(0xffffffffu, k0, 8 * n);
+}
+
+// the node's values from its cnt incidences' parts: lane adds every fourth one of value lane % 8
+__device__ __forceinline__ void values_of_node4(const double *part, int cnt, int lane, double *x)
+{
+    const int n = lane & 7;
+    double t = 0.;
+    if (n < 5)
+        for (int k = lane >> 3; k < cnt; k += 4) t = __dadd_rn(t, part[k * 5 + n]);
+    t = __dadd_rn(t, __shfl_xor_sync(0xffffffffu, t, 8));
+    t = __dadd_rn(t, __shfl_xor_sync(0xffffffffu, t, 16));
+#pragma unroll
+    for (int k = 0; k < 5; k++) x[k] = __shfl_sync(0xffffffffu, t, k);
+}
+
+// all sweeps of level 0 (one warp) or 1 (a cluster of four blocks of four warps)
+template <int LEVEL>
+__global__ void __launch_bounds__(LEVEL == 0 ? 32 : 128) small4_kernel(LevelPtrs<double> L, int iters, unsigned int *err, int separate)
+{
+    constexpr int N1 = (1 << LEVEL) + 1, NN = N1 * N1 * N1 * N1, NI = ipow(16, LEVEL), NC = LEVEL == 0 ? 1 : 4, IPB = NI / NC;
+    __shared__ double2 xy[NN];
+    __shared__ double As[16][IPB][16], Bs[16][IPB][16];
+    __shared__ double part[16][5];
+    __shared__ uint32_t tab[16][IPB];
+    cg::cluster_group cluster = cg::this_cluster();
+    const int rank = NC > 1 ? (int)cluster.block_rank() : 0;
+    auto level_sync = [&]() {
+        if constexpr (NC > 1) cluster.sync();
+        else __syncwarp();
+    };
+    for (int k = threadIdx.x; k < NN; k += blockDim.x) xy[k] = ld2(L.xy, k);
+    for (int k = threadIdx.x; k < 16 * IPB * 16; k += blockDim.x)
+    {
+        const int c = k / (16 * IPB), slot = (k >> 4) % IPB, cc = k & 15;
+        const uint32_t e = g_incidences4[small_base4(LEVEL) + c * NI + rank * IPB + slot];
+        const int node = (int)(e & 8191u);
+        owned_entry4(L, N1, node, (int)(e >> 13) & 15, cc, As[c][slot][cc], Bs[c][slot][cc]);
+        if (cc == 0)
+        {
+            // the block of the node's first incidence, where its incidences meet
+            const uint32_t *all = g_incidences4 + small_base4(LEVEL) + c * NI;
+            int own = rank * IPB + slot;
+            while ((all[own] >> 17 & 31u) == 0) own--;
+            tab[c][slot] = e | (relaxed(L, node) ? 1u << 22 : 0u) | (uint32_t)(own / IPB) << 23;
+        }
+    }
+    const int slot = (int)threadIdx.x >> 5, lane = (int)threadIdx.x & 31, global = rank * IPB + slot;
+    const int stride[4] = {N1 * N1 * N1, N1 * N1, N1, 1};
+    Lane4D ln;
+    ln.init(lane, 0.5 / 4096.0);
+    if constexpr (NC == 1) __syncthreads();
+    else cluster.sync();  // every replica ready before any remote write
+    for (int it = 0; it < iters; it++)
+    {
+#pragma unroll 1
+        for (int c = 0; c < 16; c++)
+        {
+            const uint32_t e = tab[c][slot];
+            const int node = (int)(e & 8191u), A = (int)(e >> 13) & 15, cnt = (int)(e >> 17) & 31;
+            const double a = lane < 16 ? As[c][slot][lane & 15] : 0., b = lane < 16 ? Bs[c][slot][lane & 15] : 0.;
+            const double old = reinterpret_cast<const double *>(xy)[2 * node + (lane & 1)];  // before the first shuffle
+            double v[5];
+            incidence4d(ln, stride, A, lane, a, b, [&](int o) { return xy[node + o]; }, v);
+            if constexpr (NC > 1)
+            {
+                if (lane < 5)
+                    cluster.map_shared_rank(&part[0][0], e >> 23 & 3u)[global * 5 + lane] =
+                        lane == 0 ? v[0] : lane == 1 ? v[1] : lane == 2 ? v[2] : lane == 3 ? v[3] : v[4];
+                cluster.sync();
+            }
+            double x[5];
+            if constexpr (NC > 1) values_of_node4(part[global], cnt, lane, x);
+            else
+#pragma unroll
+                for (int k = 0; k < 5; k++) x[k] = v[k];
+            double p;
+            if (cnt && (e >> 22 & 1u) && small_step<double>(x[0], x[1], x[2], x[3], x[4], lane & 1, separate, p))
+            {
+                const double cur = __dadd_rn(old, p);
+                if (lane < 2 && !isfinite(cur)) atomicOr(err, (unsigned int)ERR_NONFINITE);
+                // lane writes component lane % 2 into replica lane / 2
+                if (lane < 2 * NC)
+                {
+                    double2 *to = xy;
+                    if constexpr (NC > 1) to = cluster.map_shared_rank(xy, (unsigned)(lane >> 1));
+                    reinterpret_cast<double *>(to)[2 * node + (lane & 1)] = cur;
+                }
+            }
+            level_sync();  // every replica updated before the next colour reads it
+        }
+    }
+    if (rank == 0)
+        for (int k = threadIdx.x; k < NN; k += blockDim.x) reinterpret_cast<double2 *>(L.xy)[k] = xy[k];
+    if constexpr (NC > 1) cluster.sync();  // no block leaves while another may still address its shared memory
+}
+
+// one colour of level 2 or 3: clusters of four blocks of four warps, 16 incidences each
+template <int LEVEL>
+__global__ void __launch_bounds__(128) small4_colour_kernel(LevelPtrs<double> L, int colour, unsigned int *err, int separate)
+{
+    constexpr int N1 = (1 << LEVEL) + 1, NI = ipow(16, LEVEL);
+    __shared__ double part[16][5];
+    cg::cluster_group cluster = cg::this_cluster();
+    const int rank = (int)cluster.block_rank(), lane = (int)threadIdx.x & 31;
+    const int slot = rank * 4 + ((int)threadIdx.x >> 5), first = ((int)blockIdx.x >> 2) * 16;  // of the cluster's 16 incidences
+    const uint32_t *tab = g_incidences4 + small_base4(LEVEL) + colour * NI + first;
+    const uint32_t e = tab[slot];
+    const int node = (int)(e & 8191u), A = (int)(e >> 13) & 15, cnt = (int)(e >> 17) & 31;
+    const int stride[4] = {N1 * N1 * N1, N1 * N1, N1, 1};
+    Lane4D ln;
+    ln.init(lane, 0.5 / 4096.0);
+    double a = 0., b = 0., v[5];
+    if (lane < 16) owned_entry4(L, N1, node, A, lane, a, b);
+    incidence4d(ln, stride, A, lane, a, b, [&](int o) { return ld2(L.xy, node + o); }, v);
+    int own = slot;
+    while ((tab[own] >> 17 & 31u) == 0) own--;
+    cluster.sync();  // the cluster's blocks have started
+    if (lane < 5)
+        cluster.map_shared_rank(&part[0][0], (unsigned)(own >> 2))[slot * 5 + lane] =
+            lane == 0 ? v[0] : lane == 1 ? v[1] : lane == 2 ? v[2] : lane == 3 ? v[3] : v[4];
+    cluster.sync();
+    double x[5], p;
+    values_of_node4(part[slot], cnt, lane, x);
+    if (cnt && relaxed(L, node) && lane < 2 && small_step<double>(x[0], x[1], x[2], x[3], x[4], lane, separate, p))
+    {
+        const double cur = __dadd_rn(L.xy[2 * (int64_t)node + lane], p);
+        if (!isfinite(cur)) atomicOr(err, (unsigned int)ERR_NONFINITE);
+        L.xy[2 * (int64_t)node + lane] = cur;
+    }
+}
+
 // a launch of `count` blocks or clusters; the blocks of a cluster on SMs of their own where the device can
 template <typename Kernel, typename... Args>
 void launch_small(Kernel kernel, int nc, int count, int threads, size_t smem, cudaStream_t s, Args... args)
@@ -641,6 +911,9 @@ void prepare_small_kernels()
     static uint32_t host[small_base(kSmallLevels)];
     host_incidences(host);
     cudaMemcpyToSymbol(g_incidences, host, sizeof(host));
+    static uint32_t host4[small_base4(kSmallLevels4)];
+    host_incidences4(host4);
+    cudaMemcpyToSymbol(g_incidences4, host4, sizeof(host4));
     g_level3_blocks = holds_16_blocks() ? 16 : 8;
     prepare_store<float>();
     prepare_store<double>();
@@ -686,6 +959,19 @@ void launch_small_colour_batch(const BatchJob<Store> *jobs, int level, int colou
             if constexpr (LEVEL < 4 || std::is_same<Store, double>::value) small_colour_batch_kernel<Store, LEVEL>
                 <<<dim3((ipow(8, LEVEL) + 7) / 8, (unsigned)std::min(65535, count - m0)), 128, 0, s>>>(jobs + m0, colour);
         });
+}
+
+bool launch_small4(const LevelPtrs<double> &L, int iters, unsigned int *err, cudaStream_t s, int separate)
+{
+    if (L.level == 0) launch_small(small4_kernel<0>, 1, 1, 32, 0, s, L, iters, err, separate);
+    else if (L.level == 1) launch_small(small4_kernel<1>, 4, 1, 128, 0, s, L, iters, err, separate);
+    else return false;
+    return true;
+}
+void launch_small4_colour(const LevelPtrs<double> &L, int colour, unsigned int *err, cudaStream_t s, int separate)
+{
+    if (L.level == 2) launch_small(small4_colour_kernel<2>, 4, 16, 128, 0, s, L, colour, err, separate);
+    else launch_small(small4_colour_kernel<3>, 4, 256, 128, 0, s, L, colour, err, separate);
 }
 
 #define EPR_SMALL(T)                                                                                              \

@@ -697,7 +697,7 @@ __global__ void __launch_bounds__(TPB, lanes_min_blocks<3, Real, Pair>() * kThre
     gs_lanes_body<3, Real, Pair, TPB>(b.L, col, cbBase, b.err, b.separate, blockIdx.x, by);
 }
 
-// All sweeps of a small 4D level (8 to 81 nodes) in one thread block: the colours follow each other
+// All sweeps of a small 4D level in float (16 and 81 nodes) in one thread block: the colours follow each other
 // behind a block barrier, which also makes each colour's writes visible to the next.  The level's
 // coefficients, and its stencils when they fit, live in shared memory for the whole schedule.
 template <int D, typename Real, bool SmemStencil>
@@ -920,7 +920,7 @@ __global__ void f2d_kernel(const float *in, double *out, int64_t n)
 
 inline unsigned int blocks_for(int64_t n, int t = kThreads) { return (unsigned int)((n + t - 1) / t); }
 
-// the 4D levels that relax in one block
+// the 4D float levels that relax in one block
 constexpr int64_t kBlockMaxNodes4 = 81;
 constexpr size_t kLevelSmemLimit = 200 * 1024;
 
@@ -968,6 +968,8 @@ void launch_gs_colour(const LevelPtrs<Real> &L, int colour, unsigned int *err, c
     if (col.n == 0) return;
     if constexpr (D == 3)
         if (small_colour_level<Real>(L.level)) return launch_small_colour<Real>(L, colour, err, s, separate, nullptr);
+    if constexpr (D == 4 && std::is_same<Real, double>::value)
+        if (small4_colour_level(L.level)) return launch_small4_colour(L, colour, err, s, separate);
     const int64_t cb = colour_block_base<D>(g, colour);
     auto launch = [&](auto pair) {
         constexpr bool Pair = decltype(pair)::value;
@@ -993,7 +995,6 @@ void prepare_gs_kernels()
 {
     prepare_small_kernels();
     cudaFuncSetAttribute(gs_level_kernel<4, float, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kLevelSmemLimit);
-    cudaFuncSetAttribute(gs_level_kernel<4, double, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kLevelSmemLimit);
 }
 
 template <int D, typename Real>
@@ -1007,7 +1008,9 @@ int launch_gs_sweeps(const LevelPtrs<Real> &L, int iters, unsigned int *err, cud
             launch_small_level<Real>(L, iters, err, s, separate, nullptr);
             return 1;
         }
-    if constexpr (D == 4)
+    if constexpr (D == 4 && std::is_same<Real, double>::value)
+        if (launch_small4(L, iters, err, s, separate)) return 1;
+    if constexpr (D == 4 && std::is_same<Real, float>::value)
         if (g.N <= kBlockMaxNodes4)
         {
             const int64_t colour0 = Colour<D>(g, 0).n;  // the colour of even nodes is the largest
