@@ -145,7 +145,8 @@ bool Context::sync_system32(int l)
         launch_d2df(L.B64, L.Bd, (int64_t)S * L.N, stream);
         return launch_ok("convert system");
     }
-    if (dim == 3 ? !(lvl32(l) ? small_colour_level<float>(l) : small_colour_level<double>(l)) : L.N > 81)  // the levels below read the natural order
+    // the small levels read the natural order
+    if (dim == 3 ? !(lvl32(l) ? small_colour_level<float>(l) : small_colour_level<double>(l)) : lvl32(l) ? L.N > 81 : l > 3)
     {
         const size_t real = lvl32(l) ? sizeof(float) : sizeof(double);
         if (dim == 3 && pair_level<3>(l))
@@ -570,20 +571,16 @@ bool Context::solve_epilogue()
     for (int l = 0; l <= depth; l++)
     {
         if (!levels[l].tmp64 && !alloc((void **)&levels[l].tmp64, sizeof(double) * 2 * levels[l].N, "alloc sol")) return false;
-        if (!cuda_ok(cudaMemcpyAsync(levels[l].tmp64, levels[l].xy64, sizeof(double) * 2 * levels[l].N, cudaMemcpyDeviceToDevice, stream), "copy")) return false;
-    }
-    for (int l = depth; l > 0; l--)
-    {
-        // tmp64[l] -= P xy64[l-1]: prolong into a scratch then subtract
-        double *scratch = nullptr;
-        if (!alloc((void **)&scratch, sizeof(double) * 2 * levels[l].N, "alloc scratch")) return false;
+        if (l == 0)
+        {
+            if (!cuda_ok(cudaMemcpyAsync(levels[0].tmp64, levels[0].xy64, sizeof(double) * 2 * levels[0].N, cudaMemcpyDeviceToDevice, stream), "copy")) return false;
+            continue;
+        }
         with_dim(this, [&](auto dd) {
             constexpr int D = decltype(dd)::value;
-            launch_prolong<D, double>(l - 1, levels[l - 1].xy64, scratch, 0, stream, status_of(l));
+            launch_hierarchical<D>(l - 1, levels[l - 1].xy64, levels[l].xy64, levels[l].tmp64, stream, status_of(l));
             return 0;
         });
-        launch_axpy<double>(levels[l].tmp64, scratch, 2 * levels[l].N, -1.0, stream);
-        release(scratch);
         if (!launch_ok("hierarchical")) return false;
     }
     solved = true;

@@ -86,6 +86,9 @@ template <int D, typename Real>
 // fineStatus (adaptive indexer): fine nodes without a function (status 0) stay zero
 void launch_prolong(int coarseLevel, const Real *coarse, Real *fine, int add, cudaStream_t s,
                     const uint8_t *fineStatus = nullptr);
+// out = fine - P coarse, pairs in double (status as above: P coarse is zero where no function is)
+template <int D>
+void launch_hierarchical(int coarseLevel, const double *coarse, const double *fine, double *out, cudaStream_t s, const uint8_t *fineStatus);
 // coarse = P^T fine, pairs
 template <int D, typename Real>
 void launch_restrict(int coarseLevel, const Real *fine, Real *coarse, cudaStream_t s);

@@ -174,7 +174,7 @@ __global__ void __launch_bounds__(kThreads) energy_kernel(LevelPtrs<Real> L, con
         {
             int E[D];
             g.elem(t, E);
-            Real x[1 << D], y[1 << D];
+            Real2<Real> f[1 << D];
             int64_t base = 0;
 #pragma unroll
             for (int d = 0; d < D; d++) base = base * (g.r + 1) + E[d];
@@ -193,7 +193,7 @@ __global__ void __launch_bounds__(kThreads) energy_kernel(LevelPtrs<Real> L, con
             NodeCtx<D> nc;
             make_ctx<D>(g, t, nc);
             Real2<Real> me = ld2(xy, t);
-            double xb = 0, xa = 0;
+            double by = 0, ax = 0, ay = 0;
             constexpr int S = Dims<D>::S;
             for (int o = 0; o < S; o++)
             {
@@ -746,7 +746,8 @@ __global__ void __launch_bounds__(kThreads) gn_matvec_kernel(LevelPtrs<Real> L, 
     if (i >= g.N) return;
     NodeCtx<D> nc;
     make_ctx<D>(g, i, nc);
-    Real s[2] = {0, 0};
+    Real2<Real> acc = {(Real)0, (Real)0};
+    const Real2<Real> own = ld2(xy, i), down = ld2(dxy, i);
 #pragma unroll 1
     for (int A = 0; A < (1 << D); A++)
     {
@@ -800,19 +801,10 @@ __global__ void __launch_bounds__(kThreads) gn_matvec_kernel(LevelPtrs<Real> L, 
     reinterpret_cast<Real2<Real> *>(out)[i] = Real2<Real>{ox, oy};
 }
 
+// the multilinear interpolant of the coarse pairs at fine node i
 template <int D, typename Real>
-__device__ __forceinline__ void prolong_at(int coarseLevel, const Real *coarse, Real *fine, int add, int64_t i,
-                                           const uint8_t *fineStatus = nullptr)
+__device__ __forceinline__ Real2<Real> prolonged(const Grid<D> &gc, const Grid<D> &gf, const Real *coarse, int64_t i)
 {
-    Grid<D> gc(coarseLevel), gf(coarseLevel + 1);
-    if (i >= gf.N) return;
-    // the adaptive prolongation reaches indexed fine functions only (ffChildNeighbors,
-    // Hat.scalars.inl:1747-1779); the others stay zero
-    if (fineStatus && fineStatus[i] == 0)
-    {
-        if (!add) reinterpret_cast<Real2<Real> *>(fine)[i] = Real2<Real>{(Real)0, (Real)0};
-        return;
-    }
     int F[D];
     gf.node(i, F);
     Real sx = 0, sy = 0;
@@ -834,9 +826,38 @@ __device__ __forceinline__ void prolong_at(int coarseLevel, const Real *coarse, 
         sx += w * v.x;
         sy += w * v.y;
     }
+    return Real2<Real>{sx, sy};
+}
+template <int D, typename Real>
+__device__ __forceinline__ void prolong_at(int coarseLevel, const Real *coarse, Real *fine, int add, int64_t i,
+                                           const uint8_t *fineStatus = nullptr)
+{
+    Grid<D> gc(coarseLevel), gf(coarseLevel + 1);
+    if (i >= gf.N) return;
+    // the adaptive prolongation reaches indexed fine functions only (ffChildNeighbors,
+    // Hat.scalars.inl:1747-1779); the others stay zero
+    if (fineStatus && fineStatus[i] == 0)
+    {
+        if (!add) reinterpret_cast<Real2<Real> *>(fine)[i] = Real2<Real>{(Real)0, (Real)0};
+        return;
+    }
+    const Real2<Real> v = prolonged<D, Real>(gc, gf, coarse, i);
     Real2<Real> *o = reinterpret_cast<Real2<Real> *>(fine);
-    if (add) { Real2<Real> cur = o[i]; o[i] = Real2<Real>{cur.x + sx, cur.y + sy}; }
-    else o[i] = Real2<Real>{sx, sy};
+    if (add) { Real2<Real> cur = o[i]; o[i] = Real2<Real>{cur.x + v.x, cur.y + v.y}; }
+    else o[i] = v;
+}
+// out = fine - P coarse (P coarse zero at fine nodes without a function): a level's hierarchical coefficients
+template <int D>
+__global__ void __launch_bounds__(256) hierarchical_kernel(int coarseLevel, const double *coarse, const double *fine, double *out,
+                                                            const uint8_t *fineStatus)
+{
+    Grid<D> gc(coarseLevel), gf(coarseLevel + 1);
+    const int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;
+    if (i >= gf.N) return;
+    double2 p = {0., 0.};
+    if (!(fineStatus && fineStatus[i] == 0)) p = prolonged<D, double>(gc, gf, coarse, i);
+    const double2 v = ld2(fine, i);
+    reinterpret_cast<double2 *>(out)[i] = double2{v.x - p.x, v.y - p.y};
 }
 template <int D, typename Real>
 __global__ void prolong_kernel(int coarseLevel, const Real *coarse, Real *fine, int add, const uint8_t *fineStatus)
@@ -1103,6 +1124,15 @@ void launch_prolong(int coarseLevel, const Real *coarse, Real *fine, int add, cu
     Grid<D> gf(coarseLevel + 1);
     prolong_kernel<D, Real><<<blocks_for(gf.N, 256), 256, 0, s>>>(coarseLevel, coarse, fine, add, fineStatus);
 }
+
+template <int D>
+void launch_hierarchical(int coarseLevel, const double *coarse, const double *fine, double *out, cudaStream_t s, const uint8_t *fineStatus)
+{
+    Grid<D> gf(coarseLevel + 1);
+    hierarchical_kernel<D><<<blocks_for(gf.N, 256), 256, 0, s>>>(coarseLevel, coarse, fine, out, fineStatus);
+}
+template void launch_hierarchical<3>(int, const double *, const double *, double *, cudaStream_t, const uint8_t *);
+template void launch_hierarchical<4>(int, const double *, const double *, double *, cudaStream_t, const uint8_t *);
 
 template <int D, typename Real>
 void launch_restrict(int coarseLevel, const Real *fine, Real *coarse, cudaStream_t s)
