@@ -102,9 +102,17 @@ bool Context::ensure_level(int l)
     if (P.precision == EPR_FP32)
     {
         if (!alloc((void **)&L.xy32, sizeof(float) * 2 * L.N, "alloc xy32")) return false;
-        if (!alloc((void **)&L.A32, sizeof(float) * S * L.N, "alloc A32")) return false;
-        if (!alloc((void **)&L.B32, sizeof(float) * S * L.N, "alloc B32")) return false;
+        if (!(dim == 3 && pair_level<3>(l)) &&
+            (!alloc((void **)&L.A32, sizeof(float) * S * L.N, "alloc A32") || !alloc((void **)&L.B32, sizeof(float) * S * L.N, "alloc B32")))
+            return false;
         if (!cuda_ok(cudaMemsetAsync(L.xy32, 0, sizeof(float) * 2 * L.N, stream), "memset xy32")) return false;
+    }
+    if (dim == 3 && pair_level<3>(l))
+    {
+        // the pair layout from the start: the relaxation of these levels reads nothing else
+        const size_t bytes = 56 * L.N * (lvl32(l) ? sizeof(float) : sizeof(double));
+        if (!alloc(&L.Acb, bytes, "alloc colour blocks")) return false;
+        if (!cuda_ok(cudaMemsetAsync(L.Acb, 0, bytes, stream), "memset colour blocks")) return false;
     }
     if (lvlDF(l))
     {
@@ -133,7 +141,7 @@ bool Context::sync_system32(int l)
 {
     Level &L = levels[l];
     size_t S = (size_t)stencil();
-    if (lvl32(l))
+    if (lvl32(l) && L.A32)
     {
         launch_convert_d2f(L.A64, L.A32, (int64_t)S * L.N, stream);
         launch_convert_d2f(L.B64, L.B32, (int64_t)S * L.N, stream);
@@ -151,8 +159,7 @@ bool Context::sync_system32(int l)
         const size_t real = lvl32(l) ? sizeof(float) : sizeof(double);
         if (dim == 3 && pair_level<3>(l))
         {
-            if (!L.Acb && !alloc(&L.Acb, 56 * L.N * real, "alloc colour blocks")) return false;
-            if (lvl32(l)) launch_to_pair_blocks<float>(l, L.A32, L.B32, (float *)L.Acb, stream);
+            if (lvl32(l)) launch_to_pair_blocks<float>(l, L.A64, L.B64, (float *)L.Acb, stream);
             else launch_to_pair_blocks<double>(l, L.A64, L.B64, (double *)L.Acb, stream);
             return launch_ok("convert system");
         }

@@ -23,7 +23,7 @@ struct Level
     double *B64 = nullptr;    // frame constraint, column stencil, offset-major
     double *tmp64 = nullptr;  // hierarchical solution after a solve
     float *xy32 = nullptr;    // float copies used when precision == EPR_FP32
-    float *A32 = nullptr;
+    float *A32 = nullptr;     // (none on float pair levels: the pair layout and the double stencils)
     float *B32 = nullptr;
     float *tmp32 = nullptr;
     void *Acb = nullptr;      // colour-blocked A and B in the level's precision (levels relaxed
@@ -156,7 +156,7 @@ inline LevelPtrs<Real> level_ptrs(Context *c, int l)
     }
     if constexpr (std::is_same<Real, double>::value) { p.xy = L.xy64; p.A = L.A64; p.B = L.B64; }
     else if constexpr (std::is_same<Real, df>::value) { p.xy = L.xyd; p.A = L.Ad; p.B = L.Bd; return p; }
-    else { p.xy = L.xy32; p.A = L.A32; p.B = L.B32; }
+    else { p.xy = L.xy32; p.A = L.A32; p.B = L.B32; p.A64 = L.A64; p.B64 = L.B64; }
     if (L.Acb && c->lvl32(l) == std::is_same<Real, float>::value)
     {
         p.Acb = (const Real *)L.Acb;

@@ -19,6 +19,10 @@ struct LevelPtrs
     Real *xy = nullptr;       // 2N interleaved (x, y)
     const Real *A = nullptr;  // 3^Dim * N column stencil of R + dWeight K (offset-major)
     const Real *B = nullptr;  // 3^Dim * N column stencil of the frame constraint
+    // double stencils, where a level keeps no natural copy in Real (A, B null: float pair levels, whose
+    // relaxation reads the pair layout; the other float kernels round the entries as they load them)
+    const double *A64 = nullptr;
+    const double *B64 = nullptr;
     const Real *Acb = nullptr;  // optional colour-blocked copies of A and B (colour_block_base); on pair
     const Real *Bcb = nullptr;  // levels both in Acb (PairLayout)
     // adaptive indexer: per node 0 (no function), 1 (indexed, held fixed), 2 (active); the
@@ -106,7 +110,7 @@ void launch_to_colour_blocks(int level, const double *M, Real *out, cudaStream_t
 
 // both natural stencils of a 3D level (level >= kPairLevel) -> its pair layout (PairLayout, 56 values per node)
 template <typename Real>
-void launch_to_pair_blocks(int level, const Real *A, const Real *B, Real *out, cudaStream_t s);
+void launch_to_pair_blocks(int level, const double *A, const double *B, Real *out, cudaStream_t s);
 
 // elementwise helpers
 template <typename Real>

@@ -129,7 +129,7 @@ __global__ void to_colour_blocks_kernel(int level, const double *M, ColourBlocks
 // both natural offset-major stencils of a 3D level -> its pair layout; one thread per lane of a
 // node, grid.y = colour
 template <typename Real>
-__global__ void to_pair_blocks_kernel(int level, const Real *A, const Real *B, ColourBlocks<3> cb, Real *out)
+__global__ void to_pair_blocks_kernel(int level, const double *A, const double *B, ColourBlocks<3> cb, Real *out)
 {
     using PL = PairLayout<Real>;
     const int c = blockIdx.y;
@@ -158,7 +158,7 @@ __global__ void to_pair_blocks_kernel(int level, const Real *A, const Real *B, C
                 stencil_offset<3>(o, off);
                 for (int d = 0; d < 3; d++) in = in && I[d] + off[d] >= 0 && I[d] + off[d] <= g.r;
             }
-            r[w] = in ? (m ? B : A)[(int64_t)o * g.N + i] : (Real)0;
+            r[w] = in ? (Real)(m ? B : A)[(int64_t)o * g.N + i] : (Real)0;
         }
         typename PL::Vec vec;
         if constexpr (PL::W == 4) vec = make_float4(r[0], r[1], r[2], r[3]);
@@ -765,12 +765,12 @@ __global__ void biquad_finish_kernel(const double *partial, int nblocks, double 
 }  // namespace
 
 template <typename Real>
-void launch_to_pair_blocks(int level, const Real *A, const Real *B, Real *out, cudaStream_t s)
+void launch_to_pair_blocks(int level, const double *A, const double *B, Real *out, cudaStream_t s)
 {
     ColourBlocks<3> cb = colour_blocks<3>(level);
     to_pair_blocks_kernel<Real><<<dim3(blocks(2 * cb.count[0]), 8), kThreads, 0, s>>>(level, A, B, cb, out);
 }
-template void launch_to_pair_blocks<float>(int, const float *, const float *, float *, cudaStream_t);
+template void launch_to_pair_blocks<float>(int, const double *, const double *, float *, cudaStream_t);
 template void launch_to_pair_blocks<double>(int, const double *, const double *, double *, cudaStream_t);
 
 template <int D, typename Real>

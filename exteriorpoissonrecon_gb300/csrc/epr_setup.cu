@@ -1488,14 +1488,19 @@ bool build_impl(Context &c, Setup &st)
 
     // ---- Galerkin hierarchy of R and B, then A = R + dWeight K on every level ----
     {
-        double *scratch = nullptr;
-        if (!dalloc(c, &scratch, galerkin_scratch<D>(depth), "galerkin scratch")) return false;
+        // the finest pair layout is written below and large enough (56 values a node against 27 x 3/4 doubles)
+        double *own = nullptr, *scratch = (double *)(D == 3 && pair_level<3>(depth) ? Lf.Acb : nullptr);
+        if (!scratch)
+        {
+            if (!dalloc(c, &own, galerkin_scratch<D>(depth), "galerkin scratch")) return false;
+            scratch = own;
+        }
         for (int l = depth; l > 0; l--)
         {
             launch_galerkin<D>(l, c.levels[l].A64, c.levels[l - 1].A64, scratch, s);
             launch_galerkin<D>(l, c.levels[l].B64, c.levels[l - 1].B64, scratch, s);
         }
-        c.release(scratch);
+        c.release(own);
     }
     if (!c.launch_ok("galerkin")) return false;
     for (int l = 0; l <= depth; l++)

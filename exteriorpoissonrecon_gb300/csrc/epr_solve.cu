@@ -31,6 +31,12 @@ __device__ __forceinline__ Real wedge_scale(int r)
     return (D == 3 ? (Real)r : (Real)1) * (Real)0.5;
 }
 
+// entry k of a level's stencils (A, B) in the level's arithmetic
+template <typename Real>
+__device__ __forceinline__ Real stencil_a(const LevelPtrs<Real> &L, int64_t k) { return L.A ? L.A[k] : (Real)L.A64[k]; }
+template <typename Real>
+__device__ __forceinline__ Real stencil_b(const LevelPtrs<Real> &L, int64_t k) { return L.B ? L.B[k] : (Real)L.B64[k]; }
+
 template <int D>
 struct NodeCtx
 {
@@ -105,8 +111,8 @@ __device__ __forceinline__ void node_fit(const LevelPtrs<Real> &L, const Grid<D>
             j += (int64_t)off[d] * nc.stride[d];
         }
         if (!ok) continue;
-        Real a = L.A[(int64_t)o * L.N + i];
-        Real b = L.B[(int64_t)o * L.N + i];
+        Real a = stencil_a(L, (int64_t)o * L.N + i);
+        Real b = stencil_b(L, (int64_t)o * L.N + i);
         Real2<Real> v = ld2(xy, j);
         ax += a * v.x;
         ay += a * v.y;
@@ -210,7 +216,7 @@ __global__ void __launch_bounds__(kThreads) energy_kernel(LevelPtrs<Real> L, con
                 }
                 if (!ok) continue;
                 Real2<Real> v = ld2(xy, j);
-                double a = (double)L.A[(int64_t)o * L.N + t], b = (double)L.B[(int64_t)o * L.N + t];
+                double a = (double)stencil_a(L, (int64_t)o * L.N + t), b = (double)stencil_b(L, (int64_t)o * L.N + t);
                 by += b * (double)v.y;
                 ax += a * (double)v.x;
                 ay += a * (double)v.y;
@@ -793,7 +799,7 @@ __global__ void __launch_bounds__(kThreads) gn_matvec_kernel(LevelPtrs<Real> L, 
             j += (int64_t)off[d] * nc.stride[d];
         }
         if (!ok) continue;
-        Real a = L.A[(int64_t)o * L.N + i];
+        Real a = stencil_a(L, (int64_t)o * L.N + i);
         Real2<Real> v = ld2(dxy, j);
         ox += a * v.x;
         oy += a * v.y;
@@ -1008,7 +1014,7 @@ void launch_gs_colour(const LevelPtrs<Real> &L, int colour, unsigned int *err, c
         gs_colour_lanes_kernel<D, Real, Pair><<<grid, kThreads, 0, s>>>(L, col, cb, err, separate);
     };
     if constexpr (D == 3)
-        if (pair_level<D>(L.level) && L.Acb) return launch(std::true_type{});
+        if (pair_level<D>(L.level)) return launch(std::true_type{});
     launch(std::false_type{});
 }
 
