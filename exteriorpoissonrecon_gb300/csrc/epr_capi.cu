@@ -156,13 +156,8 @@ bool Context::sync_system32(int l)
     // the small levels read the natural order
     if (dim == 3 ? !(lvl32(l) ? small_colour_level<float>(l) : small_colour_level<double>(l)) : lvl32(l) ? L.N > 81 : l > 3)
     {
+        if (dim == 3 && pair_level<3>(l)) return pair_system(*this, l, 0.);
         const size_t real = lvl32(l) ? sizeof(float) : sizeof(double);
-        if (dim == 3 && pair_level<3>(l))
-        {
-            if (lvl32(l)) launch_to_pair_blocks<float>(l, L.A64, L.B64, (float *)L.Acb, stream);
-            else launch_to_pair_blocks<double>(l, L.A64, L.B64, (double *)L.Acb, stream);
-            return launch_ok("convert system");
-        }
         const size_t bytes = S * L.N * real;
         if (!L.Acb && (!alloc(&L.Acb, bytes, "alloc colour blocks") || !alloc(&L.Bcb, bytes, "alloc colour blocks"))) return false;
         auto blocks = [&](auto dd) {

@@ -178,6 +178,8 @@ void set_global_error(const std::string &msg);
 // A64[level] += dWeight K (the Dirichlet stiffness of the level, with the reference's
 // resolution-1 stencil table, see epr_setup.cu)
 bool add_dirichlet(Context &c, int level);
+// A64[level] += w K and the level's pair layout from A64 and B64 (3D levels from kPairLevel on)
+bool pair_system(Context &c, int level, double w);
 bool add_dirichlet_to(Context &c, int level, double *dst, double w);
 
 }  // namespace epr

@@ -108,10 +108,6 @@ void launch_galerkin(int fineLevel, const double *Mf, double *Mc, double *scratc
 template <int D, typename Real>
 void launch_to_colour_blocks(int level, const double *M, Real *out, cudaStream_t s);
 
-// both natural stencils of a 3D level (level >= kPairLevel) -> its pair layout (PairLayout, 56 values per node)
-template <typename Real>
-void launch_to_pair_blocks(int level, const double *A, const double *B, Real *out, cudaStream_t s);
-
 // elementwise helpers
 template <typename Real>
 void launch_scale(Real *v, int64_t n, double s, cudaStream_t st);

@@ -126,47 +126,6 @@ __global__ void to_colour_blocks_kernel(int level, const double *M, ColourBlocks
     for (int o = 0; o < Dims<D>::S; o++) dst[o * n] = (Real)M[(int64_t)o * g.N + i];
 }
 
-// both natural offset-major stencils of a 3D level -> its pair layout; one thread per lane of a
-// node, grid.y = colour
-template <typename Real>
-__global__ void to_pair_blocks_kernel(int level, const double *A, const double *B, ColourBlocks<3> cb, Real *out)
-{
-    using PL = PairLayout<Real>;
-    const int c = blockIdx.y;
-    const int64_t t = blockIdx.x * (int64_t)blockDim.x + threadIdx.x, j = t >> 1, n = cb.count[c];
-    const int s = (int)(t & 1);
-    if (j >= n) return;
-    Grid<3> g(level);
-    Colour<3> col(g, c);
-    int I[3];
-    col.node(j, I);
-    const int64_t i = g.node(I);
-    typename PL::Vec *dst = reinterpret_cast<typename PL::Vec *>(out + cb.base[c] / 27 * PL::kNode);
-#pragma unroll
-    for (int v = 0; v < PL::G; v++)
-    {
-        Real r[PL::W];
-#pragma unroll
-        for (int w = 0; w < PL::W; w++)
-        {
-            int o, m;
-            PL::entry(s, v * PL::W + w, o, m);
-            bool in = o >= 0;
-            if (in)
-            {
-                int off[3];
-                stencil_offset<3>(o, off);
-                for (int d = 0; d < 3; d++) in = in && I[d] + off[d] >= 0 && I[d] + off[d] <= g.r;
-            }
-            r[w] = in ? (Real)(m ? B : A)[(int64_t)o * g.N + i] : (Real)0;
-        }
-        typename PL::Vec vec;
-        if constexpr (PL::W == 4) vec = make_float4(r[0], r[1], r[2], r[3]);
-        else vec = make_double2(r[0], r[1]);
-        dst[(v * n + j) * 2 + s] = vec;
-    }
-}
-
 // natural offset-major double stencil -> the multigrid's vector colour blocks; grid.y = colour
 template <int D, typename Real>
 __global__ void to_colour_blocks_vec_kernel(int level, const double *M, ColourBlocks<D> cb, Real *out)
@@ -763,15 +722,6 @@ __global__ void biquad_finish_kernel(const double *partial, int nblocks, double 
 }
 
 }  // namespace
-
-template <typename Real>
-void launch_to_pair_blocks(int level, const double *A, const double *B, Real *out, cudaStream_t s)
-{
-    ColourBlocks<3> cb = colour_blocks<3>(level);
-    to_pair_blocks_kernel<Real><<<dim3(blocks(2 * cb.count[0]), 8), kThreads, 0, s>>>(level, A, B, cb, out);
-}
-template void launch_to_pair_blocks<float>(int, const double *, const double *, float *, cudaStream_t);
-template void launch_to_pair_blocks<double>(int, const double *, const double *, double *, cudaStream_t);
 
 template <int D, typename Real>
 void launch_to_colour_blocks(int level, const double *M, Real *out, cudaStream_t s)
