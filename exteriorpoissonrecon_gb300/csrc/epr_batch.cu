@@ -233,12 +233,13 @@ int64_t record(epr_batch &b)
                 return;
             }
             int cnt = P.count;
+            bool after = false;
             for (int k = 0; k < P.iters[0]; k++)
             {
                 while (cnt > 0 && P.iters[cnt - 1] <= k) cnt--;  // members done with this level
                 for (int c = 0; c < 8; c++)
                 {
-                    launch_colour_batch<Real>(jobs, l, c, cnt, b.tile[l], s);
+                    after = launch_colour_batch<Real>(jobs, l, c, cnt, b.tile[l], s, after) || after;
                     launches++;
                 }
             }
@@ -508,7 +509,7 @@ int epr_batch_tune(epr_batch *b, int reps, double *ms_out)
             auto sweep = [&](auto tag) {
                 using Real = decltype(tag);
                 const BatchJob<Real> *jobs = reinterpret_cast<const BatchJob<Real> *>(b->dtab + P.off);
-                for (int c = 0; c < 8; c++) launch_colour_batch<Real>(jobs, l, c, P.count, t, b->stream);
+                for (int c = 0; c < 8; c++) launch_colour_batch<Real>(jobs, l, c, P.count, t, b->stream, c > 0);
             };
             auto one = [&]() {
                 if (P.type == kTypeFloat) sweep(float());

@@ -51,9 +51,10 @@ void launch_grad_norm(const LevelPtrs<Real> &L, const Real *xy, const Reduce &re
 // writes N x 5 doubles (Q20, Q02, Q11, Q10, Q01)
 template <int D, typename Real>
 void launch_quadfit(const LevelPtrs<Real> &L, const Real *xy, double *out, cudaStream_t s);
-// separate != 0: the reference's SeparateGaussSeidelSolve update (x first, then y with the new x)
+// separate != 0: the reference's SeparateGaussSeidelSolve update (x first, then y with the new x).  after: the
+// launch before it on the stream is another colour of the level (launch_colour).  Returns whether it launched.
 template <int D, typename Real>
-void launch_gs_colour(const LevelPtrs<Real> &L, int colour, unsigned int *err, cudaStream_t s, int separate = 0);
+bool launch_gs_colour(const LevelPtrs<Real> &L, int colour, unsigned int *err, cudaStream_t s, int separate = 0, bool after = false);
 // double-float levels: pairs stored as x 2^-k with k = kexp[level] (epr_df.cuh)
 void launch_df_push(const double *in, df *out, int64_t n, int *kexp, int level, cudaStream_t s);
 void launch_df_pull(const df *in, double *out, int64_t n, const int *kexp, int level, cudaStream_t s);
@@ -74,12 +75,13 @@ constexpr bool small_colour_level(int level) { return level < 4 || (level == 4 &
 // 4D in double: levels 0 and 1 in one launch, 2 and 3 by per-colour launches of the same lanes
 constexpr bool small4_colour_level(int level) { return level == 2 || level == 3; }
 bool launch_small4(const LevelPtrs<double> &L, int iters, unsigned int *err, cudaStream_t s, int separate);  // false: not a level it takes
-void launch_small4_colour(const LevelPtrs<double> &L, int colour, unsigned int *err, cudaStream_t s, int separate);
+void launch_small4_colour(const LevelPtrs<double> &L, int colour, unsigned int *err, cudaStream_t s, int separate, bool after);
 void prepare_small_kernels();
 template <typename Real>
 void launch_small_level(const LevelPtrs<Real> &L, int iters, unsigned int *err, cudaStream_t s, int separate, int *kexp);
 template <typename Real>
-void launch_small_colour(const LevelPtrs<Real> &L, int colour, unsigned int *err, cudaStream_t s, int separate, const int *kexp);
+void launch_small_colour(const LevelPtrs<Real> &L, int colour, unsigned int *err, cudaStream_t s, int separate, const int *kexp,
+                         bool after = false);
 // sets the kernels' shared-memory limits and uploads the small levels' tables (once per device, before any
 // stream capture)
 void prepare_gs_kernels();
@@ -150,9 +152,9 @@ template <typename Real>
 void launch_small_level_batch(const BatchJob<Real> *jobs, int level, int count, cudaStream_t s);
 // one colour of a level of jobs[0..count)
 template <typename Real>
-void launch_small_colour_batch(const BatchJob<Real> *jobs, int level, int colour, int count, cudaStream_t s);
+void launch_small_colour_batch(const BatchJob<Real> *jobs, int level, int colour, int count, cudaStream_t s, bool after);
 template <typename Real>
-void launch_colour_batch(const BatchJob<Real> *jobs, int level, int colour, int count, int tile, cudaStream_t s);
+bool launch_colour_batch(const BatchJob<Real> *jobs, int level, int colour, int count, int tile, cudaStream_t s, bool after);
 // fine += P coarse for jobs[0..count) (src coarse, dst fine)
 template <typename Real>
 void launch_prolong_add_batch(const XferJob *jobs, int coarseLevel, int count, cudaStream_t s);

@@ -507,6 +507,7 @@ __device__ __forceinline__ void small_colour_body(const LevelPtrs<Store> &L, int
     Real a, b;
     owned_entry<Real, Store>(L, N1, node, A, r & 7, a, b);
     const int I[3] = {node / (N1 * N1), (node / N1) % N1, node % N1};
+    await_previous();
     for (int o = r; o < 27; o += 16)
     {
         const int J[3] = {I[0] + o / 9 - 1, I[1] + (o / 3) % 3 - 1, I[2] + o % 3 - 1};
@@ -517,6 +518,7 @@ __device__ __forceinline__ void small_colour_body(const LevelPtrs<Store> &L, int
     __syncwarp();
     const Real *mine = reinterpret_cast<const Real *>(around[slot]);
     const Real t = incidence16<Real, 3>(ln, mine, 13, A, r, true, a, b);
+    next_may_start();
     if (!(r & 1)) part[slot * 8 + (r >> 3) * 4 + ((r & 7) >> 1)] = t;
     __syncthreads();
     Real x[8], p;
@@ -794,7 +796,9 @@ __global__ void __launch_bounds__(128) small4_colour_kernel(LevelPtrs<double> L,
     ln.init(lane, 0.5 / 4096.0);
     double a = 0., b = 0., v[5];
     if (lane < 16) owned_entry4(L, N1, node, A, lane, a, b);
+    await_previous();
     incidence4d(ln, stride, A, lane, a, b, [&](int o) { return ld2(L.xy, node + o); }, v);
+    next_may_start();
     int own = slot;
     while ((tab[own] >> 17 & 31u) == 0) own--;
     cluster.sync();  // the cluster's blocks have started
@@ -810,27 +814,6 @@ __global__ void __launch_bounds__(128) small4_colour_kernel(LevelPtrs<double> L,
         if (!isfinite(cur)) atomicOr(err, (unsigned int)ERR_NONFINITE);
         L.xy[2 * (int64_t)node + lane] = cur;
     }
-}
-
-// a launch of `count` blocks or clusters; the blocks of a cluster on SMs of their own where the device can
-template <typename Kernel, typename... Args>
-void launch_small(Kernel kernel, int nc, int count, int threads, size_t smem, cudaStream_t s, Args... args)
-{
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3((unsigned)(nc * count), 1, 1);
-    cfg.blockDim = dim3((unsigned)threads, 1, 1);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = s;
-    cudaLaunchAttribute attr[2];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = (unsigned)nc;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    attr[1].id = cudaLaunchAttributeClusterSchedulingPolicyPreference;
-    attr[1].val.clusterSchedulingPolicyPreference = cudaClusterSchedulingPolicySpread;
-    cfg.attrs = attr;
-    cfg.numAttrs = nc > 1 ? 2 : 0;
-    cudaLaunchKernelEx(&cfg, kernel, args...);
 }
 
 template <typename F>
@@ -926,7 +909,7 @@ void launch_small_level(const LevelPtrs<Store> &L, int iters, unsigned int *err,
     with_shape<Store>(L.level, [&](auto lv, auto nb) {
         constexpr int LEVEL = decltype(lv)::value, NB = decltype(nb)::value;
         using SH = SmallShape<Store, LEVEL, NB>;
-        launch_small(small_kernel<Store, LEVEL, NB>, NB, 1, SH::kThreads, SH::kBytes, s, L, iters, err, separate, kexp);
+        launch_colour(small_kernel<Store, LEVEL, NB>, dim3(NB), NB, SH::kThreads, SH::kBytes, s, false, L, iters, err, separate, kexp);
     });
 }
 
@@ -937,48 +920,50 @@ void launch_small_level_batch(const BatchJob<Store> *jobs, int level, int count,
     with_shape<Store>(level, [&](auto lv, auto nb) {
         constexpr int LEVEL = decltype(lv)::value, NB = decltype(nb)::value;
         using SH = SmallShape<Store, LEVEL, NB>;
-        launch_small(small_batch_kernel<Store, LEVEL, NB>, NB, count, SH::kThreads, SH::kBytes, s, jobs);
+        launch_colour(small_batch_kernel<Store, LEVEL, NB>, dim3(NB * count), NB, SH::kThreads, SH::kBytes, s, false, jobs);
     });
 }
 
 template <typename Store>
-void launch_small_colour(const LevelPtrs<Store> &L, int colour, unsigned int *err, cudaStream_t s, int separate, const int *kexp)
+void launch_small_colour(const LevelPtrs<Store> &L, int colour, unsigned int *err, cudaStream_t s, int separate, const int *kexp, bool after)
 {
     with_level(L.level, [&](auto lv) {
         constexpr int LEVEL = decltype(lv)::value;
-        if constexpr (LEVEL < 4 || std::is_same<Store, double>::value) small_colour_kernel<Store, LEVEL><<<(ipow(8, LEVEL) + 7) / 8, 128, 0, s>>>(L, colour, err, separate, kexp);
+        if constexpr (LEVEL < 4 || std::is_same<Store, double>::value)
+            launch_colour(small_colour_kernel<Store, LEVEL>, dim3((ipow(8, LEVEL) + 7) / 8), 1, 128, 0, s, after, L, colour, err, separate, kexp);
     });
 }
 
 template <typename Store>
-void launch_small_colour_batch(const BatchJob<Store> *jobs, int level, int colour, int count, cudaStream_t s)
+void launch_small_colour_batch(const BatchJob<Store> *jobs, int level, int colour, int count, cudaStream_t s, bool after)
 {
     for (int m0 = 0; m0 < count; m0 += 65535)
         with_level(level, [&](auto lv) {
             constexpr int LEVEL = decltype(lv)::value;
-            if constexpr (LEVEL < 4 || std::is_same<Store, double>::value) small_colour_batch_kernel<Store, LEVEL>
-                <<<dim3((ipow(8, LEVEL) + 7) / 8, (unsigned)std::min(65535, count - m0)), 128, 0, s>>>(jobs + m0, colour);
+            if constexpr (LEVEL < 4 || std::is_same<Store, double>::value)
+                launch_colour(small_colour_batch_kernel<Store, LEVEL>, dim3((ipow(8, LEVEL) + 7) / 8, (unsigned)std::min(65535, count - m0)), 1, 128,
+                              0, s, after || m0 > 0, jobs + m0, colour);
         });
 }
 
 bool launch_small4(const LevelPtrs<double> &L, int iters, unsigned int *err, cudaStream_t s, int separate)
 {
-    if (L.level == 0) launch_small(small4_kernel<0>, 1, 1, 32, 0, s, L, iters, err, separate);
-    else if (L.level == 1) launch_small(small4_kernel<1>, 4, 1, 128, 0, s, L, iters, err, separate);
+    if (L.level == 0) launch_colour(small4_kernel<0>, dim3(1), 1, 32, 0, s, false, L, iters, err, separate);
+    else if (L.level == 1) launch_colour(small4_kernel<1>, dim3(4), 4, 128, 0, s, false, L, iters, err, separate);
     else return false;
     return true;
 }
-void launch_small4_colour(const LevelPtrs<double> &L, int colour, unsigned int *err, cudaStream_t s, int separate)
+void launch_small4_colour(const LevelPtrs<double> &L, int colour, unsigned int *err, cudaStream_t s, int separate, bool after)
 {
-    if (L.level == 2) launch_small(small4_colour_kernel<2>, 4, 16, 128, 0, s, L, colour, err, separate);
-    else launch_small(small4_colour_kernel<3>, 4, 256, 128, 0, s, L, colour, err, separate);
+    if (L.level == 2) launch_colour(small4_colour_kernel<2>, dim3(64), 4, 128, 0, s, after, L, colour, err, separate);
+    else launch_colour(small4_colour_kernel<3>, dim3(1024), 4, 128, 0, s, after, L, colour, err, separate);
 }
 
 #define EPR_SMALL(T)                                                                                              \
     template void launch_small_level<T>(const LevelPtrs<T> &, int, unsigned int *, cudaStream_t, int, int *);      \
     template void launch_small_level_batch<T>(const BatchJob<T> *, int, int, cudaStream_t);                       \
-    template void launch_small_colour<T>(const LevelPtrs<T> &, int, unsigned int *, cudaStream_t, int, const int *); \
-    template void launch_small_colour_batch<T>(const BatchJob<T> *, int, int, int, cudaStream_t);
+    template void launch_small_colour<T>(const LevelPtrs<T> &, int, unsigned int *, cudaStream_t, int, const int *, bool); \
+    template void launch_small_colour_batch<T>(const BatchJob<T> *, int, int, int, cudaStream_t, bool);
 EPR_SMALL(float)
 EPR_SMALL(double)
 EPR_SMALL(df)

@@ -375,7 +375,8 @@ __device__ __forceinline__ void apply_step(const LevelPtrs<Real> &L, Real *xy, i
 // not move along; so each neighbour is one of the corners already in the lane's registers.
 // Ac, Bc (optional): the colour's block of the colour-blocked stencils, the node being the colour's
 // jc-th of nc; otherwise the natural stencils L.A, L.B are read.
-template <int D, typename Real>
+// Chained: the caller is a colour's kernel, which may start before the colour ahead of it is done.
+template <int D, typename Real, bool Chained = false>
 __device__ __forceinline__ void gs_update_lanes_at(const LevelPtrs<Real> &L, Real *xy, const Grid<D> &g, const int *I, bool active,
                                                    int A, unsigned int *err, int separate = 0, const Real *Ac = nullptr,
                                                    const Real *Bc = nullptr, int64_t jc = 0, int64_t nc = 0)
@@ -411,6 +412,29 @@ __device__ __forceinline__ void gs_update_lanes_at(const LevelPtrs<Real> &L, Rea
         i = iu;
         if (ok)
         {
+            const int64_t step = Ac ? nc : L.N;
+            const Real *pA = (Ac ? Ac + jc : L.A + i) + (int64_t)Dims<D>::CENTER * step;
+            const Real *pB = (Ac ? Bc + jc : L.B + i) + (int64_t)Dims<D>::CENTER * step;
+            int64_t so[D];
+#pragma unroll
+            for (int d = 0; d < D; d++) so[d] = cbit<D>(A, d) ? -(int64_t)ipow(3, D - 1 - d) * step : (int64_t)ipow(3, D - 1 - d) * step;
+            const int other = A ^ first;
+            Real ca[C], cb[C];
+#pragma unroll
+            for (int cc = 0; cc < C; cc++)
+            {
+                ca[cc] = cb[cc] = (Real)0;
+                if ((other & ~cc & (C - 1)) == 0)
+                {
+                    int64_t o = 0;
+#pragma unroll
+                    for (int d = 0; d < D; d++)
+                        if (cbit<D>(cc, d)) o += so[d];
+                    ca[cc] = pA[o];
+                    if (cc) cb[cc] = pB[o];
+                }
+            }
+            if constexpr (Chained) await_previous();
 #pragma unroll
             for (int cc = 0; cc < C; cc++)
             {
@@ -420,25 +444,13 @@ __device__ __forceinline__ void gs_update_lanes_at(const LevelPtrs<Real> &L, Rea
                     if (cbit<D>(cc, d)) jj += sd[d];
                 f[cc] = ld2(xy, (int64_t)(uint32_t)jj);
             }
-            const int64_t step = Ac ? nc : L.N;
-            const Real *pA = (Ac ? Ac + jc : L.A + i) + (int64_t)Dims<D>::CENTER * step;
-            const Real *pB = (Ac ? Bc + jc : L.B + i) + (int64_t)Dims<D>::CENTER * step;
-            int64_t so[D];
-#pragma unroll
-            for (int d = 0; d < D; d++) so[d] = cbit<D>(A, d) ? -(int64_t)ipow(3, D - 1 - d) * step : (int64_t)ipow(3, D - 1 - d) * step;
-            const int other = A ^ first;
+            acen = ca[0];
 #pragma unroll
             for (int cc = 0; cc < C; cc++)
                 if ((other & ~cc & (C - 1)) == 0)
                 {
-                    int64_t o = 0;
-#pragma unroll
-                    for (int d = 0; d < D; d++)
-                        if (cbit<D>(cc, d)) o += so[d];
-                    const Real a = pA[o];
-                    av = O::fma(a, f[cc], av);
-                    if (cc == 0) acen = a;
-                    else bv = O::fma(pB[o], f[cc], bv);
+                    av = O::fma(ca[cc], f[cc], av);
+                    if (cc) bv = O::fma(cb[cc], f[cc], bv);
                 }
 #pragma unroll
             for (int cc = 1; cc < C; cc++) f[cc] = O::sub(f[cc], f[0]);
@@ -506,6 +518,7 @@ __device__ __forceinline__ void gs_update_pair3(const LevelPtrs<Real> &L, Real *
         const typename PL::Vec *pc = reinterpret_cast<const typename PL::Vec *>(stencils) + 2 * jc + s;
 #pragma unroll
         for (int v = 0; v < PL::G; v++) cv[v] = stream_load(pc + 2 * v * nc);
+        await_previous();
         if (side && lo1 && hi1 && lo2 && hi2)
         {
 #pragma unroll
@@ -610,11 +623,22 @@ __device__ __forceinline__ void gs_update_pair3(const LevelPtrs<Real> &L, Real *
             }
         fit_to_model<3, Real>(sums, wedge_scale<3, Real>(g.r), av, bv, acen, sh, q);
     }
+    if constexpr (sizeof(Real) == 8) next_may_start();
 #pragma unroll
     for (int k = 0; k < 5; k++) q[k] = O::add(q[k], __shfl_xor_sync(0xffffffffu, q[k], 1));
     if (!active || s) return;
     apply_step<Real>(L, xy, i, q, sh, separate, err);
 }
+
+// Whether a level's colours start ahead of the end of the colour before (launch_colour).  Depth 8, all sweeps
+// of a level, chained against not: float levels 4, 5, 6: 2.5, 1.5, 1.8 ms against 4.0, 2.3, 2.0, and 0.6 ms less
+// each of levels 7 and 8; double level 3: 10.7 against 13.0, level 6: 49.1 against 49.8.  The blocks that start
+// early are placed where the colour before leaves room, so they are spread unevenly: of no account where
+// latency counts, but where a few blocks per SM keep the FP64 pipe busy the kernel waits for the fullest SM.  So
+// in double a block lets the next colour start only when its own FP64 work is done (level 4: 12.2 ms; at its
+// start: 37.5; unchained: 12.4), and a lane per element in double (level 5: 18.0 ms; chained: 21.0) is not chained.
+template <typename Real, bool Pair>
+__host__ __device__ constexpr bool chains_colours() { return sizeof(Real) == 4 || Pair; }
 
 // lanes per node of the colour kernels of the large levels
 template <int D, bool Pair>
@@ -634,6 +658,7 @@ template <int D, typename Real, bool Pair>
 __device__ __forceinline__ void gs_node_lanes(const LevelPtrs<Real> &L, const Grid<D> &g, const int *I, bool active, int lane, unsigned int *err,
                                               int separate, const Colour<D> &col, int64_t cbBase, int64_t jc)
 {
+    if constexpr (sizeof(Real) == 4) next_may_start();
     if constexpr (Pair)
     {
         // a colour's block starts after 27 values per node of the colours before it
@@ -641,7 +666,7 @@ __device__ __forceinline__ void gs_node_lanes(const LevelPtrs<Real> &L, const Gr
         return;
     }
     const Real *Ac = L.Acb ? L.Acb + cbBase : nullptr, *Bc = L.Bcb ? L.Bcb + cbBase : nullptr;
-    if constexpr (!Pair) gs_update_lanes_at<D, Real>(L, L.xy, g, I, active, lane, err, separate, Ac, Bc, jc, col.n);
+    if constexpr (!Pair) gs_update_lanes_at<D, Real, true>(L, L.xy, g, I, active, lane, err, separate, Ac, Bc, jc, col.n);
 }
 
 // One colour, groups of lanes along the colour's nodes of the last two axes: grid.x = blocks of
@@ -988,34 +1013,44 @@ void launch_quadfit(const LevelPtrs<Real> &L, const Real *xy, double *out, cudaS
 }
 
 template <int D, typename Real>
-void launch_gs_colour(const LevelPtrs<Real> &L, int colour, unsigned int *err, cudaStream_t s, int separate)
+bool launch_gs_colour(const LevelPtrs<Real> &L, int colour, unsigned int *err, cudaStream_t s, int separate, bool after)
 {
     Grid<D> g(L.level);
     Colour<D> col(g, colour);
-    if (col.n == 0) return;
+    if (col.n == 0) return false;
     if constexpr (D == 3)
-        if (small_colour_level<Real>(L.level)) return launch_small_colour<Real>(L, colour, err, s, separate, nullptr);
+        if (small_colour_level<Real>(L.level))
+        {
+            launch_small_colour<Real>(L, colour, err, s, separate, nullptr, after);
+            return true;
+        }
     if constexpr (D == 4 && std::is_same<Real, double>::value)
-        if (small4_colour_level(L.level)) return launch_small4_colour(L, colour, err, s, separate);
+        if (small4_colour_level(L.level))
+        {
+            launch_small4_colour(L, colour, err, s, separate, after);
+            return true;
+        }
     const int64_t cb = colour_block_base<D>(g, colour);
     auto launch = [&](auto pair) {
         constexpr bool Pair = decltype(pair)::value;
         constexpr int NPB = kThreads / lanes_per_node<D, Pair>();
+        const bool chained = after && chains_colours<Real, Pair>();
         if (L.alist)
         {
             // adaptive level: only the colour's active nodes
             const int count = L.aoff[colour + 1] - L.aoff[colour];
             if (count > 0)
-                gs_colour_lanes_list_kernel<D, Real, Pair><<<blocks_for(count, NPB), kThreads, 0, s>>>(L, col, cb, L.alist + L.aoff[colour],
-                                                                                                      count, err, separate);
-            return;
+                launch_colour(gs_colour_lanes_list_kernel<D, Real, Pair>, dim3(blocks_for(count, NPB)), 1, kThreads, 0, s, chained, L, col, cb,
+                              L.alist + L.aoff[colour], count, err, separate);
+            return count > 0;
         }
         dim3 grid(blocks_for((int64_t)col.cnt[D - 2] * col.cnt[D - 1], NPB), (unsigned)(D == 3 ? col.cnt[0] : col.cnt[0] * col.cnt[1]));
-        gs_colour_lanes_kernel<D, Real, Pair><<<grid, kThreads, 0, s>>>(L, col, cb, err, separate);
+        launch_colour(gs_colour_lanes_kernel<D, Real, Pair>, grid, 1, kThreads, 0, s, chained, L, col, cb, err, separate);
+        return true;
     };
     if constexpr (D == 3)
         if (pair_level<D>(L.level)) return launch(std::true_type{});
-    launch(std::false_type{});
+    return launch(std::false_type{});
 }
 
 void prepare_gs_kernels()
@@ -1049,8 +1084,13 @@ int launch_gs_sweeps(const LevelPtrs<Real> &L, int iters, unsigned int *err, cud
             return 1;
         }
     int n = 0;
+    bool after = false;
     for (int it = 0; it < iters; it++)
-        for (int c = 0; c < (1 << D); c++) { launch_gs_colour<D, Real>(L, c, err, s, separate); n++; }
+        for (int c = 0; c < (1 << D); c++)
+        {
+            after = launch_gs_colour<D, Real>(L, c, err, s, separate, after) || after;
+            n++;
+        }
     return n;
 }
 
@@ -1188,41 +1228,47 @@ void launch_convert_f2d(const float *in, double *out, int64_t n, cudaStream_t st
 // lockstep batches (3D)
 // ---------------------------------------------------------------------------------------------
 template <typename Real, int TPB, bool Pair>
-static void launch_lanes_batch_as(const BatchJob<Real> *jobs, const Colour<3> &col, int64_t cb, int count, cudaStream_t s)
+static void launch_lanes_batch_as(const BatchJob<Real> *jobs, const Colour<3> &col, int64_t cb, int count, cudaStream_t s, bool after)
 {
     constexpr int NPB = TPB / lanes_per_node<3, Pair>();
     // grid.y = reconstruction x axis-0 count, at most 65,535: chunks of reconstructions
     const int per = std::max(1, 65535 / col.cnt[0]);
+    constexpr bool chained = chains_colours<Real, Pair>();
     for (int m0 = 0; m0 < count; m0 += per)
     {
         const int cnt = std::min(per, count - m0);
         dim3 grid(blocks_for((int64_t)col.cnt[1] * col.cnt[2], NPB), (unsigned)(cnt * col.cnt[0]));
-        gs_colour_lanes_batch_kernel<Real, TPB, Pair><<<grid, TPB, 0, s>>>(jobs + m0, col, cb);
+        launch_colour(gs_colour_lanes_batch_kernel<Real, TPB, Pair>, grid, 1, TPB, 0, s, chained && (after || m0 > 0), jobs + m0, col, cb);
     }
 }
 template <typename Real, int TPB>
 static void launch_lanes_batch(const BatchJob<Real> *jobs, int level, const Colour<3> &col, int64_t cb, int count,
-                               cudaStream_t s)
+                               cudaStream_t s, bool after)
 {
-    if (pair_level<3>(level)) launch_lanes_batch_as<Real, TPB, true>(jobs, col, cb, count, s);
-    else launch_lanes_batch_as<Real, TPB, false>(jobs, col, cb, count, s);
+    if (pair_level<3>(level)) launch_lanes_batch_as<Real, TPB, true>(jobs, col, cb, count, s, after);
+    else launch_lanes_batch_as<Real, TPB, false>(jobs, col, cb, count, s, after);
 }
 
 template <typename Real>
-void launch_colour_batch(const BatchJob<Real> *jobs, int level, int colour, int count, int tile, cudaStream_t s)
+bool launch_colour_batch(const BatchJob<Real> *jobs, int level, int colour, int count, int tile, cudaStream_t s, bool after)
 {
-    if (count <= 0) return;
+    if (count <= 0) return false;
     Grid<3> g(level);
     Colour<3> col(g, colour);
-    if (col.n == 0) return;
+    if (col.n == 0) return false;
     const int64_t cb = colour_block_base<3>(g, colour);
-    if (small_colour_level<Real>(level)) return launch_small_colour_batch<Real>(jobs, level, colour, count, s);
-    if constexpr (std::is_same<Real, df>::value) return;  // double-float levels are 3D levels <= 3
+    if (small_colour_level<Real>(level))
+    {
+        launch_small_colour_batch<Real>(jobs, level, colour, count, s, after);
+        return true;
+    }
+    if constexpr (std::is_same<Real, df>::value) return false;  // double-float levels are 3D levels <= 3
     else
     {
-        if (tile == 0) launch_lanes_batch<Real, 64>(jobs, level, col, cb, count, s);
-        else if (tile == 2) launch_lanes_batch<Real, 256>(jobs, level, col, cb, count, s);
-        else launch_lanes_batch<Real, 128>(jobs, level, col, cb, count, s);
+        if (tile == 0) launch_lanes_batch<Real, 64>(jobs, level, col, cb, count, s, after);
+        else if (tile == 2) launch_lanes_batch<Real, 256>(jobs, level, col, cb, count, s, after);
+        else launch_lanes_batch<Real, 128>(jobs, level, col, cb, count, s, after);
+        return true;
     }
 }
 
@@ -1250,9 +1296,9 @@ void launch_df_push_batch(const XferJob *jobs, int64_t n, int level, int count, 
     if (count > 0 && n) df_push_batch_kernel<<<count, 256, 0, s>>>(jobs, n, level);
 }
 
-template void launch_colour_batch<float>(const BatchJob<float> *, int, int, int, int, cudaStream_t);
-template void launch_colour_batch<double>(const BatchJob<double> *, int, int, int, int, cudaStream_t);
-template void launch_colour_batch<df>(const BatchJob<df> *, int, int, int, int, cudaStream_t);
+template bool launch_colour_batch<float>(const BatchJob<float> *, int, int, int, int, cudaStream_t, bool);
+template bool launch_colour_batch<double>(const BatchJob<double> *, int, int, int, int, cudaStream_t, bool);
+template bool launch_colour_batch<df>(const BatchJob<df> *, int, int, int, int, cudaStream_t, bool);
 template void launch_prolong_add_batch<float>(const XferJob *, int, int, cudaStream_t);
 template void launch_prolong_add_batch<double>(const XferJob *, int, int, cudaStream_t);
 
@@ -1260,7 +1306,7 @@ template void launch_prolong_add_batch<double>(const XferJob *, int, int, cudaSt
     template void launch_energy<D, R>(const LevelPtrs<R> &, const R *, const Reduce &, cudaStream_t);   \
     template void launch_quadfit<D, R>(const LevelPtrs<R> &, const R *, double *, cudaStream_t);        \
     template void launch_grad_norm<D, R>(const LevelPtrs<R> &, const R *, const Reduce &, cudaStream_t); \
-    template void launch_gs_colour<D, R>(const LevelPtrs<R> &, int, unsigned int *, cudaStream_t, int); \
+    template bool launch_gs_colour<D, R>(const LevelPtrs<R> &, int, unsigned int *, cudaStream_t, int, bool); \
     template int launch_gs_sweeps<D, R>(const LevelPtrs<R> &, int, unsigned int *, cudaStream_t, int); \
     template void launch_gn_matvec<D, R>(const LevelPtrs<R> &, const R *, const R *, R *, cudaStream_t); \
     template void launch_prolong<D, R>(int, const R *, R *, int, cudaStream_t, const uint8_t *);                         \

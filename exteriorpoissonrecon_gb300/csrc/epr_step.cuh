@@ -9,6 +9,46 @@
 
 namespace epr {
 
+// Colours of a sweep follow each other as launches of a few microseconds.  Each lets the next one's blocks
+// start as soon as its own have (next_may_start), which then load what no colour writes, the stencils and
+// tables, and wait for the whole of it, its writes included, before they touch a coefficient
+// (await_previous).  Chained that way a launch also waits for every one before: the one it waits for cannot
+// end before its own wait.  Without the attribute (launch_colour's first) both do nothing.
+__device__ __forceinline__ void next_may_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void await_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+// a colour's launch of `grid` blocks, in clusters of nc (on SMs of their own where the device can).
+// after: the launch before it on the stream is a colour too; the first of a sequence must follow what
+// wrote the stencils in full
+template <typename... P, typename... A>
+void launch_colour(void (*kernel)(P...), dim3 grid, int nc, int threads, size_t smem, cudaStream_t s, bool after, A... args)
+{
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3((unsigned)threads, 1, 1);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute attr[3];
+    int n = 0;
+    if (nc > 1)
+    {
+        attr[n].id = cudaLaunchAttributeClusterDimension;
+        attr[n].val.clusterDim.x = (unsigned)nc;
+        attr[n].val.clusterDim.y = 1;
+        attr[n++].val.clusterDim.z = 1;
+        attr[n].id = cudaLaunchAttributeClusterSchedulingPolicyPreference;
+        attr[n++].val.clusterSchedulingPolicyPreference = cudaClusterSchedulingPolicySpread;
+    }
+    if (after)
+    {
+        attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[n++].val.programmaticStreamSerializationAllowed = 1;
+    }
+    cfg.attrs = attr;
+    cfg.numAttrs = n;
+    cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+}
+
 template <typename Real>
 __device__ __forceinline__ Real2<Real> ld2(const Real *xy, int64_t i)
 {
