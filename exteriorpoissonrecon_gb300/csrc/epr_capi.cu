@@ -285,6 +285,18 @@ bool Context::gs(int l, int iters)
     return launch_ok("gs");
 }
 
+bool Context::sweeps(int l, int iters)
+{
+    // solves relax in float with the modal fit; a caller's own sweeps keep the Gauss rule's bits
+    if (iters <= 0 || !lvl32(l) || !(dim == 3 ? gauss_level<3>(l) : gauss_level<4>(l))) return gs(l, iters);
+    launches += with_dim(this, [&](auto dd) {
+        constexpr int D = decltype(dd)::value;
+        return launch_gauss_sweeps<D>(level_ptrs<float>(this, l), iters, d_err, stream, P.separate);
+    });
+    stats.node_updates += (int64_t)iters * levels[l].N;
+    return launch_ok("sweeps");
+}
+
 bool Context::check_errors()
 {
     unsigned int h = 0;
@@ -820,7 +832,7 @@ int epr_gs(epr_ctx *ctx, int level, int iters)
     EPR_CHECK_CTX(ctx);
     EPR_CHECK_LEVEL(ctx, level);
     if (iters < 0) { ctx->fail(EPR_ERR_ARG, "negative iteration count"); return EPR_ERR_ARG; }
-    EPR_RETURN(ctx, ctx->gs(level, iters) && ctx->check_errors());
+    EPR_RETURN(ctx, ctx->sweeps(level, iters) && ctx->check_errors());
 }
 
 int epr_prolong(epr_ctx *ctx, int level)

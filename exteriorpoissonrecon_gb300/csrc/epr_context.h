@@ -124,6 +124,7 @@ struct Context
     bool pull_xy(int l);
     bool energy(int l, double *out3);
     bool gs(int l, int iters);
+    bool sweeps(int l, int iters);  // gs for a caller that runs sweeps by itself (epr_gs)
     bool relax_levels(int minD, int maxD, bool useGraph);
     bool check_errors();
     bool prolong_add(int l);

