@@ -56,7 +56,7 @@ sys.path.insert(0, ROOT)
 # depth-7 launch (profiles/gs_colour_lanes_kernel_link_depth7_fp32.txt,
 # profiles/linear_gs_colour_kernel_link_depth7_fp32.txt); a depth-8 launch's traffic is these times
 # its colour nodes (traffic grows in proportion with the nodes).
-GS_DRAM_BYTES_PER_COLOUR_NODE_FP32 = (76.39296e6 + 4.034304e6) / 274625
+GS_DRAM_BYTES_PER_COLOUR_NODE_FP32 = (78.715904e6 + 1.755392e6) / 274625
 LGS_DRAM_BYTES_PER_COLOUR_NODE_FP32 = (42.062336e6 + 768) / 274625
 
 
@@ -273,12 +273,11 @@ def kernel_rooflines(r, dim, depth, precision, clk):
     gs_bytes = 2 * rs * N + colour_nodes * (2 * S * rs + 2 * rs)
     achieved = gs_bytes / (gs_ms * 1e-3) / 1e9
     fp32 = precision == "fp32" and dim == 3  # the captures are of the 3D float kernels
-    # the quartic relaxation is bound by FP32/FP64 issue, not by HBM: its algorithmic FLOPs per node
-    # update (this formulation: per incident element and wedge component 4 derivative tables of
-    # ~34 flops and 2 x 2 x 3^(D-2) Gauss points of ~21 flops; plus the 3^D-point stencil column)
-    # against the nominal FP32 rate of 152 SMs x 128 lanes x 2 flops at the sampled SM clock
-    K = dim * (dim - 1) // 2
-    node_flops = (2 ** dim) * K * (4 * 34 + 4 * 3 ** (dim - 2) * 21) + 8 * S + 30
+    # the quartic relaxation is bound by FP32/FP64 issue and load latency: its algorithmic FLOPs per node
+    # update (the modal fit, per incident element: signed sums of the corner differences, six squares
+    # and six Gauss-Jacobi points in 3D, 24 points with two squares each in 4D; plus the 3^D-point
+    # stencil column) against the nominal FP32 rate of 152 SMs x 128 lanes x 2 flops at the sampled SM clock
+    node_flops = (2 ** dim) * {3: 366, 4: 1934}[dim] + 8 * S + 30
     gs_flops = node_flops * colour_nodes
     sm_mhz = (clk or {}).get("sm_mhz") or 2070.0
     fp32_nominal = 152 * 128 * 2 * sm_mhz * 1e6 / 1e12
@@ -287,7 +286,7 @@ def kernel_rooflines(r, dim, depth, precision, clk):
     roofline = {"bound": "hbm", "kernel": "gs_colour_lanes_kernel", "achieved": achieved, "peak": hbm_peak,
                 "unit": "GB/s", "frac": achieved / hbm_peak, "peak_source": peak_kind, "traffic": gs_traffic,
                 "launch_ms": gs_ms, "algorithmic_bytes_per_launch": gs_bytes,
-                "note": ("FMA-bound quartic relaxation; bytes = coefficient read + stencil columns + update writes; "
+                "note": ("issue-bound quartic relaxation; bytes = coefficient read + stencil columns + update writes; "
                          "the finest level's colour launches take share_of_step of the step, the rest is the "
                          "coarser levels (levels 0-3: thousands of latency-bound launches)"),
                 "compute": {"algorithmic_flops_per_launch": gs_flops, "achieved_tflops": gs_flops / (gs_ms * 1e-3) / 1e12,

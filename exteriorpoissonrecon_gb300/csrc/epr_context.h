@@ -26,8 +26,8 @@ struct Level
     float *A32 = nullptr;     // (none on float pair levels: the pair layout and the double stencils)
     float *B32 = nullptr;
     float *tmp32 = nullptr;
-    void *Acb = nullptr;      // colour-blocked A and B in the level's precision (levels relaxed
-    void *Bcb = nullptr;      // by one kernel per colour)
+    void *Acb = nullptr;      // colour-blocked A and B in the level's precision (levels relaxed by one
+    void *Bcb = nullptr;      // kernel per colour; on pair levels both in Acb, the pair layout)
     df *xyd = nullptr;        // double-float copies of a coarse band level (coefficients stored
     df *Ad = nullptr;         // as x 2^-k, k = d_kexp[level]; stencils unscaled)
     df *Bd = nullptr;
