@@ -181,6 +181,8 @@ void set_global_error(const std::string &msg);
 bool add_dirichlet(Context &c, int level);
 // A64[level] += w K and the level's pair layout from A64 and B64 (3D levels from kPairLevel on)
 bool pair_system(Context &c, int level, double w);
+// backs a caller's output array with memory before the device copies into it
+void populate(void *p, size_t bytes);
 bool add_dirichlet_to(Context &c, int level, double *dst, double w);
 
 }  // namespace epr

@@ -330,6 +330,11 @@ int epr_generate_samples(int device, const epr_sampler *sp, size_t n, double *po
     if (cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking) != cudaSuccess) { cudaGetLastError(); epr::set_global_error("stream"); return EPR_ERR_CUDA; }
     epr::Generated g;
     cudaError_t e = D == 3 ? epr::generate<3>(*sp, (int64_t)n, s, g) : epr::generate<4>(*sp, (int64_t)n, s, g);
+    if (e == cudaSuccess)
+    {
+        epr::populate(pos, sizeof(double) * D * g.total);
+        epr::populate(skew, sizeof(double) * K * g.total);
+    }
     if (e == cudaSuccess) e = cudaMemcpyAsync(pos, g.pos, sizeof(double) * D * g.total, cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaMemcpyAsync(skew, g.skew, sizeof(double) * K * g.total, cudaMemcpyDeviceToHost, s);
     if (g.pos) cudaFreeAsync(g.pos, s);

@@ -1723,6 +1723,7 @@ bool Setup::get(Context &c, const std::string &name, double *out, size_t cap, si
         if (!out) return true;
         if (!src) { c.fail(EPR_ERR_STATE, "'%s' is not available before epr_build", name.c_str()); return false; }
         if (cap < num) { c.fail(EPR_ERR_ARG, "output too small (%zu < %zu)", cap, num); return false; }
+        populate(out, sizeof(double) * num);
         return c.cuda_ok(cudaMemcpyAsync(out, src, sizeof(double) * num, cudaMemcpyDeviceToHost, c.stream), "copy") &&
                c.cuda_ok(cudaStreamSynchronize(c.stream), "sync");
     };

@@ -146,6 +146,8 @@ int epr_get_regular_coefficients(epr_ctx *ctx, double *x, double *y)
     if (ok)
     {
         gather_pairs_kernel<<<nblk(Nf, 256), 256, 0, s>>>(a, nullptr, Nf, planar, planar + Nf);
+        populate(x, sizeof(double) * Nf);
+        populate(y, sizeof(double) * Nf);
         ok = ctx->launch_ok("regular coefficients") &&
              ctx->cuda_ok(cudaMemcpyAsync(x, planar, sizeof(double) * Nf, cudaMemcpyDeviceToHost, s), "copy") &&
              ctx->cuda_ok(cudaMemcpyAsync(y, planar + Nf, sizeof(double) * Nf, cudaMemcpyDeviceToHost, s), "copy") &&
