@@ -154,7 +154,7 @@ bool Context::sync_system32(int l)
         // the small levels' kernels read the stencils in natural order
         launch_d2df(L.A64, L.Ad, (int64_t)S * L.N, stream);
         launch_d2df(L.B64, L.Bd, (int64_t)S * L.N, stream);
-        return launch_ok("convert system");
+        return L.synced = launch_ok("convert system");
     }
     // the small levels read the natural order
     if (dim == 3 ? !(lvl32(l) ? small_colour_level<float>(l) : small_colour_level<double>(l)) : lvl32(l) ? L.N > 81 : l > 3)
@@ -162,7 +162,9 @@ bool Context::sync_system32(int l)
         if (dim == 3 && pair_level<3>(l)) return pair_system(*this, l, 0.);
         const size_t real = lvl32(l) ? sizeof(float) : sizeof(double);
         const size_t bytes = S * L.N * real;
-        if (!L.Acb && (!alloc(&L.Acb, bytes, "alloc colour blocks") || !alloc(&L.Bcb, bytes, "alloc colour blocks"))) return false;
+        // one array for both: either none is there or both are
+        if (!L.Acb && !alloc(&L.Acb, 2 * bytes, "alloc colour blocks")) return false;
+        L.Bcb = (char *)L.Acb + bytes;
         auto blocks = [&](auto dd) {
             constexpr int D = decltype(dd)::value;
             if (lvl32(l))
@@ -179,7 +181,14 @@ bool Context::sync_system32(int l)
         if (dim == 3) blocks(std::integral_constant<int, 3>{});
         else blocks(std::integral_constant<int, 4>{});
     }
-    return launch_ok("convert system");
+    return L.synced = launch_ok("convert system");
+}
+
+// The copies of a level that no build and no epr_set_level_system has reached: those of its double stencils,
+// which are zero from the start
+bool Context::level_ready(int l)
+{
+    return !(lvl32(l) || lvlDF(l)) || levels[l].synced || sync_system32(l);
 }
 
 // device coefficients <-> the precision the solve works in
@@ -213,7 +222,7 @@ Context::~Context()
         for (Level &L : levels)
         {
             release(L.xy64); release(L.xy32); release(L.A64); release(L.B64); release(L.A32); release(L.B32);
-            release(L.tmp64); release(L.tmp32); release(L.Acb); release(L.Bcb);
+            release(L.tmp64); release(L.tmp32); release(L.Acb);
             release(L.xyd); release(L.Ad); release(L.Bd);
         }
         release(red.partial); release(red.out); release(d_err); release(d_fit); release(d_kexp);
@@ -290,6 +299,7 @@ bool Context::gs(int l, int iters)
 
 bool Context::sweeps(int l, int iters)
 {
+    if (!level_ready(l)) return false;
     // solves relax in float with the modal fit; a caller's own sweeps keep the Gauss rule's bits
     if (iters <= 0 || !lvl32(l) || !(dim == 3 ? gauss_level<3>(l) : gauss_level<4>(l))) return gs(l, iters);
     launches += with_dim(this, [&](auto dd) {
@@ -842,7 +852,7 @@ int epr_quadfit(epr_ctx *ctx, int level, double *out)
     if (!out) { ctx->fail(EPR_ERR_ARG, "null output"); return EPR_ERR_ARG; }
     epr::Level &L = ctx->levels[level];
     double *d = nullptr;
-    bool ok = ctx->alloc((void **)&d, sizeof(double) * 5 * L.N, "alloc fit");
+    bool ok = ctx->level_ready(level) && ctx->alloc((void **)&d, sizeof(double) * 5 * L.N, "alloc fit");
     if (ok && ctx->lvlDF(level)) ok = ctx->pull_xy(level);  // a double-float level's fit in double
     if (ok)
     {
@@ -900,6 +910,7 @@ int epr_gn_matvec(epr_ctx *ctx, int level, const double *dx, const double *dy, d
     double *d64 = nullptr, *o64 = nullptr;
     float *d32 = nullptr, *o32 = nullptr;
     bool fp32 = ctx->lvl32(level);
+    if (!ctx->level_ready(level)) EPR_RETURN(ctx, false);
     if (ctx->lvlDF(level) && !ctx->pull_xy(level)) EPR_RETURN(ctx, false);  // evaluated in double
     bool ok = ctx->alloc((void **)&d64, sizeof(double) * 2 * L.N, "alloc") && ctx->alloc((void **)&o64, sizeof(double) * 2 * L.N, "alloc") &&
               ctx->cuda_ok(cudaMemcpyAsync(d64, h.data(), sizeof(double) * 2 * L.N, cudaMemcpyHostToDevice, ctx->stream), "upload");

@@ -27,7 +27,8 @@ struct Level
     float *B32 = nullptr;
     float *tmp32 = nullptr;
     void *Acb = nullptr;      // colour-blocked A and B in the level's precision (levels relaxed by one
-    void *Bcb = nullptr;      // kernel per colour; on pair levels both in Acb, the pair layout)
+    void *Bcb = nullptr;      // kernel per colour), in one allocation; on pair levels Acb alone, the pair layout
+    bool synced = false;      // the copies in other precisions and orders have been made from A64 and B64
     df *xyd = nullptr;        // double-float copies of a coarse band level (coefficients stored
     df *Ad = nullptr;         // as x 2^-k, k = d_kexp[level]; stencils unscaled)
     df *Bd = nullptr;
@@ -120,6 +121,7 @@ struct Context
     bool lvl32(int l) const;  // level l computes in float
     bool lvlDF(int l) const;  // level l computes in double-float (a 3D coarse band level)
     bool sync_system32(int l);
+    bool level_ready(int l);
     bool push_xy(int l);
     bool pull_xy(int l);
     bool energy(int l, double *out3);

@@ -1694,7 +1694,7 @@ bool pair_system(Context &c, int level, double w)
         pair_system_kernel<float><<<dim3(blocks, PairLayout<float>::G), 256, 0, c.stream>>>(level, w, L.A64, L.B64, (float *)L.Acb);
     else
         pair_system_kernel<double><<<dim3(blocks, PairLayout<double>::G), 256, 0, c.stream>>>(level, w, L.A64, L.B64, (double *)L.Acb);
-    return c.launch_ok("pair layout");
+    return L.synced = c.launch_ok("pair layout");
 }
 
 bool add_dirichlet(Context &c, int level) { return add_dirichlet_to(c, level, c.levels[level].A64, c.P.d_weight); }
