@@ -17,11 +17,19 @@
 //    for a warp's FP64 instruction however many of its lanes are active.
 //  * Double-float runs on loosely normalised pairs: sums keep the error term of the leading parts but are
 //    renormalised only before a product or where they are stored, so that a chain of sums costs one
-//    addition's latency each instead of thirteen operations'.
-// Float levels compute in double-float and store float: the arithmetic is not what their phases wait for.
+//    addition's latency each instead of thirteen operations'.  The sums that cancel are done in full: a node's
+//    over its lanes and incidences, the two differences of its step, the update (FullSums).
+// Float levels compute in double-float, loose throughout, and store float: the arithmetic is not what their phases
+// wait for, and its error not what their result shows.
 //
-// Levels 0, 1, 2, 3 of a depth-8 schedule (20,480, 10,240, 5,120 and 2,560 phases): 15.0, 8.6, 6.0 and 6.2 ms
-// in double-float and 48.5, 27.9, 15.5 and 13.0 ms in double.  With the incidence on 12 Gauss points of
+// Error of one and of eight sweeps in double-float against 80-bit arithmetic, as a ratio to the 12-point Gauss rule
+// on fully normalised pairs (geometric means over 140 systems of each level 0-3: random ones and those of built
+// curves at several stages of their relaxation; standard error 0.03): 1.00, 0.97, 0.91, 0.96 at 0.80, 0.69, 1.25,
+// 2.71 us a phase of a built curve's system.  All sums loose: 1.28, 1.22, 1.07, 1.18 at 0.72, 0.59, 1.17, 2.45 us;
+// every sum and product in full: 0.95, 0.89, 0.88, 0.95 at 1.03, 0.83, 1.61, 3.58 us.
+//
+// Levels 0, 1, 2, 3 of a depth-8 schedule (20,480, 10,240, 5,120 and 2,560 phases): 16.5, 9.7, 6.4 and 6.9 ms
+// in double-float and 48.8, 28.3, 15.6 and 10.6 ms in double.  With the incidence on 12 Gauss points of
 // one warp, fully normalised pairs and a launch per colour from level 2 on they took 42, 34, 33.5 and
 // 17.7 ms, and 92, 73, 58 and 29 ms.  Four lanes per incidence (a component each) were slower wherever
 // tried (double 72, 71, 38 and 24 ms; double-float level 3 on eight SMs 7.5 ms).
@@ -83,27 +91,34 @@ struct Loose<df>
     static __device__ __forceinline__ df times2(df a) { return df(2.f * a.hi, 2.f * a.lo); }
 };
 
-// -1 / (2 d): from the float reciprocal of the leading part, one (double-float) or two (double) Newton
-// corrections from the remainder
+// Sums with an error relative to the result
+template <typename Real>
+struct FullSums
+{
+    static __device__ __forceinline__ Real add(Real a, Real b) { return Ops<Real>::add(a, b); }
+    static __device__ __forceinline__ Real muladd(Real a, Real b, Real c) { return add(Loose<Real>::mul(a, b), c); }
+};
+template <>
+struct FullSums<double> : Loose<double>
+{
+};
+// the sums of a level stored as Store
+template <typename Store>
+using SmallSums = typename std::conditional<std::is_same<Store, float>::value, Loose<df>, FullSums<Store>>::type;
+
+// -1 / (2 d): in double-float from the float reciprocal of the leading part and one Newton correction from the
+// remainder
 __device__ __forceinline__ df minus_half_over(df d)
 {
     const float r = __frcp_rn(d.hi), m = -0.5f * r;
     const float rem = __fmaf_rn(-m, d.lo, __fmaf_rn(-m, d.hi, -0.5f));
     return quick_two_sum(m, __fmul_rn(rem, r));
 }
-__device__ __forceinline__ double minus_half_over(double d)
-{
-    const float f = (float)d;
-    if (!(fabsf(f) > 1e-30f && fabsf(f) < 1e30f)) return -0.5 / d;
-    const double r = (double)__frcp_rn(f);
-    double m = -0.5 * r;
-    m = __fma_rn(__fma_rn(-d, m, -0.5), r, m);
-    return __fma_rn(__fma_rn(-d, m, -0.5), r, m);
-}
+__device__ __forceinline__ double minus_half_over(double d) { return -0.5 / d; }
 
 // Component w (0 x, 1 y) of a node's step from q0, q1 (the model's Q20, Q02), cross = -Q11 / 2 and half the
 // gradient (g0, g1): -H^{-1} grad / 2, or the separate update; false where it is not applied
-template <typename Real>
+template <typename Real, typename Sum = Loose<Real>>
 __device__ __forceinline__ bool small_step(Real q0, Real q1, Real cross, Real g0, Real g1, int w, int separate, Real &p)
 {
     using L = Loose<Real>;
@@ -116,9 +131,9 @@ __device__ __forceinline__ bool small_step(Real q0, Real q1, Real cross, Real g0
         return true;
     }
     // det H = 4 d
-    const Real d = L::norm(L::muladd(q0, q1, -L::mul(cross, cross)));
+    const Real d = L::norm(Sum::muladd(q0, q1, -L::mul(cross, cross)));
     const Real a = w ? q0 : q1, ga = w ? g1 : g0, gb = w ? g0 : g1;
-    const Real n = L::norm(L::muladd(a, ga, L::mul(cross, gb)));
+    const Real n = L::norm(Sum::muladd(a, ga, L::mul(cross, gb)));
     if (!exceeds<Real>(abs_value<Real>(d), 0.25e-20)) return false;
     p = L::norm(L::mul(n, minus_half_over(d)));
     return true;
@@ -242,7 +257,7 @@ struct Lane16
 };
 
 // the lane's sum over the incidence: value 2 (k / 4) + (k / 2) % 2 of its field
-template <typename Real, int N1>
+template <typename Real, typename Sum, int N1>
 __device__ __forceinline__ Real incidence16(const Lane16<Real> &ln, const Real *xy, int node, int A, int r, bool wedge, Real a, Real b)
 {
     using L = Loose<Real>;
@@ -286,20 +301,20 @@ __device__ __forceinline__ Real incidence16(const Lane16<Real> &ln, const Real *
     }
     // sum over the field's eight lanes, the values halved with the lanes
     const bool h4 = (k & 4) != 0, h2 = (k & 2) != 0;
-    const Real t0 = L::add(h4 ? v[2] : v[0], shfl_xor_any(h4 ? v[0] : v[2], 4));
-    const Real t1 = L::add(h4 ? v[3] : v[1], shfl_xor_any(h4 ? v[1] : v[3], 4));
-    Real t = L::add(h2 ? t1 : t0, shfl_xor_any(h2 ? t0 : t1, 2));
-    t = L::add(t, shfl_xor_any(t, 1));
+    const Real t0 = Sum::add(h4 ? v[2] : v[0], shfl_xor_any(h4 ? v[0] : v[2], 4));
+    const Real t1 = Sum::add(h4 ? v[3] : v[1], shfl_xor_any(h4 ? v[1] : v[3], 4));
+    Real t = Sum::add(h2 ? t1 : t0, shfl_xor_any(h2 ? t0 : t1, 2));
+    t = Sum::add(t, shfl_xor_any(t, 1));
     return L::norm(t);
 }
 
 // The node's step by its 16 lanes, lane r the component r % 2; x[0..3] the x lanes' values, x[4..7] the y lanes'
-template <typename Real>
+template <typename Real, typename Sum>
 __device__ __forceinline__ bool group_step(const Real *x, int r, int separate, Real &p)
 {
     using L = Loose<Real>;
     const Real cross = L::norm(L::add(x[3], x[7])), g0 = L::norm(L::add(x[5], x[2])), g1 = L::norm(L::add(x[1], x[6]));
-    return small_step<Real>(x[4], x[0], cross, g0, g1, r & 1, separate, p);
+    return small_step<Real, Sum>(x[4], x[0], cross, g0, g1, r & 1, separate, p);
 }
 // the group's eight values from its lanes' sums (level 0: a single incidence)
 template <typename Real>
@@ -309,14 +324,19 @@ __device__ __forceinline__ void values_of_incidence(Real t, Real *x)
     for (int n = 0; n < 8; n++) x[n] = shfl_group<16>(t, (n >> 2) * 8 + (n & 3) * 2);
 }
 // ... from the sums of the node's cnt incidences in shared memory: lane r adds every second incidence of
-// value r % 8, the halves meet by a shuffle
-template <typename Real>
+// value r % 8 in pairs, the halves meet by a shuffle
+template <typename Real, typename Sum>
 __device__ __forceinline__ void values_of_node(const Real *part, int slot, int cnt, int r, Real *x)
 {
-    using L = Loose<Real>;
-    Real t = (Real)0;
-    for (int k = r >> 3; k < cnt; k += 2) t = L::add(t, part[(slot + k) * 8 + (r & 7)]);
-    t = L::norm(L::add(t, shfl_xor_any(t, 8)));
+    Real v[4];
+#pragma unroll
+    for (int n = 0; n < 4; n++)
+    {
+        const int k = 2 * n + (r >> 3);
+        v[n] = k < cnt ? part[(slot + k) * 8 + (r & 7)] : (Real)0;
+    }
+    Real t = Sum::add(Sum::add(v[0], v[1]), Sum::add(v[2], v[3]));
+    t = Loose<Real>::norm(Sum::add(t, shfl_xor_any(t, 8)));
 #pragma unroll
     for (int n = 0; n < 8; n++) x[n] = shfl_group<16>(t, n);
 }
@@ -347,6 +367,7 @@ __device__ __forceinline__ void small_body(const LevelPtrs<Store> &L, int iters,
     using Real = typename SH::Real;
     using V = Real2<Real>;
     using LA = Loose<Real>;
+    using Sum = SmallSums<Store>;
     constexpr int N1 = SH::N1, NN = SH::NN, IPB = SH::IPB, NC = SH::NC;
     constexpr bool kDF = std::is_same<Store, df>::value;
     extern __shared__ __align__(16) unsigned char small_smem[];
@@ -402,14 +423,14 @@ __device__ __forceinline__ void small_body(const LevelPtrs<Store> &L, int iters,
             const int node = (int)(e & 8191u), A = (int)(e >> 13) & 7, cnt = live ? (int)(e >> 16) & 15 : 0;
             const int own = 8 * (c * IPB + at) + (r & 7);
             const Real old = reinterpret_cast<const Real *>(xy)[2 * node + (r & 1)];  // before the first shuffle
-            const Real t = incidence16<Real, N1>(ln, reinterpret_cast<const Real *>(xy), node, A, r, wedge, As[own], Bs[own]);
+            const Real t = incidence16<Real, Sum, N1>(ln, reinterpret_cast<const Real *>(xy), node, A, r, wedge, As[own], Bs[own]);
             Real x[8];
             if constexpr (LEVEL == 0) values_of_incidence<Real>(t, x);
             else
             {
                 if (!(r & 1)) part[slot * 8 + (r >> 3) * 4 + ((r & 7) >> 1)] = t;
                 __syncthreads();
-                values_of_node<Real>(part, slot, cnt, r, x);
+                values_of_node<Real, Sum>(part, slot, cnt, r, x);
             }
             if constexpr (NC > 1)
                 if (pending)
@@ -418,9 +439,9 @@ __device__ __forceinline__ void small_body(const LevelPtrs<Store> &L, int iters,
                     pending = false;
                 }
             Real p;
-            if (cnt && (e >> 20 & 1u) && group_step<Real>(x, r, separate, p))
+            if (cnt && (e >> 20 & 1u) && group_step<Real, Sum>(x, r, separate, p))
             {
-                const Real cur = LA::norm(LA::add(old, p));
+                const Real cur = LA::norm(Sum::add(old, p));
                 if (r < 2 && !finite_value<Real>(cur)) atomicOr(err, (unsigned int)ERR_NONFINITE);
                 // lane r writes component r % 2 into replicas r / 2, r / 2 + 8
 #pragma unroll
@@ -490,6 +511,7 @@ __device__ __forceinline__ void small_colour_body(const LevelPtrs<Store> &L, int
     using Real = SmallReal<Store>;
     using V = Real2<Real>;
     using LA = Loose<Real>;
+    using Sum = SmallSums<Store>;
     constexpr int N1 = SH::N1, NI = SH::NI;
     __shared__ Real part[8 * 8];
     __shared__ V around[8][27];  // every incidence's node with its neighbours, widened
@@ -517,15 +539,15 @@ __device__ __forceinline__ void small_colour_body(const LevelPtrs<Store> &L, int
     }
     __syncwarp();
     const Real *mine = reinterpret_cast<const Real *>(around[slot]);
-    const Real t = incidence16<Real, 3>(ln, mine, 13, A, r, true, a, b);
+    const Real t = incidence16<Real, Sum, 3>(ln, mine, 13, A, r, true, a, b);
     next_may_start();
     if (!(r & 1)) part[slot * 8 + (r >> 3) * 4 + ((r & 7) >> 1)] = t;
     __syncthreads();
     Real x[8], p;
-    values_of_node<Real>(part, slot, cnt, r, x);
-    if (cnt && relaxed(L, node) && group_step<Real>(x, r, separate, p) && r < 2)
+    values_of_node<Real, Sum>(part, slot, cnt, r, x);
+    if (cnt && relaxed(L, node) && group_step<Real, Sum>(x, r, separate, p) && r < 2)
     {
-        const Real cur = LA::norm(LA::add(mine[26 + r], p));
+        const Real cur = LA::norm(Sum::add(mine[26 + r], p));
         if (!finite_value<Real>(cur)) atomicOr(err, (unsigned int)ERR_NONFINITE);
         L.xy[2 * node + r] = narrow<Store>(cur);
     }
