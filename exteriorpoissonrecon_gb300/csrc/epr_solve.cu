@@ -464,6 +464,9 @@ __device__ __forceinline__ void gs_update_lanes_at(const LevelPtrs<Real> &L, Rea
                 }
         }
     }
+    // the lanes without an element too: one of them may hold the node and write it
+    if constexpr (Chained)
+        if (!ok) await_previous();
     if constexpr (shears<Real>())
         if (!separate) sh = shear_of(group_sum<D>(sxy), group_sum<D>(sxx), group_sum<D>(syy));
     if (ok)
@@ -587,6 +590,7 @@ __device__ __forceinline__ void gs_update_pair3(const LevelPtrs<Real> &L, Real *
             }
         }
     }
+    if (!active) await_previous();  // every thread waits
     if constexpr (shears<Real>())
         if (!separate)
         {
