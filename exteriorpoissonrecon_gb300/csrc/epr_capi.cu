@@ -22,6 +22,7 @@
 #include "epr_common.cuh"
 #include "epr_context.h"
 #include "epr_kernels.h"
+#include "epr_prepare.h"
 #include "epr_mg.h"
 #include "epr_poly.h"
 
@@ -34,7 +35,6 @@ thread_local std::string g_error;
 // (CUDA_DEVICE_MAX_CONNECTIONS, 8 unless the process raises it before CUDA starts)
 constexpr int kBatchThreads = 8;
 
-std::mutex g_create_mutex;
 
 }  // namespace
 
@@ -733,14 +733,14 @@ epr_ctx *epr_create(int dim, int depth, const epr_params *params)
         g_error = std::string("cannot select CUDA device: ") + cudaGetErrorString(cudaGetLastError());
         return nullptr;
     }
+    // the incidence tables of the small levels and the kernels' attributes: without them a relaxation does nothing
+    static epr::PerDevice<char> prepared;
+    char done;
+    cudaError_t prepare = cudaSuccess;
+    if (!prepared.get(p.device, done, [&](char &) { return (prepare = epr::prepare_gs_kernels()) == cudaSuccess; }))
     {
-        std::lock_guard<std::mutex> lock(g_create_mutex);
-        static uint64_t prepared = 0;  // devices whose kernel attributes are set
-        if (p.device >= 0 && p.device < 64 && !(prepared & (1ull << p.device)))
-        {
-            epr::prepare_gs_kernels();
-            prepared |= 1ull << p.device;
-        }
+        g_error = std::string("cannot prepare the device's kernels: ") + cudaGetErrorString(prepare);
+        return nullptr;
     }
     epr_ctx *c = new epr_ctx;
     c->dim = dim;

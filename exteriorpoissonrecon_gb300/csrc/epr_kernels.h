@@ -82,7 +82,7 @@ constexpr bool small_colour_level(int level) { return level < 4 || (level == 4 &
 constexpr bool small4_colour_level(int level) { return level == 2 || level == 3; }
 bool launch_small4(const LevelPtrs<double> &L, int iters, unsigned int *err, cudaStream_t s, int separate);  // false: not a level it takes
 void launch_small4_colour(const LevelPtrs<double> &L, int colour, unsigned int *err, cudaStream_t s, int separate, bool after);
-void prepare_small_kernels();
+cudaError_t prepare_small_kernels();
 template <typename Real>
 void launch_small_level(const LevelPtrs<Real> &L, int iters, unsigned int *err, cudaStream_t s, int separate, int *kexp);
 template <typename Real>
@@ -90,7 +90,7 @@ void launch_small_colour(const LevelPtrs<Real> &L, int colour, unsigned int *err
                          bool after = false);
 // sets the kernels' shared-memory limits and uploads the small levels' tables (once per device, before any
 // stream capture)
-void prepare_gs_kernels();
+cudaError_t prepare_gs_kernels();
 template <int D, typename Real>
 void launch_gn_matvec(const LevelPtrs<Real> &L, const Real *xy, const Real *dxy, Real *out, cudaStream_t s);
 // fine (2 N_f) = P coarse (2 N_c), pairs; add != 0 accumulates

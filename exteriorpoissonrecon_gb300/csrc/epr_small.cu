@@ -890,18 +890,23 @@ void with_shape(int level, F &&f)
 }
 
 template <typename Store>
-void prepare_store()
+cudaError_t prepare_store()
 {
+    cudaError_t err = cudaSuccess;
+    auto set = [&](const void *k, cudaFuncAttribute a, int v) {
+        if (err == cudaSuccess) err = cudaFuncSetAttribute(k, a, v);
+    };
     for (int l = 0; l < kSmallLevels; l++)
         with_shape<Store>(l, [&](auto lv, auto nb) {
             constexpr int LEVEL = decltype(lv)::value, NB = decltype(nb)::value;
             const int bytes = (int)SmallShape<Store, LEVEL, NB>::kBytes;
             for (const void *k : {(const void *)small_kernel<Store, LEVEL, NB>, (const void *)small_batch_kernel<Store, LEVEL, NB>})
             {
-                cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-                if (NB > 8) cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+                set(k, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+                if (NB > 8) set(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
             }
         });
+    return err;
 }
 
 bool holds_16_blocks()
@@ -932,18 +937,20 @@ bool holds_16_blocks()
 
 }  // namespace
 
-void prepare_small_kernels()
+cudaError_t prepare_small_kernels()
 {
     static uint32_t host[small_base(kSmallLevels)];
     host_incidences(host);
-    cudaMemcpyToSymbol(g_incidences, host, sizeof(host));
     static uint32_t host4[small_base4(kSmallLevels4)];
     host_incidences4(host4);
-    cudaMemcpyToSymbol(g_incidences4, host4, sizeof(host4));
     g_level3_blocks = holds_16_blocks() ? 16 : 8;
-    prepare_store<float>();
-    prepare_store<double>();
-    prepare_store<df>();
+    cudaError_t e = cudaMemcpyToSymbol(g_incidences, host, sizeof(host));
+    if (e == cudaSuccess) e = cudaMemcpyToSymbol(g_incidences4, host4, sizeof(host4));
+    if (e == cudaSuccess) e = prepare_store<float>();
+    if (e == cudaSuccess) e = prepare_store<double>();
+    if (e == cudaSuccess) e = prepare_store<df>();
+    if (e != cudaSuccess) cudaGetLastError();  // reported by the caller
+    return e;
 }
 
 template <typename Store>

@@ -1057,10 +1057,10 @@ bool launch_gs_colour(const LevelPtrs<Real> &L, int colour, unsigned int *err, c
     return launch(std::false_type{});
 }
 
-void prepare_gs_kernels()
+cudaError_t prepare_gs_kernels()
 {
-    prepare_small_kernels();
-    cudaFuncSetAttribute(gs_level_kernel<4, float, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kLevelSmemLimit);
+    if (const cudaError_t e = prepare_small_kernels()) return e;
+    return cudaFuncSetAttribute(gs_level_kernel<4, float, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kLevelSmemLimit);
 }
 
 template <int D, typename Real>
