@@ -84,6 +84,7 @@ struct epr_batch
     int tile[kMaxLevels];
     cudaGraphExec_t graph = nullptr;
     int64_t graphLaunches = 0;
+    int blocks3 = 16;  // level 3's cluster: the smallest of the members'
     double relax_ms = 0;
     std::string err;
 
@@ -134,6 +135,8 @@ bool make_plan(epr_batch &b)
         top = std::max(top, maxD[i]);
     }
     if (top >= kMaxLevels) return b.fail("depth too large for a lockstep batch");
+    b.blocks3 = 16;
+    for (const Context *c : b.ctxs) b.blocks3 = std::min(b.blocks3, c->blocks3);
     b.levels.clear();
     b.xfers.clear();
     b.image.clear();
@@ -228,7 +231,7 @@ int64_t record(epr_batch &b)
             const BatchJob<Real> *jobs = reinterpret_cast<const BatchJob<Real> *>(b.dtab + P.off);
             if (P.tiny)
             {
-                launch_small_level_batch<Real>(jobs, l, P.count, s);
+                launch_small_level_batch<Real>(jobs, l, P.count, b.blocks3, s);
                 launches++;
                 return;
             }

@@ -734,10 +734,10 @@ epr_ctx *epr_create(int dim, int depth, const epr_params *params)
         return nullptr;
     }
     // the incidence tables of the small levels and the kernels' attributes: without them a relaxation does nothing
-    static epr::PerDevice<char> prepared;
-    char done;
+    static epr::PerDevice<int> prepared;
+    int blocks3;
     cudaError_t prepare = cudaSuccess;
-    if (!prepared.get(p.device, done, [&](char &) { return (prepare = epr::prepare_gs_kernels()) == cudaSuccess; }))
+    if (!prepared.get(p.device, blocks3, [&](int &most) { return (prepare = epr::prepare_gs_kernels(&most)) == cudaSuccess; }))
     {
         g_error = std::string("cannot prepare the device's kernels: ") + cudaGetErrorString(prepare);
         return nullptr;
@@ -747,6 +747,9 @@ epr_ctx *epr_create(int dim, int depth, const epr_params *params)
     c->depth = depth;
     c->P = p;
     if (const char *v = getenv("EPR_ALLOC_CAP_BYTES")) c->alloc_cap = (size_t)strtoull(v, nullptr, 10);
+    c->blocks3 = blocks3;
+    if (const char *v = getenv("EPR_CLUSTER_LEVELS"))
+        if (atoi(v) == 8) c->blocks3 = 8;
     if (const char *v = getenv("EPR_ADAPTIVE_LISTS")) c->adaptive_lists = atoi(v) != 0;
     c->levels.resize(depth + 1);
     if (cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking) != cudaSuccess ||

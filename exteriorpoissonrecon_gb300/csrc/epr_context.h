@@ -100,6 +100,9 @@ struct Context
     // adaptive levels relax per-colour lists of their active nodes (EPR_ADAPTIVE_LISTS=0 at context
     // creation: every node of the colour, the inactive ones skipped; the same bits)
     bool adaptive_lists = true;
+    // blocks of level 3's cluster: the most that the device holds, 16 or 8 (EPR_CLUSTER_LEVELS=8 at context
+    // creation: 8; the same bits)
+    int blocks3 = 8;
     const uint8_t *status_of(int l) const { return adapt.empty() ? nullptr : adapt[l].status; }
     void release_adaptive();
     MGHierarchy *mg = nullptr;  // linear multigrid storage (epr_mg.cu), allocated on first use
@@ -150,6 +153,7 @@ inline LevelPtrs<Real> level_ptrs(Context *c, int l)
     LevelPtrs<Real> p;
     p.level = l;
     p.N = L.N;
+    p.blocks3 = c->blocks3;
     if (!c->adapt.empty())
     {
         const AdaptiveLevel &A = c->adapt[l];

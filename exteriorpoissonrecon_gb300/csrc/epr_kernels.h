@@ -33,6 +33,7 @@ struct LevelPtrs
     // lists instead of the whole colour.  Null for the regular grid.
     const int *alist = nullptr;
     int aoff[17] = {0};
+    int blocks3 = 8;  // blocks of level 3's cluster, 8 or 16 (the same bits)
 };
 
 // Scratch for deterministic two-pass reductions
@@ -82,7 +83,8 @@ constexpr bool small_colour_level(int level) { return level < 4 || (level == 4 &
 constexpr bool small4_colour_level(int level) { return level == 2 || level == 3; }
 bool launch_small4(const LevelPtrs<double> &L, int iters, unsigned int *err, cudaStream_t s, int separate);  // false: not a level it takes
 void launch_small4_colour(const LevelPtrs<double> &L, int colour, unsigned int *err, cudaStream_t s, int separate, bool after);
-cudaError_t prepare_small_kernels();
+// blocks3: the largest cluster of level 3 that the device holds, 16 or 8 blocks
+cudaError_t prepare_small_kernels(int *blocks3);
 template <typename Real>
 void launch_small_level(const LevelPtrs<Real> &L, int iters, unsigned int *err, cudaStream_t s, int separate, int *kexp);
 template <typename Real>
@@ -90,7 +92,7 @@ void launch_small_colour(const LevelPtrs<Real> &L, int colour, unsigned int *err
                          bool after = false);
 // sets the kernels' shared-memory limits and uploads the small levels' tables (once per device, before any
 // stream capture)
-cudaError_t prepare_gs_kernels();
+cudaError_t prepare_gs_kernels(int *blocks3);
 template <int D, typename Real>
 void launch_gn_matvec(const LevelPtrs<Real> &L, const Real *xy, const Real *dxy, Real *out, cudaStream_t s);
 // fine (2 N_f) = P coarse (2 N_c), pairs; add != 0 accumulates
@@ -155,7 +157,7 @@ constexpr int kLanesTiles[3] = {64, 128, 256};
 constexpr int kDefaultTile = 1;  // index into the table: the solo solve's shape (128 threads)
 // all sweeps of a small level of `count` reconstructions (jobs[0..count))
 template <typename Real>
-void launch_small_level_batch(const BatchJob<Real> *jobs, int level, int count, cudaStream_t s);
+void launch_small_level_batch(const BatchJob<Real> *jobs, int level, int count, int blocks3, cudaStream_t s);
 // one colour of a level of jobs[0..count)
 template <typename Real>
 void launch_small_colour_batch(const BatchJob<Real> *jobs, int level, int colour, int count, cudaStream_t s, bool after);

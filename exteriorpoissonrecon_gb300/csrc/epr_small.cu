@@ -869,35 +869,33 @@ void with_level(int level, F &&f)
     else f(std::integral_constant<int, 4>{});
 }
 
-// Level 3's cluster: 16 blocks where the device can hold such a cluster (512 incidences of about 600
-// instructions: issue-bound, 2.4 us a colour phase against 3.8 on 8 blocks), else 8.  The node sums run in one order
-// whatever the cluster size, so the results are the same bits.
-int g_level3_blocks = 8;
-
-// f(level, blocks) as constants for a small level
+// f(level, blocks) as constants for a small level.  Level 3 runs on a cluster of `blocks3` blocks, 16 or 8: 16 where
+// the device can hold such a cluster (512 incidences of about 600 instructions: issue-bound, 2.7 us a colour phase
+// against 4.1 on 8 blocks).  The node sums run in one order whatever the cluster size, so the results are the same
+// bits.
 template <typename Store, typename F>
-void with_shape(int level, F &&f)
+void with_shape(int level, int blocks3, F &&f)
 {
     with_level(level, [&](auto lv) {
         constexpr int LEVEL = decltype(lv)::value;
         if constexpr (small_level<Store>(LEVEL))
         {
             if constexpr (LEVEL == 3)
-                if (g_level3_blocks == 16) return f(lv, std::integral_constant<int, 16>{});
+                if (blocks3 == 16) return f(lv, std::integral_constant<int, 16>{});
             f(lv, std::integral_constant<int, (LEVEL < 2 ? 1 : 8)>{});
         }
     });
 }
 
 template <typename Store>
-cudaError_t prepare_store()
+cudaError_t prepare_store(int blocks3)
 {
     cudaError_t err = cudaSuccess;
     auto set = [&](const void *k, cudaFuncAttribute a, int v) {
         if (err == cudaSuccess) err = cudaFuncSetAttribute(k, a, v);
     };
-    for (int l = 0; l < kSmallLevels; l++)
-        with_shape<Store>(l, [&](auto lv, auto nb) {
+    auto shape = [&](int l, int blocks) {
+        with_shape<Store>(l, blocks, [&](auto lv, auto nb) {
             constexpr int LEVEL = decltype(lv)::value, NB = decltype(nb)::value;
             const int bytes = (int)SmallShape<Store, LEVEL, NB>::kBytes;
             for (const void *k : {(const void *)small_kernel<Store, LEVEL, NB>, (const void *)small_batch_kernel<Store, LEVEL, NB>})
@@ -906,6 +904,9 @@ cudaError_t prepare_store()
                 if (NB > 8) set(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
             }
         });
+    };
+    for (int l = 0; l < kSmallLevels; l++) shape(l, 8);
+    if (blocks3 == 16) shape(3, 16);
     return err;
 }
 
@@ -937,18 +938,18 @@ bool holds_16_blocks()
 
 }  // namespace
 
-cudaError_t prepare_small_kernels()
+cudaError_t prepare_small_kernels(int *blocks3)
 {
     static uint32_t host[small_base(kSmallLevels)];
     host_incidences(host);
     static uint32_t host4[small_base4(kSmallLevels4)];
     host_incidences4(host4);
-    g_level3_blocks = holds_16_blocks() ? 16 : 8;
+    *blocks3 = holds_16_blocks() ? 16 : 8;
     cudaError_t e = cudaMemcpyToSymbol(g_incidences, host, sizeof(host));
     if (e == cudaSuccess) e = cudaMemcpyToSymbol(g_incidences4, host4, sizeof(host4));
-    if (e == cudaSuccess) e = prepare_store<float>();
-    if (e == cudaSuccess) e = prepare_store<double>();
-    if (e == cudaSuccess) e = prepare_store<df>();
+    if (e == cudaSuccess) e = prepare_store<float>(*blocks3);
+    if (e == cudaSuccess) e = prepare_store<double>(*blocks3);
+    if (e == cudaSuccess) e = prepare_store<df>(*blocks3);
     if (e != cudaSuccess) cudaGetLastError();  // reported by the caller
     return e;
 }
@@ -956,7 +957,7 @@ cudaError_t prepare_small_kernels()
 template <typename Store>
 void launch_small_level(const LevelPtrs<Store> &L, int iters, unsigned int *err, cudaStream_t s, int separate, int *kexp)
 {
-    with_shape<Store>(L.level, [&](auto lv, auto nb) {
+    with_shape<Store>(L.level, L.blocks3, [&](auto lv, auto nb) {
         constexpr int LEVEL = decltype(lv)::value, NB = decltype(nb)::value;
         using SH = SmallShape<Store, LEVEL, NB>;
         launch_colour(small_kernel<Store, LEVEL, NB>, dim3(NB), NB, SH::kThreads, SH::kBytes, s, false, L, iters, err, separate, kexp);
@@ -964,10 +965,10 @@ void launch_small_level(const LevelPtrs<Store> &L, int iters, unsigned int *err,
 }
 
 template <typename Store>
-void launch_small_level_batch(const BatchJob<Store> *jobs, int level, int count, cudaStream_t s)
+void launch_small_level_batch(const BatchJob<Store> *jobs, int level, int count, int blocks3, cudaStream_t s)
 {
     if (count <= 0) return;
-    with_shape<Store>(level, [&](auto lv, auto nb) {
+    with_shape<Store>(level, blocks3, [&](auto lv, auto nb) {
         constexpr int LEVEL = decltype(lv)::value, NB = decltype(nb)::value;
         using SH = SmallShape<Store, LEVEL, NB>;
         launch_colour(small_batch_kernel<Store, LEVEL, NB>, dim3(NB * count), NB, SH::kThreads, SH::kBytes, s, false, jobs);
@@ -1011,7 +1012,7 @@ void launch_small4_colour(const LevelPtrs<double> &L, int colour, unsigned int *
 
 #define EPR_SMALL(T)                                                                                              \
     template void launch_small_level<T>(const LevelPtrs<T> &, int, unsigned int *, cudaStream_t, int, int *);      \
-    template void launch_small_level_batch<T>(const BatchJob<T> *, int, int, cudaStream_t);                       \
+    template void launch_small_level_batch<T>(const BatchJob<T> *, int, int, int, cudaStream_t);                      \
     template void launch_small_colour<T>(const LevelPtrs<T> &, int, unsigned int *, cudaStream_t, int, const int *, bool); \
     template void launch_small_colour_batch<T>(const BatchJob<T> *, int, int, int, cudaStream_t, bool);
 EPR_SMALL(float)

@@ -1057,9 +1057,9 @@ bool launch_gs_colour(const LevelPtrs<Real> &L, int colour, unsigned int *err, c
     return launch(std::false_type{});
 }
 
-cudaError_t prepare_gs_kernels()
+cudaError_t prepare_gs_kernels(int *blocks3)
 {
-    if (const cudaError_t e = prepare_small_kernels()) return e;
+    if (const cudaError_t e = prepare_small_kernels(blocks3)) return e;
     return cudaFuncSetAttribute(gs_level_kernel<4, float, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kLevelSmemLimit);
 }
 
