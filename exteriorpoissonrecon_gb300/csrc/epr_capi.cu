@@ -74,12 +74,16 @@ bool Context::alloc(void **p, size_t bytes, const char *what)
         return false;
     }
     alloc_total += bytes;
-    return cuda_ok(cudaMallocAsync(p, bytes, stream), what);
+    if (!cuda_ok(cudaMallocAsync(p, bytes, stream), what)) return false;
+    live.insert(*p);
+    return true;
 }
 
 void Context::release(void *p)
 {
-    if (p) cudaFreeAsync(p, stream);
+    if (!p) return;
+    live.erase(p);
+    cudaFreeAsync(p, stream);
 }
 
 int64_t Context::nodes(int level) const
@@ -229,6 +233,7 @@ Context::~Context()
         setup.release(*this);
         release_adaptive();
         release_mg(*this);
+        while (!live.empty()) release(*live.begin());  // what a call that failed half-way still held
         if (solve_graph) cudaGraphExecDestroy(solve_graph);
         cudaStreamSynchronize(stream);
         cudaStreamDestroy(stream);

@@ -2,6 +2,7 @@
 #pragma once
 #include <cstdint>
 #include <string>
+#include <unordered_set>
 #include <vector>
 
 #include <cuda_runtime.h>
@@ -93,6 +94,7 @@ struct Context
     // EPR_ALLOC_CAP_BYTES environment variable at epr_create; allocations beyond it fail as an
     // out-of-memory would (EPR_ERR_NOMEM)
     size_t alloc_cap = 0, alloc_total = 0;
+    std::unordered_set<void *> live;  // the context's device allocations
     Setup setup;
     // the adaptive indexer's levels (empty for the regular grid), built with the system
     std::vector<AdaptiveLevel> adapt;
