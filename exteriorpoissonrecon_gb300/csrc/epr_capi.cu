@@ -117,9 +117,8 @@ bool Context::ensure_level(int l)
     if (dim == 3 && pair_level<3>(l))
     {
         // the pair layout from the start: the relaxation of these levels reads nothing else
-        const size_t bytes = 56 * L.N * (lvl32(l) ? sizeof(float) : sizeof(double));
-        if (!alloc(&L.Acb, bytes, "alloc colour blocks")) return false;
-        if (!cuda_ok(cudaMemsetAsync(L.Acb, 0, bytes, stream), "memset colour blocks")) return false;
+        if (!ensure_blocks(l)) return false;
+        if (!cuda_ok(cudaMemsetAsync(L.Acb, 0, block_bytes(l), stream), "memset colour blocks")) return false;
     }
     if (lvlDF(l))
     {
@@ -142,6 +141,27 @@ bool Context::lvlDF(int l) const
            l <= kMaxDFLevel && l >= P.fp64_from && l < P.fp64_levels;
 }
 
+// bytes of a level's colour blocks (both stencils; on pair levels the pair layout): none on the small levels,
+// which read the natural order
+size_t Context::block_bytes(int l) const
+{
+    const bool f = lvl32(l);
+    const int64_t N = nodes(l);
+    if (dim == 3 ? (f ? small_colour_level<float>(l) : small_colour_level<double>(l)) : f ? N <= 81 : l <= 3) return 0;
+    return (dim == 3 && pair_level<3>(l) ? PairLayout<float>::kNode : 2 * stencil()) * N * (f ? sizeof(float) : sizeof(double));
+}
+
+bool Context::ensure_blocks(int l)
+{
+    Level &L = levels[l];
+    const size_t bytes = block_bytes(l);
+    if (!bytes || L.Acb) return true;
+    // one array for both stencils: either none is there or both are
+    if (!alloc(&L.Acb, bytes, "alloc colour blocks")) return false;
+    if (!(dim == 3 && pair_level<3>(l))) L.Bcb = (char *)L.Acb + bytes / 2;
+    return true;
+}
+
 // refreshes the derived copies of a level's system: the float stencils (float levels) and the
 // colour-blocked stencils of the levels that are relaxed by one kernel per colour
 bool Context::sync_system32(int l)
@@ -160,15 +180,10 @@ bool Context::sync_system32(int l)
         launch_d2df(L.B64, L.Bd, (int64_t)S * L.N, stream);
         return L.synced = launch_ok("convert system");
     }
-    // the small levels read the natural order
-    if (dim == 3 ? !(lvl32(l) ? small_colour_level<float>(l) : small_colour_level<double>(l)) : lvl32(l) ? L.N > 81 : l > 3)
+    if (block_bytes(l))
     {
         if (dim == 3 && pair_level<3>(l)) return pair_system(*this, l, 0.);
-        const size_t real = lvl32(l) ? sizeof(float) : sizeof(double);
-        const size_t bytes = S * L.N * real;
-        // one array for both: either none is there or both are
-        if (!L.Acb && !alloc(&L.Acb, 2 * bytes, "alloc colour blocks")) return false;
-        L.Bcb = (char *)L.Acb + bytes;
+        if (!ensure_blocks(l)) return false;
         auto blocks = [&](auto dd) {
             constexpr int D = decltype(dd)::value;
             if (lvl32(l))
@@ -188,11 +203,12 @@ bool Context::sync_system32(int l)
     return L.synced = launch_ok("convert system");
 }
 
-// The copies of a level that no build and no epr_set_level_system has reached: those of its double stencils,
-// which are zero from the start
+// The copies of a level that no build and no epr_set_level_system has reached, or whose colour blocks a build left
+// as scratch: those of its double stencils, which are zero from the start
 bool Context::level_ready(int l)
 {
-    return !(lvl32(l) || lvlDF(l)) || levels[l].synced || sync_system32(l);
+    const bool copies = lvl32(l) || lvlDF(l) || levels[l].Acb;
+    return !copies || levels[l].synced || sync_system32(l);
 }
 
 // device coefficients <-> the precision the solve works in
@@ -537,6 +553,7 @@ bool Context::solve_prologue()
     const bool fp32 = P.precision == EPR_FP32;
     for (int l = 0; l <= depth; l++)
     {
+        if (!level_ready(l)) return false;
         if (P.warm_start && l == minD) continue;  // the given start
         if (!cuda_ok(cudaMemsetAsync(levels[l].xy64, 0, sizeof(double) * 2 * levels[l].N, stream), "clear")) return false;
         if (fp32 && !cuda_ok(cudaMemsetAsync(levels[l].xy32, 0, sizeof(float) * 2 * levels[l].N, stream), "clear")) return false;

@@ -126,6 +126,8 @@ struct Context
     bool lvl32(int l) const;  // level l computes in float
     bool lvlDF(int l) const;  // level l computes in double-float (a 3D coarse band level)
     bool sync_system32(int l);
+    size_t block_bytes(int l) const;
+    bool ensure_blocks(int l);
     bool level_ready(int l);
     bool push_xy(int l);
     bool pull_xy(int l);

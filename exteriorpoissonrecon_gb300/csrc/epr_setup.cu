@@ -1588,19 +1588,20 @@ bool build_impl(Context &c, Setup &st)
     if (!dalloc(c, &st.S, gfine.NE * K, "S") || !dalloc(c, &st.leaf, gfine.NE, "leaf")) return false;
     {
         SkewGrids<D> G;
-        std::vector<double *> sums(depth + 1, nullptr);
         G.g[0] = st.skewGrid[0];
+        // the sums in the finest B, which is written in full below; what was built before ends here
+        c.have_system = false;
+        double *sums = c.levels[depth].B64;
         for (int l = 1; l <= depth; l++)
         {
             Grid<D> gl(l);
-            if (!dalloc(c, &sums[l], gl.N * K, "frame sums")) return false;
-            accumulate_frames_kernel<D><<<nblocks(gl.N, 256), 256, 0, s>>>(l, st.skewGrid[l], G.g[l - 1], sums[l]);
-            G.g[l] = sums[l];
+            accumulate_frames_kernel<D><<<nblocks(gl.N, 256), 256, 0, s>>>(l, st.skewGrid[l], G.g[l - 1], sums);
+            G.g[l] = sums;
+            sums += gl.N * K;
         }
         for (int t = 0; t <= depth + 1 && t < 12; t++) G.refined[t] = st.refinedS[t];
         G.depth = depth;
         element_frame_kernel<D><<<nblocks(gfine.NE, 128), 128, 0, s>>>(G, st.S, st.leaf, c.P.project);
-        for (double *p : sums) c.release(p);
     }
     // the adaptive indexer: its tables, and the frame field restricted to its elements for c and B
     const double *Sfit = st.S;
@@ -1628,11 +1629,16 @@ bool build_impl(Context &c, Setup &st)
     {
         if (!device_sum(c, st.measure, n, 1, dsum + 1)) return false;
         scale_by_kernel<<<1, 32, 0, s>>>(dsum + 2, dsum + 1, c.P.s_weight, n);
-        double *mass = nullptr;
-        if (!dalloc(c, &mass, (size_t)nc * CellPairs<D>::N, "cell masses")) return false;
+        // in the finest B too, where it holds them (fewer occupied cells than 0.75 (0.59 in 4D) times the nodes)
+        double *own = nullptr, *mass = Lf.B64;
+        if (nc * CellPairs<D>::N > S * Lf.N)
+        {
+            if (!dalloc(c, &own, (size_t)nc * CellPairs<D>::N, "cell masses")) return false;
+            mass = own;
+        }
         cell_mass_kernel<D><<<nblocks(nc, 4), 128, 0, s>>>(st.pos, st.noise, st.order, st.cellStart, st.cellKey, nc, depth, c.P.n_sigma, mass);
         screening_kernel<D><<<nblocks(Lf.N, 128), 128, 0, s>>>(mass, st.cellOfFinest, depth, dsum + 2, Lf.A64);
-        c.release(mass);
+        c.release(own);
     }
     constraint_kernel<D><<<nblocks(Lf.N, 128), 128, 0, s>>>(Sfit, depth, Lf.B64);
     c.release(Smasked);
@@ -1640,13 +1646,17 @@ bool build_impl(Context &c, Setup &st)
 
     // ---- Galerkin hierarchy of R and B, then A = R + dWeight K on every level ----
     {
-        // the finest pair layout is written below and large enough (56 values a node against 27 x 3/4 doubles)
-        double *own = nullptr, *scratch = (double *)(D == 3 && pair_level<3>(depth) ? Lf.Acb : nullptr);
-        if (!scratch)
+        // scratch: the finest level's colour blocks, which are written below, where it has any
+        for (int l = 0; l <= depth; l++)
+            if (!c.ensure_blocks(l)) return false;
+        const size_t need = galerkin_scratch<D>(depth);
+        double *own = nullptr, *scratch = (double *)Lf.Acb;
+        if (c.block_bytes(depth) < need * sizeof(double))
         {
-            if (!dalloc(c, &own, galerkin_scratch<D>(depth), "galerkin scratch")) return false;
+            if (!dalloc(c, &own, need, "galerkin scratch")) return false;
             scratch = own;
         }
+        else Lf.synced = false;
         for (int l = depth; l > 0; l--)
         {
             launch_galerkin<D>(l, c.levels[l].A64, c.levels[l - 1].A64, scratch, s);
