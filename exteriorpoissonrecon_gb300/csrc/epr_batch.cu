@@ -507,7 +507,9 @@ int epr_batch_tune(epr_batch *b, int reps, double *ms_out)
         ok = ok && b->ok(cudaStreamSynchronize(b->stream), "tune save");
         double best = 1e300;
         int bestTile = kDefaultTile;
-        for (int t = 0; ok && t < 3; t++)
+        // levels 3 and 4 in double have one shape: timed once, and left at the default
+        const bool one_shape = P.type == kTypeDouble && small_colour_level<double>(l);
+        for (int t = 0; ok && t < (one_shape ? 1 : 3); t++)
         {
             auto sweep = [&](auto tag) {
                 using Real = decltype(tag);
@@ -526,8 +528,9 @@ int epr_batch_tune(epr_batch *b, int reps, double *ms_out)
             ok = b->ok(cudaStreamSynchronize(b->stream), "tune");
             float ms = 0;
             cudaEventElapsedTime(&ms, b->e0, b->e1);
-            if (ms_out) ms_out[3 * nl + t] = ms / reps;
-            if (ms < best) { best = ms; bestTile = t; }
+            if (ms_out)
+                for (int k = t; k < (one_shape ? 3 : t + 1); k++) ms_out[3 * nl + k] = ms / reps;
+            if (!one_shape && ms < best) { best = ms; bestTile = t; }
         }
         for (int k = 0; k < P.count; k++)
         {

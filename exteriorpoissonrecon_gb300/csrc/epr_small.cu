@@ -871,7 +871,7 @@ void with_level(int level, F &&f)
 
 // f(level, blocks) as constants for a small level.  Level 3 runs on a cluster of `blocks3` blocks, 16 or 8: 16 where
 // the device can hold such a cluster (512 incidences of about 600 instructions: issue-bound, 2.7 us a colour phase
-// against 4.1 on 8 blocks).  The node sums run in one order whatever the cluster size, so the results are the same
+// against 4.3 on 8 blocks).  The node sums run in one order whatever the cluster size, so the results are the same
 // bits.
 template <typename Store, typename F>
 void with_shape(int level, int blocks3, F &&f)

@@ -211,9 +211,9 @@ int epr_solve(epr_ctx *ctx, epr_stats *stats);
 int epr_batch_solve(epr_ctx *const *ctxs, int n, int build, int threads, epr_stats *stats, int *status);
 
 /* Lockstep batch of 3D reconstructions: the cascadic schedule of every member advances level by
- * level, and each level's relaxation is a few launches for all members together (levels 0-1: one
- * block per member for all its sweeps; from level 2 on one launch per sweep and colour whose grid
- * spans the colour's nodes of every member still sweeping that level).  The whole relaxation is
+ * level, and each level's relaxation is a few launches for all members together (levels 0-3, in
+ * double 0-2: a block or a cluster of blocks per member for all its sweeps; above them one launch per
+ * sweep and colour whose grid spans the colour's nodes of every member still sweeping that level).  The whole relaxation is
  * one CUDA graph, captured on the first epr_batch_run and replayed while the members' arrays stay
  * where they are.  Members may differ in depth, samples, sweep counts and parameters, but must run
  * the plain cascadic schedule (no multigrid, single level, verbose, warm start or target energy),
@@ -228,11 +228,11 @@ epr_batch *epr_batch_create(epr_ctx *const *ctxs, int n, int threads);
  * shared by all members.  stats / status as for epr_batch_solve. */
 int epr_batch_run(epr_batch *b, int build, epr_stats *stats, int *status);
 /* The autotuner: for every level relaxed by per-colour launches, times `reps` sweeps of all members
- * in each of the three block shapes of its colour kernel (levels whose colours have at most 125
- * nodes: 1, 2 or 4 nodes per block of the point-split kernel; larger levels: 64, 128 or 256 threads
- * per block of the lane kernel) on the members' current coefficients, which it restores, and keeps
- * the fastest shape per level for the next runs.  No shape changes any node's arithmetic.  ms_out
- * (may be NULL) receives 3 mean sweep times per tuned level, coarsest first.  Needs built members. */
+ * in each of the three block shapes of its colour kernel (64, 128 or 256 threads per block) on the
+ * members' current coefficients, which it restores, and keeps the fastest shape per level for the
+ * next runs; levels 3 and 4 in double have one shape, whose time it gives three times.  No shape
+ * changes any node's arithmetic.  ms_out (may be NULL) receives 3 mean sweep times per tuned level,
+ * coarsest first.  Needs built members. */
 int epr_batch_tune(epr_batch *b, int reps, double *ms_out);
 /* Sets level's block shape index (0-2; level -1: every level) by hand, in place of the tuner's. */
 int epr_batch_set_tile(epr_batch *b, int level, int tile);

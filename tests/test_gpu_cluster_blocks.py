@@ -1,6 +1,6 @@
 """Level 3's cluster on 16 blocks against 8 (EPR_CLUSTER_LEVELS=8 at context creation): the same bits, alone and in
 a lockstep batch, in float and double-float, on the regular grid and with the adaptive indexer.  The choice is a
-context's own; that it is one shows in the time of a phase (2.7 against 4.1 us)."""
+context's own; that it is one shows in the time of a phase (2.7 against 4.3 us)."""
 import time
 
 import numpy as np
