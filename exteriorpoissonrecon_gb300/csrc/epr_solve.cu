@@ -387,18 +387,20 @@ __device__ __forceinline__ void gs_update_lanes_at(const LevelPtrs<Real> &L, Rea
     int64_t i = 0;
     Real q[5] = {(Real)0, (Real)0, (Real)0, (Real)0, (Real)0};
     V f[C], av = {(Real)0, (Real)0}, bv = {(Real)0, (Real)0};
+    Real ca[C], cb[C];
     Real acen = (Real)0, sxy = (Real)0, sxx = (Real)0, syy = (Real)0;
     Shear<Real> sh = {(Real)0, (Real)0};
+    // node indices in 32 bits (every supported grid has < 2^32 nodes); signed strides of the
+    // element mirrored so that the node is its corner 0
+    int sd[D], other = 0;
+    uint32_t iu = 0;
     bool ok = active;
     if (active)
     {
-        // node indices in 32 bits (every supported grid has < 2^32 nodes); signed strides of the
-        // element mirrored so that the node is its corner 0
-        int st[D], sd[D];
+        int st[D];
         st[D - 1] = 1;
 #pragma unroll
         for (int d = D - 2; d >= 0; d--) st[d] = st[d + 1] * (g.r + 1);
-        uint32_t iu = 0;
         int first = 0;  // the lower-numbered existing side of every axis, as corner bits
 #pragma unroll
         for (int d = 0; d < D; d++)
@@ -410,6 +412,7 @@ __device__ __forceinline__ void gs_update_lanes_at(const LevelPtrs<Real> &L, Rea
             if (I[d] >= g.r) first |= 1 << (D - 1 - d);
         }
         i = iu;
+        other = A ^ first;
         if (ok)
         {
             const int64_t step = Ac ? nc : L.N;
@@ -418,8 +421,6 @@ __device__ __forceinline__ void gs_update_lanes_at(const LevelPtrs<Real> &L, Rea
             int64_t so[D];
 #pragma unroll
             for (int d = 0; d < D; d++) so[d] = cbit<D>(A, d) ? -(int64_t)ipow(3, D - 1 - d) * step : (int64_t)ipow(3, D - 1 - d) * step;
-            const int other = A ^ first;
-            Real ca[C], cb[C];
 #pragma unroll
             for (int cc = 0; cc < C; cc++)
             {
@@ -434,39 +435,40 @@ __device__ __forceinline__ void gs_update_lanes_at(const LevelPtrs<Real> &L, Rea
                     if (cc) cb[cc] = pB[o];
                 }
             }
-            if constexpr (Chained) await_previous();
-#pragma unroll
-            for (int cc = 0; cc < C; cc++)
-            {
-                int jj = (int)iu;
-#pragma unroll
-                for (int d = 0; d < D; d++)
-                    if (cbit<D>(cc, d)) jj += sd[d];
-                f[cc] = ld2(xy, (int64_t)(uint32_t)jj);
-            }
-            acen = ca[0];
-#pragma unroll
-            for (int cc = 0; cc < C; cc++)
-                if ((other & ~cc & (C - 1)) == 0)
-                {
-                    av = O::fma(ca[cc], f[cc], av);
-                    if (cc) bv = O::fma(cb[cc], f[cc], bv);
-                }
-#pragma unroll
-            for (int cc = 1; cc < C; cc++) f[cc] = O::sub(f[cc], f[0]);
-            if constexpr (shears<Real>())
-#pragma unroll
-                for (int d = 0; d < D; d++)
-                {
-                    sxy = O::fma(f[1 << d].x, f[1 << d].y, sxy);
-                    sxx = O::fma(f[1 << d].x, f[1 << d].x, sxx);
-                    syy = O::fma(f[1 << d].y, f[1 << d].y, syy);
-                }
         }
     }
-    // the lanes without an element too: one of them may hold the node and write it
-    if constexpr (Chained)
-        if (!ok) await_previous();
+    // every lane, also one without an element: it may hold the node and write it
+    if constexpr (Chained) await_previous();
+    if (ok)
+    {
+#pragma unroll
+        for (int cc = 0; cc < C; cc++)
+        {
+            int jj = (int)iu;
+#pragma unroll
+            for (int d = 0; d < D; d++)
+                if (cbit<D>(cc, d)) jj += sd[d];
+            f[cc] = ld2(xy, (int64_t)(uint32_t)jj);
+        }
+        acen = ca[0];
+#pragma unroll
+        for (int cc = 0; cc < C; cc++)
+            if ((other & ~cc & (C - 1)) == 0)
+            {
+                av = O::fma(ca[cc], f[cc], av);
+                if (cc) bv = O::fma(cb[cc], f[cc], bv);
+            }
+#pragma unroll
+        for (int cc = 1; cc < C; cc++) f[cc] = O::sub(f[cc], f[0]);
+        if constexpr (shears<Real>())
+#pragma unroll
+            for (int d = 0; d < D; d++)
+            {
+                sxy = O::fma(f[1 << d].x, f[1 << d].y, sxy);
+                sxx = O::fma(f[1 << d].x, f[1 << d].x, sxx);
+                syy = O::fma(f[1 << d].y, f[1 << d].y, syy);
+            }
+    }
     if constexpr (shears<Real>())
         if (!separate) sh = shear_of(group_sum<D>(sxy), group_sum<D>(sxx), group_sum<D>(syy));
     if (ok)
