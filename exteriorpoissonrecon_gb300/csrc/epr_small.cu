@@ -17,19 +17,20 @@
 //    for a warp's FP64 instruction however many of its lanes are active.
 //  * Double-float runs on loosely normalised pairs: sums keep the error term of the leading parts but are
 //    renormalised only before a product or where they are stored, so that a chain of sums costs one
-//    addition's latency each instead of thirteen operations'.  The sums that cancel are done in full: a node's
-//    over its lanes and incidences, the two differences of its step, the update (FullSums).
+//    addition's latency each instead of thirteen operations'.  The sums that cancel most are done in full: an
+//    incidence's over its lanes, the two differences of the step, the update (FullSums).
 // Float levels compute in double-float, loose throughout, and store float: the arithmetic is not what their phases
 // wait for, and its error not what their result shows.
 //
 // Error of one and of eight sweeps in double-float against 80-bit arithmetic, as a ratio to the 12-point Gauss rule
 // on fully normalised pairs (geometric means over 140 systems of each level 0-3: random ones and those of built
-// curves at several stages of their relaxation; standard error 0.03): 1.00, 0.97, 0.91, 0.96 at 0.80, 0.69, 1.25,
-// 2.71 us a phase of a built curve's system.  All sums loose: 1.28, 1.22, 1.07, 1.18 at 0.72, 0.59, 1.17, 2.45 us;
-// every sum and product in full: 0.95, 0.89, 0.88, 0.95 at 1.03, 0.83, 1.61, 3.58 us.
+// curves at several stages of their relaxation; standard error 0.03): 1.00, 0.96, 0.93, 1.00 at 0.80, 0.63, 1.20,
+// 2.61 us a phase of a built curve's system.  All sums loose, a node's incidences one after another: 1.28, 1.22, 1.07, 1.18
+// at 0.72, 0.59, 1.17, 2.45 us; the node sums in full as well: 1.00, 0.97, 0.91, 0.96 at 0.80, 0.69, 1.25, 2.71 us; every
+// sum and product in full: 0.95, 0.89, 0.88, 0.95 at 1.03, 0.83, 1.61, 3.58 us.
 //
-// Levels 0, 1, 2, 3 of a depth-8 schedule (20,480, 10,240, 5,120 and 2,560 phases): 16.5, 9.7, 6.4 and 6.9 ms
-// in double-float and 48.8, 28.3, 15.6 and 10.6 ms in double.  With the incidence on 12 Gauss points of
+// Levels 0, 1, 2, 3 of a depth-8 schedule (20,480, 10,240, 5,120 and 2,560 phases): 16.5, 9.2, 6.1 and 6.7 ms
+// in double-float and 48.8, 28.3, 15.6 and 10.7 ms in double.  With the incidence on 12 Gauss points of
 // one warp, fully normalised pairs and a launch per colour from level 2 on they took 42, 34, 33.5 and
 // 17.7 ms, and 92, 73, 58 and 29 ms.  Four lanes per incidence (a component each) were slower wherever
 // tried (double 72, 71, 38 and 24 ms; double-float level 3 on eight SMs 7.5 ms).
@@ -346,9 +347,10 @@ __device__ __forceinline__ void values_of_incidence(Real t, Real *x)
 }
 // ... from the sums of the node's cnt incidences in shared memory: lane r adds every second incidence of
 // value r % 8 in pairs, the halves meet by a shuffle
-template <typename Real, typename Sum>
+template <typename Real>
 __device__ __forceinline__ void values_of_node(const Real *part, int slot, int cnt, int r, Real *x)
 {
+    using L = Loose<Real>;
     Real v[4];
 #pragma unroll
     for (int n = 0; n < 4; n++)
@@ -356,8 +358,8 @@ __device__ __forceinline__ void values_of_node(const Real *part, int slot, int c
         const int k = 2 * n + (r >> 3);
         v[n] = k < cnt ? part[(slot + k) * 8 + (r & 7)] : (Real)0;
     }
-    Real t = Sum::add(Sum::add(v[0], v[1]), Sum::add(v[2], v[3]));
-    t = Loose<Real>::norm(Sum::add(t, shfl_xor_any(t, 8)));
+    Real t = L::add(L::add(v[0], v[1]), L::add(v[2], v[3]));
+    t = L::norm(L::add(t, shfl_xor_any(t, 8)));
 #pragma unroll
     for (int n = 0; n < 8; n++) x[n] = shfl_group<16>(t, n);
 }
@@ -451,7 +453,7 @@ __device__ __forceinline__ void small_body(const LevelPtrs<Store> &L, int iters,
             {
                 if (!(r & 1)) part[slot * 8 + (r >> 3) * 4 + ((r & 7) >> 1)] = t;
                 __syncthreads();
-                values_of_node<Real, Sum>(part, slot, cnt, r, x);
+                values_of_node<Real>(part, slot, cnt, r, x);
             }
             if constexpr (NC > 1)
                 if (pending)
@@ -565,7 +567,7 @@ __device__ __forceinline__ void small_colour_body(const LevelPtrs<Store> &L, int
     if (!(r & 1)) part[slot * 8 + (r >> 3) * 4 + ((r & 7) >> 1)] = t;
     __syncthreads();
     Real x[8], p;
-    values_of_node<Real, Sum>(part, slot, cnt, r, x);
+    values_of_node<Real>(part, slot, cnt, r, x);
     if (cnt && relaxed(L, node) && group_step<Real, Sum>(x, r, separate, p) && r < 2)
     {
         const Real cur = LA::norm(Sum::add(mine[26 + r], p));
