@@ -131,6 +131,14 @@ bool make_plan(epr_batch &b)
         const int m = std::min(c->P.min_solve_depth, c->depth);
         if (minD >= 0 && m != minD) return b.fail(who + "all members need the same minimum solve depth");
         minD = m;
+        // levels that no build has reached (a member with systems of the caller's)
+        bool made = false;
+        for (int l = 0; l <= c->depth; l++)
+        {
+            made = made || !c->levels[l].synced;
+            if (!c->level_ready(l)) return b.fail(who + c->err);
+        }
+        if (made && !b.ok(cudaStreamSynchronize(c->stream), "level copies")) return false;
         maxD[i] = c->P.max_solve_depth < 0 ? c->depth : std::min(c->P.max_solve_depth, c->depth);
         top = std::max(top, maxD[i]);
     }

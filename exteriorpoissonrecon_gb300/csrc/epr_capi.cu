@@ -114,12 +114,6 @@ bool Context::ensure_level(int l)
             return false;
         if (!cuda_ok(cudaMemsetAsync(L.xy32, 0, sizeof(float) * 2 * L.N, stream), "memset xy32")) return false;
     }
-    if (dim == 3 && pair_level<3>(l))
-    {
-        // the pair layout from the start: the relaxation of these levels reads nothing else
-        if (!ensure_blocks(l)) return false;
-        if (!cuda_ok(cudaMemsetAsync(L.Acb, 0, block_bytes(l), stream), "memset colour blocks")) return false;
-    }
     if (lvlDF(l))
     {
         if (!alloc((void **)&L.xyd, sizeof(df) * 2 * L.N, "alloc xy df")) return false;
@@ -182,8 +176,8 @@ bool Context::sync_system32(int l)
     }
     if (block_bytes(l))
     {
-        if (dim == 3 && pair_level<3>(l)) return pair_system(*this, l, 0.);
         if (!ensure_blocks(l)) return false;
+        if (dim == 3 && pair_level<3>(l)) return pair_system(*this, l, 0.);
         auto blocks = [&](auto dd) {
             constexpr int D = decltype(dd)::value;
             if (lvl32(l))
@@ -203,11 +197,13 @@ bool Context::sync_system32(int l)
     return L.synced = launch_ok("convert system");
 }
 
-// The copies of a level that no build and no epr_set_level_system has reached, or whose colour blocks a build left
-// as scratch: those of its double stencils, which are zero from the start
+// What the relaxation and the float operators of a level read beside its double stencils.  A build and
+// epr_set_level_system make it; here for a level that neither has reached, or whose colour blocks a build left as
+// scratch, from the double stencils (zero from the start).  Float and double-float levels, and pair levels, whose
+// relaxation reads the pair layout alone, cannot do without; the others fall back on the natural order.
 bool Context::level_ready(int l)
 {
-    const bool copies = lvl32(l) || lvlDF(l) || levels[l].Acb;
+    const bool copies = lvl32(l) || lvlDF(l) || levels[l].Acb || (dim == 3 && pair_level<3>(l));
     return !copies || levels[l].synced || sync_system32(l);
 }
 
@@ -298,6 +294,7 @@ bool Context::energy(int l, double *out3)
 
 bool Context::gs(int l, int iters)
 {
+    if (!level_ready(l)) return false;
     bool fp32 = lvl32(l);
     if (lvlDF(l))
     {
@@ -1145,7 +1142,7 @@ int epr_time_kernel(epr_ctx *ctx, const char *kernel, int level, int reps, doubl
     double *scratch = nullptr;
     void *pair = nullptr, *out = nullptr;
     size_t rs = fp32 ? sizeof(float) : sizeof(double);
-    bool ok = ctx->alloc((void **)&scratch, sizeof(double) * 5 * L.N, "alloc") && ctx->alloc(&pair, rs * 2 * L.N, "alloc") &&
+    bool ok = ctx->level_ready(level) && ctx->alloc((void **)&scratch, sizeof(double) * 5 * L.N, "alloc") && ctx->alloc(&pair, rs * 2 * L.N, "alloc") &&
               ctx->alloc(&out, rs * 2 * L.N, "alloc") && ctx->cuda_ok(cudaMemsetAsync(pair, 0, rs * 2 * L.N, ctx->stream), "memset");
     if (ok && (k == "prolong" && level >= ctx->depth)) { ctx->fail(EPR_ERR_ARG, "no finer level"); ok = false; }
     if (ok && k != "gs" && k != "energy" && k != "quadfit" && k != "prolong" && k != "gn")

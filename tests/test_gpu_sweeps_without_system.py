@@ -84,3 +84,38 @@ def test_sweep_after_a_build_that_ran_out_of_memory(monkeypatch):
     r = epr.Reconstructor(3, 4, pu, sk, precision="fp32")
     r.solve()
     r.close()
+
+
+@pytest.mark.parametrize("dim,depth", [(3, 6), (4, 4)])
+@pytest.mark.parametrize("precision", ["fp32", "fp64"])
+def test_timer_and_solve_without_a_build(dim, depth, precision):
+    """The kernel timer on a context that was never built; a solve and a batch of a context with a system on its
+    finest level alone, the others' stencils zero."""
+    r = epr.Reconstructor(dim, depth, build=False, precision=precision)
+    for level in range(depth + 1):
+        for kernel in ("gs", "energy", "quadfit", "gn"):
+            assert r.time_kernel(kernel, level, 1) > 0
+    r.close()
+    if dim == 4 and precision == "fp64":
+        return
+    out = []
+    for way in ("solve", "batch", "tuned"):
+        r = epr.Reconstructor(dim, depth, build=False, precision=precision, dWeight=0.0)
+        rng = np.random.default_rng(5)
+        R = 0.02 * rng.uniform(-1, 1, (r.nodes(depth), 3 ** dim))
+        R[:, 3 ** dim // 2] = 1.0
+        r.set_level_system(depth, R, 0.1 * R, 1.0)
+        if way == "solve":
+            r.solve()
+        elif dim == 3:
+            b = epr.LockstepBatch([r])
+            if way == "tuned":
+                b.tune(reps=1)
+            b.run()
+            b.close()
+        else:
+            r.solve()
+        out.append(r.coefficients(depth))
+        r.close()
+    for other in out[1:]:
+        assert all(np.array_equal(u, v) for u, v in zip(out[0], other))
