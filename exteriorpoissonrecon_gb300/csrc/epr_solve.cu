@@ -168,7 +168,8 @@ __device__ __forceinline__ void block_sum_store(double *v, double *dst)
     }
 }
 
-template <int D, typename Real>
+// Natural: the level keeps its stencils in Real, so that no load asks (12 to 14 % of the float kernel)
+template <int D, typename Real, bool Natural>
 __global__ void __launch_bounds__(kThreads) energy_kernel(LevelPtrs<Real> L, const Real *xy, double *partial)
 {
     Grid<D> g(L.level);
@@ -216,7 +217,8 @@ __global__ void __launch_bounds__(kThreads) energy_kernel(LevelPtrs<Real> L, con
                 }
                 if (!ok) continue;
                 Real2<Real> v = ld2(xy, j);
-                double a = (double)stencil_a(L, (int64_t)o * L.N + t), b = (double)stencil_b(L, (int64_t)o * L.N + t);
+                const int64_t k = (int64_t)o * L.N + t;
+                const double a = (double)(Natural ? L.A[k] : (Real)L.A64[k]), b = (double)(Natural ? L.B[k] : (Real)L.B64[k]);
                 by += b * (double)v.y;
                 ax += a * (double)v.x;
                 ay += a * (double)v.y;
@@ -995,7 +997,8 @@ void launch_energy(const LevelPtrs<Real> &L, const Real *xy, const Reduce &red, 
     int nb = (int)blocks_for(total);
     if (nb > Reduce::kMaxBlocks) nb = Reduce::kMaxBlocks;
     if (nb < 1) nb = 1;
-    energy_kernel<D, Real><<<nb, kThreads, 0, s>>>(L, xy, red.partial);
+    if (L.A) energy_kernel<D, Real, true><<<nb, kThreads, 0, s>>>(L, xy, red.partial);
+    else energy_kernel<D, Real, false><<<nb, kThreads, 0, s>>>(L, xy, red.partial);
     double scale0 = (D == 3 ? (double)g.r : 1.0) * 0.5;
     finish_kernel<<<1, 96, 0, s>>>(red.partial, nb, 3, red.out, scale0);
 }
