@@ -126,8 +126,8 @@ bool Context::ensure_level(int l)
 
 bool Context::lvl32(int l) const { return P.precision == EPR_FP32 && !(l >= P.fp64_from && l < P.fp64_levels); }
 
-// the coarsest 3D levels of a float solve's band, in double-float when asked (their kernels are the
-// point-split and single-block ones, which take the pair type)
+// the coarsest 3D levels of a float solve's band, in double-float when asked (the levels whose sweeps
+// are one launch, epr_small.cu, in the pair type)
 constexpr int kMaxDFLevel = 3;
 bool Context::lvlDF(int l) const
 {
@@ -318,7 +318,7 @@ bool Context::gs(int l, int iters)
 bool Context::sweeps(int l, int iters)
 {
     if (!level_ready(l)) return false;
-    // solves relax in float with the modal fit; a caller's own sweeps keep the Gauss rule's bits
+    // a caller's own float sweeps of the larger levels keep the Gauss rule's bits (epr_gauss.cu)
     if (iters <= 0 || !lvl32(l) || !(dim == 3 ? gauss_level<3>(l) : gauss_level<4>(l))) return gs(l, iters);
     launches += with_dim(this, [&](auto dd) {
         constexpr int D = decltype(dd)::value;

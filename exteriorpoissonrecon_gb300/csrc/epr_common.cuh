@@ -146,7 +146,8 @@ __host__ __device__ inline int64_t colour_block_base(const Grid<D> &g, int colou
 // axis 0 (A and B of the nine offsets of its plane, then of the node's plane A for lane 0 and B
 // without the centre for lane 1; zero where an offset leaves the grid), padded to 28, as G 16-byte
 // vectors; vector v sits at (v n + j) 2 + s, so that a warp's loads are contiguous.  The rule is the level
-// alone, so that every way to relax a level (solo, listed, batched) computes the same bits.  Measured on
+// alone, so that every way a solve relaxes a level (solo, listed, batched) computes the same bits (a caller's own
+// float sweeps: epr_gauss.cu).  Measured on
 // one colour (float / double): level 6 8.2 against 10.3 us and 157 against 184 us, level 5 with
 // 4,913 nodes no gain (6.2 / 41 us either way: too few warps for the longer thread).
 constexpr int kPairLevel = 6;

@@ -7,11 +7,13 @@
 // fitting energy integrates its Frobenius norm (Hat.inl:358-370: the packed inner product counts
 // every off-diagonal entry twice).  The reference evaluates these integrals through precomputed
 // per-node stencils of 1,358 (3D) / 22,952 (4D) coefficients (Hat.products.inl:32-107).  Here
-// they are integrated per element and per component:
-//   component (P,Q) of W is linear in xi_P and xi_Q and quadratic in the other coordinates, so the
-//   product of two such components is integrated exactly by a 2 x 2 x 3^(D-2) Gauss rule
-//   (12 points in 3D, 36 in 4D).  Gradients at the Gauss points come from sum factorisation:
-//   corner differences along one axis, then 1-D interpolation axis by axis.
+// they are integrated per element and per component, exactly, in one of two ways:
+//   * the node fits of a solve's relaxation, the 3D energy and the Gauss-Newton product on signed sums of the corner
+//     differences and their minors (below, "Quadratic-fit integrals");
+//   * the 4D energy, the alternating system, the bi-quadratic fit (epr_mg.cu) and a caller's own float sweeps
+//     (epr_gauss.cu) on a Gauss rule: component (P,Q) of W is linear in xi_P and xi_Q and quadratic in the other
+//     coordinates, so the product of two such components takes 2 x 2 x 3^(D-2) points (12 in 3D, 36 in 4D), with
+//     gradients by sum factorisation (corner differences along one axis, then 1-D interpolation axis by axis).
 //
 // All routines work in reference-element units; integrals over the physical element (side 1/r)
 // are the returned sums times r^(4-D)/2, which the callers apply (a power of two: exact).

@@ -1,18 +1,19 @@
 // Paired Gauss-Seidel sweeps in float that a caller runs by itself (epr_gs), on the 2 x 2 x 3^(D-2)-point Gauss
-// rule.
+// rule: levels of more than 729 nodes (gauss_level).
 //
 // A solve relaxes with the modal fit, whose last bits differ.  Over a whole solve that does not show (relative
 // differences of 1e-7), but at nodes where the fields' gradients are nearly parallel one sweep divides by a
-// determinant of the size of its own rounding error: the value of such a node is good to two or three digits
-// in float, whichever rule computes it, and of a field of 10^5 to 10^6 nodes a handful are like that.  A program
-// that drives single sweeps sees them, so its sweeps keep the arithmetic, operation for operation, that their
-// results have always had.
+// determinant of the size of the Gauss rule's rounding error: of a field of 10^5 to 10^6 nodes a handful are good to
+// two or three digits (in L2 up to 1e-5 off 64 bits; the modal fit with its shear 5e-7).  A program that drives single
+// sweeps sees the two rules' difference there, so its sweeps keep the arithmetic, operation for operation, that their
+// results have always had.  What it gives up is the fit's accuracy at those nodes and half its speed, and that
+// such a program's own schedule of sweeps and prolongations ends where epr_solve ends to rounding only.
 //
 // Bound by instruction issue: a node's 2^D elements take 36 points each in 3D and 216 in 4D (a depth-8 colour
 // 600 us, where the modal rule on two lanes per node takes 183 us).  Resident blocks of 128 threads asked of the
-// compiler, a call with its copies: 4D level 5, two sweeps, 2 blocks (255 registers) 10.3 ms, 3 blocks 8.75, 5 blocks
-// 11.4 (spills); 3D level 6, four sweeps, 9 blocks 0.89 ms, 7 blocks 0.86, 6 blocks 0.89.  The colours are chained
-// (launch_colour).
+// compiler, a call with its copies, compared side by side: 4D level 5, two sweeps, 2 blocks (255 registers) 10.3 ms, 3
+// blocks 8.75, 5 blocks 11.4 (spills); 3D level 6, four sweeps, 9 blocks 0.89 ms, 7 blocks 0.86, 6 blocks 0.89 (by
+// themselves the chosen ones take 8.5 and 0.92 ms).  The colours are chained (launch_colour).
 #include <algorithm>
 #include <cmath>
 

@@ -60,20 +60,21 @@ bool launch_gs_colour(const LevelPtrs<Real> &L, int colour, unsigned int *err, c
 void launch_df_push(const double *in, df *out, int64_t n, int *kexp, int level, cudaStream_t s);
 void launch_df_pull(const df *in, double *out, int64_t n, const int *kexp, int level, cudaStream_t s);
 void launch_d2df(const double *in, df *out, int64_t n, cudaStream_t s);
-// iters full sweeps (all 2^D colours in order); the small levels run all sweeps in one launch, larger
-// ones launch one kernel per colour.  Returns the number of kernels launched.
-// The sweeps of a caller that runs them by itself, in float, on levels that take a launch per colour
-// (gauss_level): the Gauss rule's arithmetic.
+// The sweeps of a caller that runs them by itself, in float, on levels of more than 729 nodes (gauss_level): the Gauss
+// rule's arithmetic, whose bits they keep (epr_gauss.cu).  The smaller levels run a solve's kernels, which are
+// nearer to 64 bits; the nodes where the rules differ visibly, one in 10^5, are not found there.
 template <int D>
 bool gauss_level(int level) { return level >= (D == 3 ? 4 : 3); }
 template <int D>
 int launch_gauss_sweeps(const LevelPtrs<float> &L, int iters, unsigned int *err, cudaStream_t s, int separate);
+// iters full sweeps (all 2^D colours in order) as a solve runs them; the small levels run all sweeps in one
+// launch, larger ones launch one kernel per colour.  Returns the number of kernels launched.
 template <int D, typename Real>
 int launch_gs_sweeps(const LevelPtrs<Real> &L, int iters, unsigned int *err, cudaStream_t s, int separate = 0);
 
 // The small 3D levels (epr_small.cu).  All sweeps in one launch: levels 0-2, and level 3 but in double;
 // levels 3 and 4 in double by its per-colour launches (a lane per element leaves three of four FP64
-// units without a warp there: level 4 14.5 us a colour).
+// units without a warp there: level 4 14.5 us a colour against 9.7).
 constexpr int kSmallLevels3 = 5;
 template <typename Real>
 constexpr bool small_level(int level) { return level < 3 || (level == 3 && !std::is_same<Real, double>::value); }

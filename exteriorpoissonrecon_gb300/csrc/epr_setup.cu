@@ -649,8 +649,9 @@ __device__ double est_depth_raw(const DensityGrids<D> &G, int maxT, const double
     return d1 + log(tg / s1) / log(s2 / s1);
 }
 
-// ascending eigenvalues of a symmetric D x D matrix (cyclic Jacobi, until what is left off the diagonal
-// cannot change a bit of it; every loop unrolled, so that the matrix stays in registers)
+// ascending eigenvalues of a symmetric D x D matrix (cyclic Jacobi, until what is left off the diagonal is below
+// 1e-20 of the matrix: the covariances here are differences good to 1e-16 of it, and their eigenvalues enter as
+// shares of the trace; every loop unrolled, so that the matrix stays in registers)
 template <int D>
 __device__ void sym_eigenvalues(double a[D][D], double *ev)
 {

@@ -1,6 +1,7 @@
-// Relaxation of the small 3D levels (levels 0-3: 8, 27, 125 and 729 nodes): all sweeps of a level in one
-// launch, on one block (levels 0 and 1) or one cluster of eight blocks (levels 2 and 3), solo and for
-// every member of a lockstep batch; double level 3 by one launch per colour.
+// Relaxation of the small levels.  3D levels 0-3 (8, 27, 125 and 729 nodes): all sweeps of a level in one launch,
+// on one block (levels 0 and 1), a cluster of eight blocks (level 2) or of 16 (level 3; eight where the device
+// holds no larger one), solo and for every member of a lockstep batch; in double levels 3 and 4 by one launch per
+// colour.  4D levels 0-3 in double further down.
 //
 // What bounds them: nothing but the dependent chain of a colour phase, thousands of times (a depth-8
 // schedule has 38,400 phases on these levels, of 1 to 125 nodes).  So the work of a phase is laid out for

@@ -490,9 +490,9 @@ __device__ __forceinline__ void gs_update_lanes_at(const LevelPtrs<Real> &L, Rea
 }
 
 // Two lanes per node (large 3D levels): issue slots and the FMA pipe set the pace (a node's 2 x 800
-// instructions against 287 bytes).  One depth-8 colour, float: 183 us alone, 177 us chained (0.52 of the measured
-// copy bandwidth on 617 MB; 171 us without the float kernels' shear, unchained) against 600 us for a lane per element on a 12-point Gauss rule and 402 us for a lane
-// per element on the rule used now; double at depth 7: 1.06 ms against 3.5 ms, the FP64 pipe busy.  Lane s takes the four
+// instructions against 287 bytes).  One depth-8 colour, float: 177 us where the colours follow each other as a solve runs them (0.52 of the measured
+// copy bandwidth on 617 MB), 183 us launched by itself, against 600 us for a lane per element on a 12-point Gauss rule and 402 us for a lane
+// per element on the rule used now (both by themselves; 171 us without the float kernels' shear); double at depth 7: 1.06 ms against 3.5 ms, the FP64 pipe busy.  Lane s takes the four
 // elements on side s of axis 0 with the 18 grid points of its own and the node's plane in registers,
 // the stencil columns of its plane, and of the node's plane the A column (lane 0) or the B column
 // (lane 1), which the pair layout keeps as one run of 16-byte vectors per lane (PairLayout); one

@@ -187,7 +187,11 @@ int epr_energy(epr_ctx *ctx, int level, double *out3);
 int epr_quadfit(epr_ctx *ctx, int level, double *out);
 /* Energy gradient (dE/dx, dE/dy). */
 int epr_gradient(epr_ctx *ctx, int level, double *gx, double *gy);
-/* iters paired Gauss-Seidel sweeps over the 2^dim parity colours, in place. */
+/* iters paired Gauss-Seidel sweeps over the 2^dim parity colours, in place.  A level without a system has zero
+ * stencils.  In EPR_FP32 the sweeps of float levels of more than 729 nodes (3D from level 4, 4D from level 3 on) use
+ * the Gauss rule, where a solve uses a fit that is nearer to double at nodes whose fields' gradients are nearly
+ * parallel; the two differ in the last bits elsewhere.  Smaller float levels keep more than float's digits between
+ * the sweeps of one call.  Double and double-float levels compute a solve's bits. */
 int epr_gs(epr_ctx *ctx, int level, int iters);
 /* coefficients[level+1] += P coefficients[level] */
 int epr_prolong(epr_ctx *ctx, int level);
