@@ -288,7 +288,7 @@ def kernel_rooflines(r, dim, depth, precision, clk):
                 "launch_ms": gs_ms, "algorithmic_bytes_per_launch": gs_bytes,
                 "note": ("issue-bound quartic relaxation; bytes = coefficient read + stencil columns + update writes; "
                          "the finest level's colour launches take share_of_step of the step, the rest is the "
-                         "coarser levels (levels 0-3: thousands of latency-bound launches)"),
+                         "coarser levels (levels 0-3: chains of thousands of dependent colours)"),
                 "compute": {"algorithmic_flops_per_launch": gs_flops, "achieved_tflops": gs_flops / (gs_ms * 1e-3) / 1e12,
                             "peak_tflops": fp32_peak,
                             "peak_source": "measured: FP32 SGEMM (cuBLAS through torch, TF32 off), 8192^3, best of 5",
