@@ -75,7 +75,17 @@ bool Context::alloc(void **p, size_t bytes, const char *what)
     }
     alloc_total += bytes;
     if (!cuda_ok(cudaMallocAsync(p, bytes, stream), what)) return false;
-    live.insert(*p);
+    try
+    {
+        live.insert(*p);
+    }
+    catch (...)  // no host memory for the record
+    {
+        cudaFreeAsync(*p, stream);
+        *p = nullptr;
+        fail(EPR_ERR_NOMEM, "%s: out of host memory", what);
+        return false;
+    }
     return true;
 }
 
