@@ -394,12 +394,12 @@ __device__ __forceinline__ void gs_update_lanes_at(const LevelPtrs<Real> &L, Rea
     Shear<Real> sh = {(Real)0, (Real)0};
     // node indices in 32 bits (every supported grid has < 2^32 nodes); signed strides of the
     // element mirrored so that the node is its corner 0
-    int sd[D], other = 0;
+    int jj[C], other = 0;
     uint32_t iu = 0;
     bool ok = active;
     if (active)
     {
-        int st[D];
+        int st[D], sd[D];
         st[D - 1] = 1;
 #pragma unroll
         for (int d = D - 2; d >= 0; d--) st[d] = st[d + 1] * (g.r + 1);
@@ -417,6 +417,14 @@ __device__ __forceinline__ void gs_update_lanes_at(const LevelPtrs<Real> &L, Rea
         other = A ^ first;
         if (ok)
         {
+#pragma unroll
+            for (int cc = 0; cc < C; cc++)
+            {
+                jj[cc] = (int)iu;
+#pragma unroll
+                for (int d = 0; d < D; d++)
+                    if (cbit<D>(cc, d)) jj[cc] += sd[d];
+            }
             const int64_t step = Ac ? nc : L.N;
             const Real *pA = (Ac ? Ac + jc : L.A + i) + (int64_t)Dims<D>::CENTER * step;
             const Real *pB = (Ac ? Bc + jc : L.B + i) + (int64_t)Dims<D>::CENTER * step;
@@ -444,14 +452,7 @@ __device__ __forceinline__ void gs_update_lanes_at(const LevelPtrs<Real> &L, Rea
     if (ok)
     {
 #pragma unroll
-        for (int cc = 0; cc < C; cc++)
-        {
-            int jj = (int)iu;
-#pragma unroll
-            for (int d = 0; d < D; d++)
-                if (cbit<D>(cc, d)) jj += sd[d];
-            f[cc] = ld2(xy, (int64_t)(uint32_t)jj);
-        }
+        for (int cc = 0; cc < C; cc++) f[cc] = ld2(xy, (int64_t)(uint32_t)jj[cc]);
         acen = ca[0];
 #pragma unroll
         for (int cc = 0; cc < C; cc++)
